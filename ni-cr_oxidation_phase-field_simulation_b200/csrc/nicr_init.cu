@@ -246,24 +246,51 @@ __device__ __forceinline__ Ext shfl_ext(Ext e, int off) {
     return Ext{__shfl_down_sync(0xffffffffu, e.v, off), __shfl_down_sync(0xffffffffu, e.i, off)};
 }
 
+// Whole rows of cells for the reductions below: warp w of the grid takes the
+// 32-column segments w, w + W, ... of the rows in reference order, one lane per
+// column, so a lane meets its cells in that order (a strict comparison keeps
+// the first extremum) and a segment costs two 32-bit divisions instead of two
+// 64-bit ones per cell. fn(c, x, row, col, idx) gets the cell and its storage
+// index; the lanes past the row's end are left out.
+template <class Fn>
+__device__ __forceinline__ void for_segments(const Grid& g, Fn fn) {
+    const int lane = threadIdx.x & 31;
+    const unsigned nseg = (unsigned)(g.nb + 31) / 32u, total = (unsigned)g.nx * (unsigned)g.na * nseg;
+    const unsigned nwarps = gridDim.x * (blockDim.x >> 5);
+    for (unsigned s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < total; s += nwarps) {
+        const unsigned r = s / nseg;
+        const int col = (int)(s - r * nseg) * 32 + lane;
+        if (col >= g.nb) continue;
+        const int x = (int)(r / (unsigned)g.na), row = (int)(r - (unsigned)x * (unsigned)g.na);
+        fn((long long)r * g.nb + col, x, row, col, (long long)r * g.pb + col);
+    }
+}
+// A later cell of the same lane replaces the extremum only when strictly beyond it.
+__device__ __forceinline__ void keep_min(Ext& e, double v, long long c) {
+    if (v < e.v) { e.v = v; e.i = c; }
+}
+__device__ __forceinline__ void keep_max(Ext& e, double v, long long c) {
+    if (e.v < v) { e.v = v; e.i = c; }
+}
+
+// Reads o, cr and phi once: bound by HBM (24 B per cell) or, when they are in
+// L2, by the double-double chains. At 128^3 (in L2) 60 us with a 64-bit
+// division pair per cell; 44 us now.
 __global__ void k_diagnostics(const Grid g, const double* __restrict__ o, const double* __restrict__ cr,
                               const double* __restrict__ p, DiagOut* partials) {
     DD acc[4] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
     Ext mn[4] = {{1., -1}, {1., -1}, {1., -1}, {1., -1}}, mx[4] = {{0., -1}, {0., -1}, {0., -1}, {0., -1}};
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.ncells; c += (long long)gridDim.x * blockDim.x) {
-        int xi, row, col;
-        decode(g, c, xi, row, col);
-        const long long idx = (long long)xi * g.plane + (long long)row * g.pb + col;
+    for_segments(g, [&](long long c, int, int, int, long long idx) {
         const double ov = o[idx], cv = cr[idx], pv = p[idx];
         acc[0] = dd_add(acc[0], ov);
         acc[1] = dd_add(acc[1], cv);
         acc[2] = dd_add(acc[2], pv);
         acc[3] = dd_add(acc[3], h(pv));
-        mn[0] = ext_min(mn[0], Ext{ov, c}); mx[0] = ext_max(mx[0], Ext{ov, c});
-        mn[1] = ext_min(mn[1], Ext{cv, c}); mx[1] = ext_max(mx[1], Ext{cv, c});
-        mn[2] = ext_min(mn[2], Ext{1. - ov - cv, c});
-        mn[3] = ext_min(mn[3], Ext{pv, c}); mx[3] = ext_max(mx[3], Ext{pv, c});
-    }
+        keep_min(mn[0], ov, c); keep_max(mx[0], ov, c);
+        keep_min(mn[1], cv, c); keep_max(mx[1], cv, c);
+        keep_min(mn[2], 1. - ov - cv, c);
+        keep_min(mn[3], pv, c); keep_max(mx[3], pv, c);
+    });
     for (int off = 16; off > 0; off >>= 1)
         for (int q = 0; q < 4; ++q) {
             mn[q] = ext_min(mn[q], shfl_ext(mn[q], off));
@@ -286,20 +313,35 @@ __global__ void k_diagnostics(const Grid g, const double* __restrict__ o, const 
     }
 }
 
+// One CTA over the partials, thread t taking t, t + 256, ... (one thread alone
+// walked 592 partials in 675 us, a chain of dependent loads; 17 us now).
 __global__ void k_diag_finalize(const DiagOut* __restrict__ partials, int nblocks, DiagOut* out) {
-    if (threadIdx.x != 0) return;
-    DiagOut r = partials[0];
-    for (int b = 1; b < nblocks; ++b) {
+    DD acc[4] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
+    Ext mn[4] = {{1., -1}, {1., -1}, {1., -1}, {1., -1}}, mx[4] = {{0., -1}, {0., -1}, {0., -1}, {0., -1}};
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
         for (int q = 0; q < 4; ++q) {
-            DD s = dd_add(DD{r.sum[q][0], r.sum[q][1]}, DD{partials[b].sum[q][0], partials[b].sum[q][1]});
-            r.sum[q][0] = s.hi; r.sum[q][1] = s.lo;
-            Ext a = ext_min(Ext{r.mn[q], r.mni[q]}, Ext{partials[b].mn[q], partials[b].mni[q]});
-            r.mn[q] = a.v; r.mni[q] = a.i;
-            Ext z = ext_max(Ext{r.mx[q], r.mxi[q]}, Ext{partials[b].mx[q], partials[b].mxi[q]});
-            r.mx[q] = z.v; r.mxi[q] = z.i;
+            acc[q] = dd_add(acc[q], DD{partials[b].sum[q][0], partials[b].sum[q][1]});
+            mn[q] = ext_min(mn[q], Ext{partials[b].mn[q], partials[b].mni[q]});
+            mx[q] = ext_max(mx[q], Ext{partials[b].mx[q], partials[b].mxi[q]});
         }
+    for (int off = 16; off > 0; off >>= 1)
+        for (int q = 0; q < 4; ++q) {
+            mn[q] = ext_min(mn[q], shfl_ext(mn[q], off));
+            mx[q] = ext_max(mx[q], shfl_ext(mx[q], off));
+        }
+    __shared__ Ext smn[32][4], smx[32][4];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    if (lane == 0) for (int q = 0; q < 4; ++q) { smn[w][q] = mn[q]; smx[w][q] = mx[q]; }
+    long long dummy = 0;
+    block_reduce<4>(acc, dummy);   // contains the __syncthreads that publishes smn/smx
+    if (threadIdx.x != 0) return;
+    for (int ww = 1; ww < nw; ++ww)
+        for (int q = 0; q < 4; ++q) { mn[q] = ext_min(mn[q], smn[ww][q]); mx[q] = ext_max(mx[q], smx[ww][q]); }
+    for (int q = 0; q < 4; ++q) {
+        out->sum[q][0] = acc[q].hi; out->sum[q][1] = acc[q].lo;
+        out->mn[q] = mn[q].v; out->mx[q] = mx[q].v;
+        out->mni[q] = mn[q].i; out->mxi[q] = mx[q].i;
     }
-    *out = r;
 }
 
 // ---- grain statistics (Model::grain_log, 3S:566-590; grain_energy 3S:546-565)
@@ -311,58 +353,82 @@ struct GrainPart {
     Ext lo, hi, slo, shi, gbmax;
     long long unassigned;
 };
-__global__ void k_grain_scalar(const GrainParams G, const double* __restrict__ eta, const double* __restrict__ s2,
+// a / b for a run constant b (xdiv_flag; the rare uncertified quotient by IEEE division)
+__device__ __forceinline__ double div_const(double a, const DivC& d) {
+    unsigned bad = 0;
+    const double q = xdiv_flag(a, d, bad);
+    return bad ? __ddiv_rn(a, d.b) : q;
+}
+// Counters of the dominant grains kept in shared memory per CTA when they fit.
+constexpr int kGrainCountCap = 1024;
+
+// Each field is read once with its three forward neighbours (L1/L2). The
+// counts of a warp's equal grains are added by one lane, to shared memory for
+// up to kGrainCountCap grains: with one 64-bit global atomic per cell, a few
+// grains of many cells serialised at their L2 addresses, and with the IEEE
+// divisions by the spacings and 64-bit index divisions that was 1227 us at
+// 128^3 with 8 fields; 207 us now (64 registers, 4 CTAs per SM: 271 us at 2).
+__global__ void __launch_bounds__(256, 4) k_grain_scalar(const GrainParams G, const double* __restrict__ eta, const double* __restrict__ s2,
                                const double* __restrict__ p, const double* __restrict__ gb,
                                unsigned long long* __restrict__ cells, GrainPart* parts) {
     const Grid& g = G.g;
+    __shared__ unsigned scount[kGrainCountCap];
+    const bool in_smem = G.neta <= kGrainCountCap;
+    if (in_smem) {
+        for (int q = threadIdx.x; q < G.neta; q += blockDim.x) scount[q] = 0;
+        __syncthreads();
+    }
     DD acc[3] = {{0., 0.}, {0., 0.}, {0., 0.}};
     Ext lo{1., -1}, hi{0., -1}, slo{CUDART_INF, -1}, shi{0., -1}, gbmax{0., -1};
     long long unassigned = 0;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.ncells; c += (long long)gridDim.x * blockDim.x) {
-        int xi, row, col;
-        decode(g, c, xi, row, col);
-        const long long idx = (long long)xi * g.plane + (long long)row * g.pb + col;
+    for_segments(g, [&](long long c, int xi, int row, int col, long long idx) {
         const double S = s2[idx], pv = p[idx], metal = 1. - h(pv), gbv = gb[idx];
-        slo = ext_min(slo, Ext{S, c});
-        shi = ext_max(shi, Ext{S, c});
+        keep_min(slo, S, c);
+        keep_max(shi, S, c);
         acc[0] = dd_add(acc[0], S);
         acc[1] = dd_add(acc[1], metal * gbv);
-        gbmax = ext_max(gbmax, Ext{gbv, c});
+        keep_max(gbmax, gbv, c);
+        // the forward neighbours (Neumann X: no term at the last plane; periodic rows and columns)
+        const bool x_on = xi < g.nx - 1 || G.x_above;
+        const long long ixp = x_on ? idx + g.plane : idx;
+        const long long iap = G.dim == 3 ? idx + (row == g.na - 1 ? -(long long)row * g.pb : (long long)g.pb) : idx;
+        const long long ibp = idx + (col == g.nb - 1 ? -col : 1);
         // current_grain (3S:527-533): eta argmax above 1e-12 in metal (phi < .5)
         int id = 0;
         double best = 1.e-12;
         double pairs = 0., Sr = 0.;
+#pragma unroll 4
         for (int q = 0; q < G.neta; ++q) {
             const double v = eta[(long long)q * g.nstore + idx];
-            lo = ext_min(lo, Ext{v, c * G.neta + q});
-            hi = ext_max(hi, Ext{v, c * G.neta + q});
+            keep_min(lo, v, c * G.neta + q);
+            keep_max(hi, v, c * G.neta + q);
             if (v > best) { best = v; id = q + 1; }
             const double sq = v * v;
             pairs += Sr * sq;
             Sr += sq;
         }
         if (pv >= .5) id = 0;
-        if (id) atomicAdd(cells + (id - 1), 1ull);
-        else if (pv < .5) ++unassigned;
-        // energy density: local terms + forward-face gradients (Neumann X, periodic rows/cols)
+        const unsigned peers = __match_any_sync(__activemask(), id);
+        if (id) {
+            if ((threadIdx.x & 31) == __ffs(peers) - 1) {
+                if (in_smem) atomicAdd(&scount[id - 1], (unsigned)__popc(peers));
+                else atomicAdd(cells + (id - 1), (unsigned long long)__popc(peers));
+            }
+        } else if (pv < .5) {
+            ++unassigned;
+        }
+        // energy density: local terms + forward-face gradients
         double density = grain_energy_density(S, G.dim == 3 ? pairs : G.pairs[idx], pv, G.W, G.A);
-        const long long ixp = idx + g.plane;
-        const long long iap = (long long)xi * g.plane + (long long)(row == g.na - 1 ? 0 : row + 1) * g.pb + col;
-        const long long ibp = (long long)xi * g.plane + (long long)row * g.pb + (col == g.nb - 1 ? 0 : col + 1);
+#pragma unroll 4
         for (int q = 0; q < G.neta; ++q) {
             const double* e = eta + (long long)q * g.nstore;
             const double ec = e[idx];
-            if (xi < g.nx - 1 || G.x_above) { const double t = (e[ixp] - ec) / G.dx; density += .5 * G.K * (t * t); }
-            if (G.dim == 3) {
-                { const double t = (e[iap] - ec) / G.da; density += .5 * G.K * (t * t); }
-                { const double t = (e[ibp] - ec) / G.db; density += .5 * G.K * (t * t); }
-            } else {
-                const double t = (e[ibp] - ec) / G.db;
-                density += .5 * G.K * (t * t);
-            }
+            if (x_on) { const double t = div_const(e[ixp] - ec, G.v_dx); density += .5 * G.K * (t * t); }
+            if (G.dim == 3) { const double t = div_const(e[iap] - ec, G.v_da); density += .5 * G.K * (t * t); }
+            { const double t = div_const(e[ibp] - ec, G.v_db); density += .5 * G.K * (t * t); }
         }
         acc[2] = dd_add(acc[2], G.dim == 3 ? density * G.dx * G.da * G.db : density * G.dx * G.db);
-    }
+    });
     // block reduction
     for (int off = 16; off > 0; off >>= 1) {
         lo = ext_min(lo, shfl_ext(lo, off)); hi = ext_max(hi, shfl_ext(hi, off));
@@ -372,7 +438,10 @@ __global__ void k_grain_scalar(const GrainParams G, const double* __restrict__ e
     __shared__ Ext se[32][5];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     if (lane == 0) { se[w][0] = lo; se[w][1] = hi; se[w][2] = slo; se[w][3] = shi; se[w][4] = gbmax; }
-    block_reduce<3>(acc, unassigned);
+    block_reduce<3>(acc, unassigned);   // contains the __syncthreads that publishes se and scount
+    if (in_smem)
+        for (int q = threadIdx.x; q < G.neta; q += blockDim.x)
+            if (scount[q]) atomicAdd(cells + q, (unsigned long long)scount[q]);
     if (threadIdx.x == 0) {
         for (int ww = 1; ww < nw; ++ww) {
             lo = ext_min(lo, se[ww][0]); hi = ext_max(hi, se[ww][1]);
@@ -388,21 +457,14 @@ __global__ void k_grain_scalar(const GrainParams G, const double* __restrict__ e
 // weighted metal amount of grain q: sum of (1-h) eta_q^2 / S over cells with S > 1e-24
 __global__ void k_grain_amount(const GrainParams G, const double* __restrict__ eta, const double* __restrict__ s2,
                                const double* __restrict__ p, double* amount_parts /* [gridDim.x][neta][2] */) {
-    const Grid& g = G.g;
     const int q = blockIdx.y;
     DD acc[1] = {{0., 0.}};
     long long dummy = 0;
-    const double* e = eta + (long long)q * g.nstore;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.ncells; c += (long long)gridDim.x * blockDim.x) {
-        int xi, row, col;
-        decode(g, c, xi, row, col);
-        const long long idx = (long long)xi * g.plane + (long long)row * g.pb + col;
-        const double S = s2[idx];
-        if (S > 1.e-24) {
-            const double v = e[idx], metal = 1. - h(p[idx]);
-            acc[0] = dd_add(acc[0], metal * v * v / S);
-        }
-    }
+    const double* e = eta + (long long)q * G.g.nstore;
+    for_segments(G.g, [&](long long, int, int, int, long long idx) {
+        const double S = s2[idx], v = e[idx], metal = 1. - h(p[idx]);
+        if (S > 1.e-24) acc[0] = dd_add(acc[0], metal * v * v / S);
+    });
     block_reduce<1>(acc, dummy);
     if (threadIdx.x == 0) {
         amount_parts[((long long)blockIdx.x * G.neta + q) * 2] = acc[0].hi;
@@ -410,34 +472,49 @@ __global__ void k_grain_amount(const GrainParams G, const double* __restrict__ e
     }
 }
 
+// CTA 0 reduces the scalars (thread t: partials t, t + 256, ...), warp w of the
+// further CTAs one grain's amount each. A single thread walking the partials
+// took 394 us for 296 of them with 8 grains; 13 us now.
 __global__ void k_grain_finalize(const GrainParams G, const GrainPart* __restrict__ parts, int nparts,
                                  const double* __restrict__ amount_parts, const unsigned long long* __restrict__ cells,
                                  GrainOut* out, double* amount_out, long long* cells_out) {
-    // one thread per grain for the amounts (block order), thread 0 for the scalars
-    for (int q = threadIdx.x; q < G.neta; q += blockDim.x) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (blockIdx.x > 0) {
+        const int q = (blockIdx.x - 1) * nw + w;
+        if (q >= G.neta) return;
         DD a{0., 0.};
-        for (int b = 0; b < nparts; ++b)
+        for (int b = lane; b < nparts; b += 32)
             a = dd_add(a, DD{amount_parts[((long long)b * G.neta + q) * 2], amount_parts[((long long)b * G.neta + q) * 2 + 1]});
-        amount_out[2 * q] = a.hi;
-        amount_out[2 * q + 1] = a.lo;
-        cells_out[q] = (long long)cells[q];
-    }
-    if (threadIdx.x == 0) {
-        GrainPart r = parts[0];
-        for (int b = 1; b < nparts; ++b) {
-            for (int q = 0; q < 3; ++q) {
-                DD s = dd_add(DD{r.sum[q][0], r.sum[q][1]}, DD{parts[b].sum[q][0], parts[b].sum[q][1]});
-                r.sum[q][0] = s.hi; r.sum[q][1] = s.lo;
-            }
-            r.lo = ext_min(r.lo, parts[b].lo); r.hi = ext_max(r.hi, parts[b].hi);
-            r.slo = ext_min(r.slo, parts[b].slo); r.shi = ext_max(r.shi, parts[b].shi);
-            r.gbmax = ext_max(r.gbmax, parts[b].gbmax);
-            r.unassigned += parts[b].unassigned;
+        for (int off = 16; off > 0; off >>= 1) a = dd_add(a, shfl_dd(a, off));
+        if (lane == 0) {
+            amount_out[2 * q] = a.hi;
+            amount_out[2 * q + 1] = a.lo;
+            cells_out[q] = (long long)cells[q];
         }
-        out->lo = r.lo.v; out->hi = r.hi.v; out->slo = r.slo.v; out->shi = r.shi.v; out->gbmax = r.gbmax.v;
-        for (int q = 0; q < 3; ++q) { out->sum[q][0] = r.sum[q][0]; out->sum[q][1] = r.sum[q][1]; }
-        out->unassigned = r.unassigned;
+        return;
     }
+    DD acc[3] = {{0., 0.}, {0., 0.}, {0., 0.}};
+    Ext e[5] = {{1., -1}, {0., -1}, {CUDART_INF, -1}, {0., -1}, {0., -1}};   // lo hi slo shi gbmax, as in the kernel above
+    long long unassigned = 0;
+    auto merge = [&](const Ext& lo, const Ext& hi, const Ext& slo, const Ext& shi, const Ext& gbm) {
+        e[0] = ext_min(e[0], lo); e[1] = ext_max(e[1], hi); e[2] = ext_min(e[2], slo);
+        e[3] = ext_max(e[3], shi); e[4] = ext_max(e[4], gbm);
+    };
+    for (int b = threadIdx.x; b < nparts; b += blockDim.x) {
+        for (int q = 0; q < 3; ++q) acc[q] = dd_add(acc[q], DD{parts[b].sum[q][0], parts[b].sum[q][1]});
+        merge(parts[b].lo, parts[b].hi, parts[b].slo, parts[b].shi, parts[b].gbmax);
+        unassigned += parts[b].unassigned;
+    }
+    for (int off = 16; off > 0; off >>= 1)
+        merge(shfl_ext(e[0], off), shfl_ext(e[1], off), shfl_ext(e[2], off), shfl_ext(e[3], off), shfl_ext(e[4], off));
+    __shared__ Ext se[32][5];
+    if (lane == 0) for (int q = 0; q < 5; ++q) se[w][q] = e[q];
+    block_reduce<3>(acc, unassigned);   // contains the __syncthreads that publishes se
+    if (threadIdx.x != 0) return;
+    for (int ww = 1; ww < nw; ++ww) merge(se[ww][0], se[ww][1], se[ww][2], se[ww][3], se[ww][4]);
+    out->lo = e[0].v; out->hi = e[1].v; out->slo = e[2].v; out->shi = e[3].v; out->gbmax = e[4].v;
+    for (int q = 0; q < 3; ++q) { out->sum[q][0] = acc[q].hi; out->sum[q][1] = acc[q].lo; }
+    out->unassigned = unassigned;
 }
 
 int grid_for(long long n, int threads, int cap) {
@@ -487,21 +564,21 @@ void launch_reduce_partials(const StepPartial* partials, int nblocks, StepPartia
 }
 void launch_grain_stats(const GrainParams& G, const double* eta, const double* s2, const double* p, const double* gb,
                         GrainWork& W, GrainOut* out, double* amount_out, long long* cells_out, cudaStream_t stream) {
-    const int nb = grid_for(G.g.ncells, 256, 148 * 2);
+    const int nb = grain_blocks(G.g.ncells);
     cudaMemsetAsync(W.cells, 0, (size_t)G.neta * sizeof(unsigned long long), stream);
     k_grain_scalar<<<nb, 256, 0, stream>>>(G, eta, s2, p, gb, W.cells, reinterpret_cast<GrainPart*>(W.parts));
     k_grain_amount<<<dim3(nb, G.neta), 256, 0, stream>>>(G, eta, s2, p, W.amount_parts);
-    k_grain_finalize<<<1, 256, 0, stream>>>(G, reinterpret_cast<const GrainPart*>(W.parts), nb, W.amount_parts, W.cells,
+    k_grain_finalize<<<1 + (G.neta + 7) / 8, 256, 0, stream>>>(G, reinterpret_cast<const GrainPart*>(W.parts), nb, W.amount_parts, W.cells,
                                            out, amount_out, cells_out);
 }
 size_t grain_part_bytes() { return sizeof(GrainPart); }
-int grain_blocks(long long ncells) { return grid_for(ncells, 256, 148 * 2); }
+int grain_blocks(long long ncells) { return grid_for(ncells, 256, 148 * 4); }
 
 void launch_diagnostics(const Grid& g, const double* o, const double* cr, const double* p, DiagOut* partials,
                         int* nblocks, DiagOut* out, cudaStream_t stream) {
     const int nb = grid_for(g.ncells, 256, 148 * 4);
     k_diagnostics<<<nb, 256, 0, stream>>>(g, o, cr, p, partials);
-    k_diag_finalize<<<1, 32, 0, stream>>>(partials, nb, out);
+    k_diag_finalize<<<1, 256, 0, stream>>>(partials, nb, out);
     if (nblocks) *nblocks = nb;
 }
 

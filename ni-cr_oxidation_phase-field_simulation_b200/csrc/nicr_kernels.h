@@ -317,6 +317,7 @@ struct GrainParams {
     Grid g;
     int dim, neta;
     double dx, da, db, K, W, A;
+    DivC v_dx, v_da, v_db;       // exact divisions by dx, da, db
     const double* pairs;   // 2D: eta_pairs of the last mask (2D:337); unused in 3D
     int x_above;           // the plane after g's last one is stored and in the domain (an X slab
                            // below another): the last plane keeps its +X gradient term

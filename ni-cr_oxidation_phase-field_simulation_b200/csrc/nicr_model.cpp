@@ -1305,6 +1305,7 @@ void Model::grain_stats(nicr_grain_stats* out, long long* cells, double* amount)
     G.g.nstore = g.nstore;
     G.dim = dim; G.neta = neta;
     G.dx = c.dx; G.da = c.dy; G.db = dim == 3 ? c.dz : c.dy;
+    G.v_dx = sp.v_dx; G.v_da = sp.v_da; G.v_db = sp.v_db;
     G.K = ec.K; G.W = c.eta_W; G.A = ec.A;
     G.pairs = pairs;
     G.x_above = x_off + sp.x_hi < c.nx ? 1 : 0;
