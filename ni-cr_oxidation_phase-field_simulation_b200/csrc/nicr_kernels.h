@@ -58,11 +58,32 @@ struct StepPartial {
     int pad;
 };
 
+// Exact divisions by the run constants (drop-in form): dx*dx etc. are the
+// Laplacian denominators (3S:193-195); X, rows (a), columns (b).
+struct DivSet {
+    DivC dxdx, dada, dbdb, dx, da, db, dt;
+};
+// The reciprocal form's run constants, folded on the host so that the kernels
+// spend one multiply-add per neighbour pair and no separate scaling.
+struct FastC {
+    double rdx;                // 1 / dx
+    double wx, wa, wb, w0;     // 1/dx^2, 1/da^2, 1/db^2 and minus twice their sum: the Laplacian's weights
+    double fx, fa, fb;         // dt / (2 dx^2) ...: the flux divergence's weights
+    double gbo, gbc;           // bulk mobility times (gb_factor - 1)
+    double px, pa, pb, p0;     // dt L 2 kp times the Laplacian's weights
+    double ex, ea, eb, e0;     // dt eta_L K times the Laplacian's weights
+    double tS, tH, t1, e2;     // dt eta_L times 3W, W + A, W, 2W
+    double x0, hS, hH;         // phi force: constant term, (W + A)/2, W/2
+    double ckO, ckCr;          // -Ck / dt
+};
+
 struct StepParams {
     Grid g;
-    double dx, da, db, dt;       // spacing along X, rows, columns
-    double dxdx, dada, dbdb;     // c.dx*c.dx etc. (lap denominators, 3S:193-195)
-    DivC v_dxdx, v_dada, v_dbdb, v_dx, v_da, v_db, v_dt;  // exact divisions by the same constants
+    double dx, dt;               // spacing along X
+    union {                      // by form: the other form's constants are not needed
+        DivSet div;              // fast == 0
+        FastC f;                 // fast == 1
+    };
     double dtL;                  // dt * Physics::L
     double layer_o;
     double gbm1_o, gbm1_cr;      // gb_factor_o - 1, gb_factor_cr - 1
@@ -86,6 +107,48 @@ struct StepParams {
     // Error word of this step: -1 st->err_key, 0/1 st->slot_err[err_slot] (slab form)
     int err_slot, pad_;
 };
+// The run constants of the configured form (spacings along X, rows, columns);
+// the other scalar members of sp are set already. Returns the exact divisions,
+// which the refresh of either form uses.
+inline DivSet fill_form_constants(StepParams& sp, int dim, double dx, double da, double db) {
+    DivSet d;
+    d.dxdx = make_divc(dx * dx);
+    d.dada = make_divc(da * da);
+    d.dbdb = make_divc(db * db);
+    d.dx = make_divc(dx);
+    d.da = make_divc(da);
+    d.db = make_divc(db);
+    d.dt = make_divc(sp.dt);
+    if (!sp.fast) {
+        sp.div = d;
+        return d;
+    }
+    FastC f{};
+    f.rdx = d.dx.rb;
+    f.wx = d.dxdx.rb;
+    f.wa = dim == 3 ? d.dada.rb : 0.;
+    f.wb = d.dbdb.rb;
+    f.w0 = -2. * (f.wx + f.wa + f.wb);
+    f.fx = 0.5 * sp.dt * (d.dx.rb * d.dx.rb);
+    f.fa = 0.5 * sp.dt * (d.da.rb * d.da.rb);
+    f.fb = 0.5 * sp.dt * (d.db.rb * d.db.rb);
+    f.gbo = Phys::bmo * sp.gbm1_o;
+    f.gbc = Phys::bmc * sp.gbm1_cr;
+    const double kp = sp.dtL * 2. * Phys::kp, ke = sp.dt_etaL * sp.eta_K;
+    f.px = kp * f.wx; f.pa = kp * f.wa; f.pb = kp * f.wb; f.p0 = -2. * (f.px + f.pa + f.pb);
+    f.ex = ke * f.wx; f.ea = ke * f.wa; f.eb = ke * f.wb; f.e0 = -2. * (f.ex + f.ea + f.eb);
+    f.tS = sp.dt_etaL * 3. * sp.eta_W;
+    f.tH = sp.dt_etaL * (sp.eta_W + sp.eta_A);
+    f.t1 = sp.dt_etaL * sp.eta_W;
+    f.e2 = 2. * f.t1;
+    f.hS = 0.5 * (sp.eta_W + sp.eta_A);
+    f.hH = 0.5 * sp.eta_W;
+    f.x0 = 1922722.2974223055 - (sp.phi_eta ? f.hH : 0.);   // foxide - fmetal at o = cr = 0, and -W/2
+    f.ckO = -Phys::ckO / sp.dt;
+    f.ckCr = -Phys::ckCr / sp.dt;
+    sp.f = f;
+    return d;
+}
 // The whole-domain values of the range fields (every plane, no offset).
 inline void whole_domain_range(StepParams& sp) {
     sp.x_lo = 0;

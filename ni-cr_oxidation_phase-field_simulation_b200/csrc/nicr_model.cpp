@@ -89,19 +89,7 @@ Model::Model(const nicr_config& cfg, const SlabSpec* slab) : c(cfg), dim(cfg.dim
 
     sp.g = g;
     sp.dx = c.dx;
-    sp.da = c.dy;
-    sp.db = dim == 3 ? c.dz : c.dy;
     sp.dt = c.dt;
-    sp.dxdx = c.dx * c.dx;
-    sp.dada = c.dy * c.dy;
-    sp.dbdb = dim == 3 ? c.dz * c.dz : c.dy * c.dy;
-    sp.v_dxdx = make_divc(sp.dxdx);
-    sp.v_dada = make_divc(sp.dada);
-    sp.v_dbdb = make_divc(sp.dbdb);
-    sp.v_dx = make_divc(sp.dx);
-    sp.v_da = make_divc(sp.da);
-    sp.v_db = make_divc(sp.db);
-    sp.v_dt = make_divc(sp.dt);
     sp.dtL = c.dt * Phys::L;
     sp.layer_o = c.layer_o;
     sp.gbm1_o = c.gb_factor_o - 1.;
@@ -124,6 +112,7 @@ Model::Model(const nicr_config& cfg, const SlabSpec* slab) : c(cfg), dim(cfg.dim
     if (c.precision != NICR_FP64 && c.precision != NICR_FP64_FAST)
         throw Error(NICR_ERR_INVALID_ARG, "precision must be NICR_FP64 or NICR_FP64_FAST");
     sp.fast = c.precision == NICR_FP64_FAST ? 1 : 0;
+    div = fill_form_constants(sp, dim, c.dx, c.dy, dim == 3 ? c.dz : c.dy);
     whole_domain_range(sp);
     if (is_slab) {
         sp.x_lo = hlo;
@@ -721,7 +710,9 @@ void Model::refresh() {
         muO = dalloc(ns); muCr = dalloc(ns); mo = dalloc(ns); mc = dalloc(ns);
     }
     const size_t e = prof_begin();
-    launch_refresh(sp, o_[cur], cr_[cur], p_[cur], gb_[gcur], muO, muCr, mo, mc, stream);
+    StepParams rp = sp;   // mu and M at rest are the drop-in form's in both forms
+    rp.div = div;
+    launch_refresh(rp, o_[cur], cr_[cur], p_[cur], gb_[gcur], muO, muCr, mo, mc, stream);
     prof_end(K_REFRESH, e, 1);
     check_cuda(cudaGetLastError(), "refresh");
 }
@@ -1305,7 +1296,7 @@ void Model::grain_stats(nicr_grain_stats* out, long long* cells, double* amount)
     G.g.nstore = g.nstore;
     G.dim = dim; G.neta = neta;
     G.dx = c.dx; G.da = c.dy; G.db = dim == 3 ? c.dz : c.dy;
-    G.v_dx = sp.v_dx; G.v_da = sp.v_da; G.v_db = sp.v_db;
+    G.v_dx = div.dx; G.v_da = div.da; G.v_db = div.db;
     G.K = ec.K; G.W = c.eta_W; G.A = ec.A;
     G.pairs = pairs;
     G.x_above = x_off + sp.x_hi < c.nx ? 1 : 0;

@@ -211,6 +211,7 @@ private:
     int slab_launch();
     void slab_commit(int nblocks, const SlabPeers& peers);
     StepParams sp{};
+    DivSet div{};                     // exact divisions by the run constants (refresh, statistics)
     size_t dev_bytes = 0;
     // state (ping-pong)
     double* o_[2] = {nullptr, nullptr};

@@ -112,19 +112,7 @@ nicr::StepParams params_for(const nicr_config& c) {
     const bool has_eta = c.grain_evolution && c.grains;
     const EtaCoef ec = eta_coef(c.gb_fwhm_grid, c.dx, c.eta_W, c.eta_kappa, c.eta_oxide_penalty);
     sp.dx = c.dx;
-    sp.da = c.dy;
-    sp.db = dim == 3 ? c.dz : c.dy;
     sp.dt = c.dt;
-    sp.dxdx = c.dx * c.dx;
-    sp.dada = c.dy * c.dy;
-    sp.dbdb = dim == 3 ? c.dz * c.dz : c.dy * c.dy;
-    sp.v_dxdx = make_divc(sp.dxdx);
-    sp.v_dada = make_divc(sp.dada);
-    sp.v_dbdb = make_divc(sp.dbdb);
-    sp.v_dx = make_divc(sp.dx);
-    sp.v_da = make_divc(sp.da);
-    sp.v_db = make_divc(sp.db);
-    sp.v_dt = make_divc(sp.dt);
     sp.dtL = c.dt * Phys::L;
     sp.layer_o = c.layer_o;
     sp.gbm1_o = c.gb_factor_o - 1.;
@@ -144,6 +132,7 @@ nicr::StepParams params_for(const nicr_config& c) {
     sp.phi_eta = has_eta ? 1 : 0;
     sp.inlet = (c.bc == NICR_BC_CONCENTRATION && c.oxygen_diffusion) ? 1 : 0;
     sp.fast = c.precision == NICR_FP64_FAST ? 1 : 0;
+    fill_form_constants(sp, dim, c.dx, c.dy, dim == 3 ? c.dz : c.dy);
     sp.xchunk = choose_xchunk(g);
     whole_domain_range(sp);
     // Longer X chunks mean fewer CTAs; the fields do not depend on the chunk

@@ -250,9 +250,9 @@ __global__ void k_refresh(const StepParams P, const double* __restrict__ o, cons
     auto lapf = [&](const double* a) {
         const double c = a[idx];
         if (DIM == 3)
-            return xdiv((a[ixp] - 2. * c + a[ixm]), P.v_dxdx) + xdiv((a[iap] - 2. * c + a[iam]), P.v_dada)
-                 + xdiv((a[ibp] - 2. * c + a[ibm]), P.v_dbdb);
-        return xdiv((a[ixp] - 2. * c + a[ixm]), P.v_dxdx) + xdiv((a[ibp] - 2. * c + a[ibm]), P.v_dbdb);
+            return xdiv((a[ixp] - 2. * c + a[ixm]), P.div.dxdx) + xdiv((a[iap] - 2. * c + a[iam]), P.div.dada)
+                 + xdiv((a[ibp] - 2. * c + a[ibm]), P.div.dbdb);
+        return xdiv((a[ixp] - 2. * c + a[ixm]), P.div.dxdx) + xdiv((a[ibp] - 2. * c + a[ibm]), P.div.dbdb);
     };
     const double oc = o[idx], cc = cr[idx];
     const double hh = h(p[idx]);

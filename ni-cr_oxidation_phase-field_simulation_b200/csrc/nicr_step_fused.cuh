@@ -280,21 +280,13 @@ struct OnePassStep {
             const CenterVals C = lead(0, s2u, gbu);
             __syncthreads();
             const double muOg = (P.bc == 1 && o_on) ? 2. * P.mu_res - C.muO : C.muO;
-            FxO = dv.dvx(-.5 * (C.mo + C.mo) * (C.muO - muOg));
-            FxCr = dv.dvx(-.5 * (C.mc + C.mc) * (C.muCr - C.muCr));
+            FxO = SK::face_x(dv, C.mo, C.mo, muOg, C.muO);
+            FxCr = SK::face_x(dv, C.mc, C.mc, C.muCr, C.muCr);
             pP = C.p;
             // the x = 0 face of plane 0 and the inlet's budget term, here rather
             // than in the march: left_flux (3S:621-628), the surface-mobility
             // closure of the O face with bc=mu, replaces the ghost face
-            if (P.bc == 1) {
-                double lf = 0.;
-                if (o_on) {
-                    const double mf = mobility(P.surface_c_ref, h(C.p), gbu, Phys::bmo, Phys::boo, P.gbm1_o);
-                    lf = dv.dvx(2. * mf * (P.mu_res - C.muO));
-                }
-                FxO = lf;
-                acc[4] = dd_add(acc[4], dv.dvx(P.dt * lf));
-            }
+            if (P.bc == 1) FxO = SK::surface_face(dv, P, o_on, C, gbu, acc[4]);
             if (P.inlet) acc[4] = dd_add(acc[4], P.layer_o - __ldg(o + (long long)row * g.pb + col));
         } else {
             SK::load_oc(P, o, cr, i0 - 2, oslot(i0 - 2), cslot(i0 - 2), offs);
@@ -311,8 +303,8 @@ struct OnePassStep {
             __syncthreads();
             const CenterVals C = lead(i0, s2u, gbu);
             __syncthreads();
-            FxO = dv.dvx(-.5 * (Pv.mo + C.mo) * (C.muO - Pv.muO));
-            FxCr = dv.dvx(-.5 * (Pv.mc + C.mc) * (C.muCr - Pv.muCr));
+            FxO = SK::face_x(dv, Pv.mo, C.mo, Pv.muO, C.muO);
+            FxCr = SK::face_x(dv, Pv.mc, C.mc, Pv.muCr, C.muCr);
             pP = Pv.p;
         }
         {
@@ -342,6 +334,11 @@ struct OnePassStep {
             } else {
                 if (__syncthreads_or(!ok)) break;
                 wait(x);   // plane nx: the clamped copy of plane nx-1 (the eta +X ghost)
+                // the ghost plane nx is the Neumann copy of plane nx-1, mu and M
+                // included: each thread copies its own point, the only one it reads
+                const int c1 = T::i1(ta, tb), lx = (x & 1) * T::S1 + c1, ux = (u & 1) * T::S1 + c1;
+                pslot(x)[c1] = pslot(u)[c1];
+                smuO[lx] = smuO[ux]; smuCr[lx] = smuCr[ux]; smo[lx] = smo[ux]; smc[lx] = smc[ux];
             }
             {
                 const double* mO = smuO + (u & 1) * T::S1;
@@ -357,87 +354,45 @@ struct OnePassStep {
                 auto cell_of = [&]() { return ((long long)u * g.na + row) * g.nb + col; };
                 // Centre (plane u) and lead (plane x) values are read back from
                 // the staging rings rather than carried in registers across the
-                // iteration (the same doubles; fewer live registers). The ghost
-                // plane nx is the Neumann copy of plane nx-1, mu and M included.
+                // iteration (the same doubles; fewer live registers).
                 CenterVals C, Lv;
                 {
                     const int c2 = T::i2(ta, tb);
-                    C.o = oslot(u)[c2]; C.cr = cslot(u)[c2]; C.p = spu[c1]; C.hh = h(C.p);
+                    C.o = oslot(u)[c2]; C.cr = cslot(u)[c2]; C.p = spu[c1]; C.hh = FAST ? h_fast(C.p) : h(C.p);
                     C.muO = mO[c1]; C.muCr = mC[c1]; C.mo = mo_[c1]; C.mc = mc_[c1];
-                    if (x <= g.nx - 1) {
-                        const int lx = (x & 1) * T::S1 + c1;
-                        Lv.p = pslot(x)[c1];
-                        Lv.muO = smuO[lx]; Lv.muCr = smuCr[lx]; Lv.mo = smo[lx]; Lv.mc = smc[lx];
-                    } else {
-                        Lv = C;
-                    }
+                    const int lx = (x & 1) * T::S1 + c1;
+                    Lv.p = pslot(x)[c1];
+                    Lv.muO = smuO[lx]; Lv.muCr = smuCr[lx]; Lv.mo = smo[lx]; Lv.mc = smc[lx];
                 }
 
-                // fluxes, phi force and Ck (3S:761-811); the trial test and the
-                // clamps below without data-dependent branches (so the scheduler
-                // sees one block); the rare bookkeeping (budget terms of changed
-                // cells, failure keys) is one branch after the stores
+                // fluxes, phi force and Ck (3S:761-811)
                 const typename SK::CoreOut R = SK::cell_core(dv, P, o_on, ck_legacy, true, C, Lv, pP, FxO, FxCr, s2u,
                                                              mO, mC, mo_, mc_, spu, c1, bp, bm, ap, am);
                 const double pp = C.p;
-                double onv = R.onv, crv = R.crv, pnv = R.pnv;
-                const double dO = R.dO, dCr = R.dCr, rightO = R.rightO, rightCr = R.rightCr;
-                const bool nonfinite = !isfinite(onv) || !isfinite(crv) || !isfinite(pnv);
-                double clO = 0., clCr = 0.;
-                bool outside = false;
-                if (bounds_legacy) {
-                    const double oc = sclamp(onv, 0., 1.), ccr = sclamp(crv, 0., 1.);
-                    if (!nonfinite) {
-                        clO = oc - onv;
-                        clCr = ccr - crv;
-                        clipped += (oc != onv || ccr != crv) ? 1 : 0;
-                        onv = oc;
-                        crv = ccr;
-                        pnv = pnv > .99999 ? 1. : pnv;
-                        pnv = pnv < 1.e-5 ? 0. : pnv;
-                    }
-                } else {
-                    outside = !nonfinite && (onv < -1.e-12 || crv < -1.e-12 || onv + crv > 1. + 1.e-12 ||
-                                             pnv < -1.e-12 || pnv > 1. + 1.e-12);
-                }
-                on[gidx] = onv; crn[gidx] = crv; pn[gidx] = pnv;
-                FxO = rightO; FxCr = rightCr;
-                if (nonfinite || outside || dO != 0. || dCr != 0. || clO != 0. || clCr != 0.) {
-                    if (nonfinite || outside)
-                        errkey = min(errkey, (unsigned long long)cell_of() * 4ull + (nonfinite ? 0ull : 1ull));
-                    // adding +-0 to a normalised double-double leaves it unchanged,
-                    // so zero increments are skipped
-                    if (dO != 0.) acc[0] = dd_add(acc[0], dO);
-                    if (dCr != 0.) acc[1] = dd_add(acc[1], dCr);
-                    if (clO != 0.) acc[2] = dd_add(acc[2], clO);
-                    if (clCr != 0.) acc[3] = dd_add(acc[3], clCr);
-                }
+                FxO = R.rightO; FxCr = R.rightCr;
+                SK::finish_cell(R, bounds_legacy, on + gidx, crn + gidx, pn + gidx, acc, clipped, errkey, cell_of);
 
-                // eta_trial (3S:514-526) at plane u: v = eta - (dt L_eta)(deta - K lap eta);
-                // the fields failing the range test are collected as bits and keyed
-                // once (the first field in reference order)
+                // eta_trial (3S:514-526) at plane u; a failing cell is keyed once, by its
+                // first failing field in reference order
                 {
                     const double* es = eslot(u);
                     const double* en = eslot(u + 1);
                     double* edst = eta_next + gidx;
-                    unsigned ebad = 0;
+                    const EtaTrial<3, typename DivOf<DM>::T> trial(dv, P, s2u, C.p);
+                    bool in_range = true;
 #pragma unroll
                     for (int q = 0; q < N; ++q) {
                         const int fq = q * L::FS;
                         const double c0 = es[e_own + fq];
-                        const double lap = dv.dvxx((en[e_own + fq] - 2. * c0 + ep[q]))
-                                         + dv.dvaa((es[ap_o + fq] - 2. * c0 + es[am_o + fq]))
-                                         + dv.dvbb((es[bp_o + fq] - 2. * c0 + es[bm_o + fq]));
-                        const double force = grain_deta(c0, s2u, C.p, P.eta_W, P.eta_A) - P.eta_K * lap;
-                        const double v = c0 - P.dt_etaL * force;
-                        ebad |= (!isfinite(v) || v < -1.e-12 || v > 1. + 1.e-12) ? (1u << q) : 0u;
+                        const double v = trial(c0, ep[q], en[e_own + fq], es[am_o + fq], es[ap_o + fq], es[bm_o + fq],
+                                               es[bp_o + fq]);
+                        in_range = in_range && eta_in_range(v);
                         *edst = v;
                         edst += g.nstore;
                         ep[q] = c0;
                     }
-                    if (ebad)
-                        errkey = min(errkey, ERR_ETA_BASE + (unsigned long long)(__ffs(ebad) - 1) *
-                                                 (unsigned long long)g.ncells + (unsigned long long)cell_of());
+                    if (!in_range)
+                        errkey = min(errkey, eta_fail_key(eta_next + gidx, N, g.nstore, g.ncells, cell_of()));
                 }
 
                 pP = pp;   // a register: the ring slot of plane u-1 takes plane u+2 next

@@ -88,61 +88,100 @@ struct Tile {
     __device__ static int i1(int a, int b) { return (a + HA1) * RB1 + (b + 1); }
 };
 
-// Division by a run constant in the two arithmetic forms: FAST=false is the
-// drop-in (xdiv: the correctly rounded quotient, bit-identical to a / b);
-// FAST=true multiplies by RN(1/b) (within one ulp of a / b).
-template <bool FAST>
-__device__ __forceinline__ double fdiv(double a, const DivC& d) {
-    if (FAST) return __dmul_rn(a, d.rb);
-    return xdiv(a, d);
-}
-
 // Divisions of the cell arithmetic, as policies the shared arithmetic (lead
-// points, cell updates) is written against. DivRun<true>: the reciprocal form.
-// DivRun<false>: the exact quotient (xdiv_flag), raising `bad` for the rare
-// quotients it cannot certify (subnormal, infinite or NaN, or a divisor out of
-// range) instead of branching, so the march carries no branch or call per
-// division; a CTA (or thread) that raised it marches again with DivExact
-// before it publishes anything, so every result is still the IEEE quotient.
-template <bool FAST>
+// points, cell updates) is written against. Reciprocal (kFast): no divisions;
+// that form's expressions use the folded constants of FastC. DivRun: the exact
+// quotient (xdiv_flag), raising `bad` for the rare quotients it cannot certify
+// (subnormal, infinite or NaN, or a divisor out of range) instead of
+// branching, so the march carries no branch or call per division; a CTA (or
+// thread) that raised it marches again with DivExact before it publishes
+// anything, so every result is still the IEEE quotient.
+struct Reciprocal {
+    static constexpr bool kFast = true;
+    const StepParams& P;
+    unsigned& bad;   // never raised
+};
 struct DivRun {
+    static constexpr bool kFast = false;
     const StepParams& P;
     unsigned& bad;
-    __device__ double q(double v, const DivC& d) const {
-        if (FAST) return v * d.rb;   // contracted into neighbouring adds where it can
-        return xdiv_flag(v, d, bad);
-    }
-    __device__ double dvx(double v) const { return q(v, P.v_dx); }
-    __device__ double dva(double v) const { return q(v, P.v_da); }
-    __device__ double dvb(double v) const { return q(v, P.v_db); }
-    __device__ double dvxx(double v) const { return q(v, P.v_dxdx); }
-    __device__ double dvaa(double v) const { return q(v, P.v_dada); }
-    __device__ double dvbb(double v) const { return q(v, P.v_dbdb); }
-    __device__ double dvt(double v) const { return q(v, P.v_dt); }
+    __device__ double q(double v, const DivC& d) const { return xdiv_flag(v, d, bad); }
+    __device__ double dvx(double v) const { return q(v, P.div.dx); }
+    __device__ double dva(double v) const { return q(v, P.div.da); }
+    __device__ double dvb(double v) const { return q(v, P.div.db); }
+    __device__ double dvxx(double v) const { return q(v, P.div.dxdx); }
+    __device__ double dvaa(double v) const { return q(v, P.div.dada); }
+    __device__ double dvbb(double v) const { return q(v, P.div.dbdb); }
+    __device__ double dvt(double v) const { return q(v, P.div.dt); }
 };
 // exact for every numerator: xdiv, with the IEEE division (an out-of-line
 // call) for numerators outside the guarded range
 struct DivExact {
+    static constexpr bool kFast = false;
     const StepParams& P;
     unsigned& bad;   // unused: every result is exact
-    __device__ double dvx(double v) const { return xdiv(v, P.v_dx); }
-    __device__ double dva(double v) const { return xdiv(v, P.v_da); }
-    __device__ double dvb(double v) const { return xdiv(v, P.v_db); }
-    __device__ double dvxx(double v) const { return xdiv(v, P.v_dxdx); }
-    __device__ double dvaa(double v) const { return xdiv(v, P.v_dada); }
-    __device__ double dvbb(double v) const { return xdiv(v, P.v_dbdb); }
-    __device__ double dvt(double v) const { return xdiv(v, P.v_dt); }
+    __device__ double dvx(double v) const { return xdiv(v, P.div.dx); }
+    __device__ double dva(double v) const { return xdiv(v, P.div.da); }
+    __device__ double dvb(double v) const { return xdiv(v, P.div.db); }
+    __device__ double dvxx(double v) const { return xdiv(v, P.div.dxdx); }
+    __device__ double dvaa(double v) const { return xdiv(v, P.div.dada); }
+    __device__ double dvbb(double v) const { return xdiv(v, P.div.dbdb); }
+    __device__ double dvt(double v) const { return xdiv(v, P.div.dt); }
 };
 // The policy of a march pass: 0 the reciprocal form; 1 the drop-in form's
 // first pass (exact quotients, out-of-range numerators flagged); 2 the drop-in
 // form's recomputation of a CTA whose first pass raised the flag.
 template <int DM> struct DivOf;
-template <> struct DivOf<0> { using T = DivRun<true>; };
-template <> struct DivOf<1> { using T = DivRun<false>; };
+template <> struct DivOf<0> { using T = Reciprocal; };
+template <> struct DivOf<1> { using T = DivRun; };
 template <> struct DivOf<2> { using T = DivExact; };
 // The error word a launch with parameters P reports its first failing trial to.
 __device__ __forceinline__ unsigned long long* err_word(const StepParams& P, Status* st) {
     return P.err_slot < 0 ? &st->err_key : &st->slot_err[P.err_slot];
+}
+
+// eta_trial's range test (3S:514-526); NaN fails it.
+__device__ __forceinline__ bool eta_in_range(double v) { return v >= -1.e-12 && v <= 1. + 1.e-12; }
+
+// eta_trial of one field at one cell: v = eta - (dt L_eta)(deta - K lap eta),
+// from the centre c, its X neighbours (m: lower, p: upper) and its row (a) and
+// column (b) neighbours. cell() gives what all fields of a cell share.
+// Reciprocal form: the increment is c (T - 2 W' c^2) - K' lap c with dt L_eta
+// folded into T, W' and the weights K' of the neighbour sums, 11 operations
+// instead of 21; the sum c + ... is rounded once, as before.
+template <int DIM, class Dv>
+struct EtaTrial {
+    const Dv& dv;
+    const StepParams& P;
+    double S, phi, T;
+    __device__ EtaTrial(const Dv& d, const StepParams& p, double s, double ph) : dv(d), P(p), S(s), phi(ph), T(0.) {
+        if constexpr (Dv::kFast) T = fma(p.f.tS, s, fma(p.f.tH, h_fast(ph), -p.f.t1));
+    }
+    __device__ double operator()(double c, double xm, double xp, double am, double ap, double bm, double bp) const {
+        if constexpr (Dv::kFast) {
+            const FastC& f = P.f;
+            double l = fma(f.e0, c, f.eb * (bp + bm));
+            if (DIM == 3) l = fma(f.ea, ap + am, l);
+            l = fma(f.ex, xp + xm, l);
+            return c - fma(c, fma(-f.e2, c * c, T), -l);
+        } else {
+            double lap;
+            if (DIM == 3)
+                lap = dv.dvxx((xp - 2. * c + xm)) + dv.dvaa((ap - 2. * c + am)) + dv.dvbb((bp - 2. * c + bm));
+            else
+                lap = dv.dvxx((xp - 2. * c + xm)) + dv.dvbb((bp - 2. * c + bm));
+            const double force = grain_deta(c, S, phi, P.eta_W, P.eta_A) - P.eta_K * lap;
+            return c - P.dt_etaL * force;
+        }
+    }
+};
+// The key of the first of n fields (in reference order) whose trial at idx, already stored, fails the range test.
+__device__ __forceinline__ unsigned long long eta_fail_key(const double* eta_next, int n, long long nstore,
+                                                           long long key_ncells, long long cell) {
+    for (int q = 0; q < n; ++q)
+        if (!eta_in_range(eta_next[(long long)q * nstore]))
+            return ERR_ETA_BASE + (unsigned long long)q * (unsigned long long)key_ncells + (unsigned long long)cell;
+    return ERR_NONE;
 }
 
 struct CenterVals {
@@ -283,29 +322,58 @@ struct StepKernel {
                                            const double* so0, const double* sop, const double* scm, const double* sc0,
                                            const double* scp, const double* sp, double* smuO, double* smuCr,
                                            double* smo, double* smc, int a, int b, double gbv) {
-        const int c2 = T::i2(a, b);
+        const int c2 = T::i2(a, b), c1 = T::i1(a, b);
         const double oc = so0[c2], cc = sc0[c2];
-        double lapO, lapC;
-        if (DIM == 3) {
-            lapO = dv.dvxx((sop[c2] - 2. * oc + som[c2]))
-                 + dv.dvaa((so0[T::i2(a + 1, b)] - 2. * oc + so0[T::i2(a - 1, b)]))
-                 + dv.dvbb((so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)]));
-            lapC = dv.dvxx((scp[c2] - 2. * cc + scm[c2]))
-                 + dv.dvaa((sc0[T::i2(a + 1, b)] - 2. * cc + sc0[T::i2(a - 1, b)]))
-                 + dv.dvbb((sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)]));
-        } else {
-            lapO = dv.dvxx((sop[c2] - 2. * oc + som[c2])) + dv.dvbb((so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)]));
-            lapC = dv.dvxx((scp[c2] - 2. * cc + scm[c2])) + dv.dvbb((sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)]));
-        }
-        const int c1 = T::i1(a, b);
         const double pc = sp[c1];
-        const double hh = h(pc);
         CenterVals v;
-        v.o = oc; v.cr = cc; v.p = pc; v.hh = hh;
-        v.muO = mu_o_local(oc, cc, hh) - 2. * Phys::ko * lapO;
-        v.muCr = mu_cr_local(oc, cc, hh) - 2. * Phys::kc * lapC;
-        v.mo = o_on ? mobility(oc, hh, gbv, Phys::bmo, Phys::boo, k.gbm1_o) : 0.;
-        v.mc = mobility(cc, hh, gbv, Phys::bmc, Phys::boc, k.gbm1_cr);
+        v.o = oc; v.cr = cc; v.p = pc;
+        if constexpr (Dv::kFast) {
+            // mu = (1-h) A + h B - 2 k lap with the inner sums as chained
+            // multiply-adds (no further from 80-bit values than the separate
+            // operations), the mobility's bulk factor folded with the GB
+            // enhancement; second differences, not weighted neighbour sums, so
+            // that mu of a uniform composition carries no rounding of 2 k / dx^2
+            const FastC& f = k.f;
+            const double hh = h_fast(pc);
+            v.hh = hh;
+            auto second = [](double m, double c, double p) { return fma(-2., c, p + m); };
+            double lapO = f.wb * second(so0[T::i2(a, b - 1)], oc, so0[T::i2(a, b + 1)]);
+            double lapC = f.wb * second(sc0[T::i2(a, b - 1)], cc, sc0[T::i2(a, b + 1)]);
+            if (DIM == 3) {
+                lapO = fma(f.wa, second(so0[T::i2(a - 1, b)], oc, so0[T::i2(a + 1, b)]), lapO);
+                lapC = fma(f.wa, second(sc0[T::i2(a - 1, b)], cc, sc0[T::i2(a + 1, b)]), lapC);
+            }
+            lapO = fma(f.wx, second(som[c2], oc, sop[c2]), lapO);
+            lapC = fma(f.wx, second(scm[c2], cc, scp[c2]), lapC);
+            const double ao = fma(12000000., oc, fma(3200000., cc, -298432.));
+            const double ac = fma(1166528.60789006, cc, fma(3200000., oc, -97045.64));
+            const double bo = fma(24000000., oc, fma(-13800000., cc, -8880000.));
+            const double bc = fma(14000000., cc, fma(-13800000., oc, 2680000.));
+            v.muO = fma(-2. * Phys::ko, lapO, fma(hh, bo, (1. - hh) * ao));
+            v.muCr = fma(-2. * Phys::kc, lapC, fma(hh, bc, (1. - hh) * ac));
+            const double mbo = fma(f.gbo, gbv, Phys::bmo), mbc = fma(f.gbc, gbv, Phys::bmc);
+            v.mo = o_on ? oc * fma(hh, Phys::boo - mbo, mbo) : 0.;
+            v.mc = cc * fma(hh, Phys::boc - mbc, mbc);
+        } else {
+            double lapO, lapC;
+            if (DIM == 3) {
+                lapO = dv.dvxx((sop[c2] - 2. * oc + som[c2]))
+                     + dv.dvaa((so0[T::i2(a + 1, b)] - 2. * oc + so0[T::i2(a - 1, b)]))
+                     + dv.dvbb((so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)]));
+                lapC = dv.dvxx((scp[c2] - 2. * cc + scm[c2]))
+                     + dv.dvaa((sc0[T::i2(a + 1, b)] - 2. * cc + sc0[T::i2(a - 1, b)]))
+                     + dv.dvbb((sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)]));
+            } else {
+                lapO = dv.dvxx((sop[c2] - 2. * oc + som[c2])) + dv.dvbb((so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)]));
+                lapC = dv.dvxx((scp[c2] - 2. * cc + scm[c2])) + dv.dvbb((sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)]));
+            }
+            const double hh = h(pc);
+            v.hh = hh;
+            v.muO = mu_o_local(oc, cc, hh) - 2. * Phys::ko * lapO;
+            v.muCr = mu_cr_local(oc, cc, hh) - 2. * Phys::kc * lapC;
+            v.mo = o_on ? mobility(oc, hh, gbv, Phys::bmo, Phys::boo, k.gbm1_o) : 0.;
+            v.mc = mobility(cc, hh, gbv, Phys::bmc, Phys::boc, k.gbm1_cr);
+        }
         smuO[c1] = v.muO; smuCr[c1] = v.muCr; smo[c1] = v.mo; smc[c1] = v.mc;
         return v;
     }
@@ -322,6 +390,48 @@ struct StepKernel {
                                         const double* mo_, const double* mc_, const double* spu, int c1, int bp,
                                         int bm, int ap, int am) {
         CoreOut r;
+        if constexpr (Dv::kFast) {
+            // faces without their factor -1/(2 dx): the carried X face too (face_x)
+            const FastC& f = k.f;
+            r.rightO = (C.mo + L.mo) * (L.muO - C.muO);
+            r.rightCr = (C.mc + L.mc) * (L.muCr - C.muCr);
+            const double oo = C.o, cc = C.cr, pp = C.p, hh = C.hh;
+            double onv = oo, crv;
+            {
+                const double m0 = mc_[c1], mu0 = mC[c1];
+                double t = f.fb * fma(m0 + mc_[bp], mC[bp] - mu0, (mc_[bm] + m0) * (mC[bm] - mu0));
+                if (DIM == 3) t = fma(f.fa, fma(m0 + mc_[ap], mC[ap] - mu0, (mc_[am] + m0) * (mC[am] - mu0)), t);
+                crv = cc + fma(f.fx, r.rightCr - leftCr, t);
+            }
+            if (o_on) {
+                const double m0 = mo_[c1], mu0 = mO[c1];
+                double t = f.fb * fma(m0 + mo_[bp], mO[bp] - mu0, (mo_[bm] + m0) * (mO[bm] - mu0));
+                if (DIM == 3) t = fma(f.fa, fma(m0 + mo_[ap], mO[ap] - mu0, (mo_[am] + m0) * (mO[am] - mu0)), t);
+                onv = oo + fma(f.fx, r.rightO - leftO, t);
+            }
+            // phi force: p (p-1) [2W (2p-1) + 30 p (p-1) X], X = foxide - fmetal plus half the eta energy's slope
+            const double pq = pp * (pp - 1.);
+            double X = fma(oo, fma(6000000., oo, fma(-17000000., cc, -8581568.)),
+                           fma(cc, fma(6416735.696054969, cc, 2777045.64), f.x0));
+            if (phi_eta) X = fma(s2u, f.hS, fma(f.hH, hh, X));
+            const double G = fma(30. * pq, X, fma(4. * Phys::W, pp, -2. * Phys::W));
+            double l = fma(f.p0, pp, f.pb * (spu[bp] + spu[bm]));
+            if (DIM == 3) l = fma(f.pa, spu[ap] + spu[am], l);
+            l = fma(f.px, L.p + pP, l);
+            r.pnv = pp + fma(-k.dtL * pq, G, l);
+            r.dO = 0.;
+            r.dCr = 0.;
+            if (ck_legacy) {
+                const double hn = h_fast(r.pnv);
+                r.dO = f.ckO * fma(Phys::oxideO - onv, hn, -((Phys::oxideO - oo) * hh));
+                r.dCr = f.ckCr * fma(Phys::oxideCr - crv, hn, -((Phys::oxideCr - cc) * hh));
+                onv += r.dO;
+                crv += r.dCr;
+            }
+            r.onv = onv;
+            r.crv = crv;
+            return r;
+        } else {
         // x faces: the right face of u is the left face of u+1 (same expression)
         r.rightO = dv.dvx(-.5 * (C.mo + L.mo) * (L.muO - C.muO));
         r.rightCr = dv.dvx(-.5 * (C.mc + L.mc) * (L.muCr - C.muCr));
@@ -376,6 +486,85 @@ struct StepKernel {
         r.onv = onv;
         r.crv = crv;
         return r;
+        }
+    }
+    // The trial test and the legacy clamps of one cell (3S:790-811), its stores
+    // (on, crn, pn: the cell's places) and bookkeeping. Cells whose new o and cr
+    // have a high word below 1.0's (in [0, 1), no sign) and a finite phi need
+    // none of the tests: one unsigned comparison instead of ten FP64 ones. All
+    // others, and cells with Ck increments, take the branch after the stores,
+    // which stores again what the clamps change. cell(): the cell's index in
+    // reference loop order.
+    template <class CellFn>
+    __device__ static void finish_cell(const CoreOut& R, bool bounds_legacy, double* on, double* crn, double* pn,
+                                       DD (&acc)[5], long long& clipped, unsigned long long& errkey, CellFn cell) {
+        const unsigned ho = (unsigned)__double2hiint(R.onv), hc = (unsigned)__double2hiint(R.crv),
+                       hp = (unsigned)__double2hiint(R.pnv);
+        double pnv = R.pnv;
+        bool plain;
+        if (bounds_legacy) {
+            plain = max(ho, hc) < 0x3FF00000u && (hp & 0x7FFFFFFFu) < 0x7FF00000u;
+            pnv = pnv > .99999 ? 1. : pnv;
+            pnv = pnv < 1.e-5 ? 0. : pnv;
+        } else {
+            plain = max(ho, hc) < 0x3FE00000u && hp < 0x3FF00000u;   // o, cr < 1/2, phi in [0, 1)
+        }
+        *on = R.onv;
+        *crn = R.crv;
+        *pn = pnv;
+        if (!plain || R.dO != 0. || R.dCr != 0.) {
+            const bool nonfinite = !isfinite(R.onv) || !isfinite(R.crv) || !isfinite(R.pnv);
+            bool outside = false;
+            if (nonfinite) {
+                *pn = R.pnv;
+            } else if (bounds_legacy) {
+                const double oc = sclamp(R.onv, 0., 1.), ccr = sclamp(R.crv, 0., 1.);
+                const double clO = oc - R.onv, clCr = ccr - R.crv;
+                if (oc != R.onv || ccr != R.crv) {
+                    ++clipped;
+                    *on = oc;
+                    *crn = ccr;
+                }
+                // adding +-0 to a normalised double-double leaves it unchanged,
+                // so zero increments are skipped
+                if (clO != 0.) acc[2] = dd_add(acc[2], clO);
+                if (clCr != 0.) acc[3] = dd_add(acc[3], clCr);
+            } else {
+                outside = R.onv < -1.e-12 || R.crv < -1.e-12 || R.onv + R.crv > 1. + 1.e-12 || R.pnv < -1.e-12 ||
+                          R.pnv > 1. + 1.e-12;
+            }
+            if (nonfinite || outside)
+                errkey = min(errkey, (unsigned long long)cell() * 4ull + (nonfinite ? 0ull : 1ull));
+            if (R.dO != 0.) acc[0] = dd_add(acc[0], R.dO);
+            if (R.dCr != 0.) acc[1] = dd_add(acc[1], R.dCr);
+        }
+    }
+    // The X face between two cells as the march carries it: the flux
+    // (exact forms) or, in the reciprocal form, the flux times -2 dx.
+    template <class Dv>
+    __device__ static double face_x(const Dv& dv, double m0, double m1, double mu0, double mu1) {
+        if constexpr (Dv::kFast) return (m0 + m1) * (mu1 - mu0);
+        else return dv.dvx(-.5 * (m0 + m1) * (mu1 - mu0));
+    }
+    // The surface-mobility closure of the O face at X = 0 with bc=mu
+    // (left_flux, 3S:621-628): the carried face, and the budget's increment.
+    template <class Dv>
+    __device__ static double surface_face(const Dv& dv, const StepParams& P, bool o_on, const CenterVals& C, double gb0,
+                                          DD& booked) {
+        double lf = 0., carry = 0., inc;
+        if (o_on) {
+            const double mf = mobility(P.surface_c_ref, h(C.p), gb0, Phys::bmo, Phys::boo, P.gbm1_o);
+            if constexpr (Dv::kFast) {
+                carry = -4. * mf * (P.mu_res - C.muO);
+                lf = (2. * mf * (P.mu_res - C.muO)) * P.f.rdx;
+            } else {
+                lf = carry = dv.dvx(2. * mf * (P.mu_res - C.muO));
+            }
+        }
+        if constexpr (Dv::kFast) inc = (P.dt * lf) * P.f.rdx;
+        else inc = dv.dvx(P.dt * lf);
+        booked = dd_add(booked, inc);
+        return carry;
     }
     // One march over the CTA's chunk with the division policy of DM (DivOf).
     // DM 1 returns true, without publishing its failure keys or budget
@@ -459,8 +648,8 @@ struct StepKernel {
             __syncthreads();
             // ghost plane -1: copies of plane 0 (3S:187, 3S:613-615, 3S:616-619)
             const double muOg = (P.bc == 1 && P.o_on) ? 2. * P.mu_res - C.muO : C.muO;
-            FxO = dv.dvx(-.5 * (C.mo + C.mo) * (C.muO - muOg));
-            FxCr = dv.dvx(-.5 * (C.mc + C.mc) * (C.muCr - C.muCr));
+            FxO = face_x(dv, C.mo, C.mo, muOg, C.muO);
+            FxCr = face_x(dv, C.mc, C.mc, C.muCr, C.muCr);
             pP = C.p;
         } else {
             load_oc(P, o, cr, i0 - 2, oslot(i0 - 2), cslot(i0 - 2), offs);
@@ -478,8 +667,8 @@ struct StepKernel {
             __syncthreads();
             C = lead(i0, gb0);
             __syncthreads();
-            FxO = dv.dvx(-.5 * (Pv.mo + C.mo) * (C.muO - Pv.muO));
-            FxCr = dv.dvx(-.5 * (Pv.mc + C.mc) * (C.muCr - Pv.muCr));
+            FxO = face_x(dv, Pv.mo, C.mo, Pv.muO, C.muO);
+            FxCr = face_x(dv, Pv.mc, C.mc, Pv.muCr, C.muCr);
             pP = Pv.p;
         }
 
@@ -516,59 +705,19 @@ struct StepKernel {
                 const int bp = T::i1(ta, tb + 1), bm = T::i1(ta, tb - 1);
                 const int ap = T::i1(ta + 1, tb), am = T::i1(ta - 1, tb);
                 const long long gidx = (long long)u * g.plane + (long long)row * g.pb + col;
-                const long long cell = ((long long)u * g.na + row) * g.nb + col + (SLAB ? P.cell_off : 0);  // reference loop order
-
                 double leftO = FxO;
                 if (u == 0 && P.bc == 1) {
-                    // left_flux (3S:621-628): surface-mobility face closure for bc=mu
-                    double lf = 0.;
-                    if (P.o_on) {
-                        const double gb0 = P.grains ? __ldg(gb + gidx) : 0.;
-                        const double mf = mobility(P.surface_c_ref, h(C.p), gb0, Phys::bmo, Phys::boo, P.gbm1_o);
-                        lf = dv.dvx(2. * mf * (P.mu_res - C.muO));
-                    }
-                    leftO = lf;
-                    acc[4] = dd_add(acc[4], dv.dvx(P.dt * lf));
+                    leftO = surface_face(dv, P, P.o_on != 0, C, P.grains ? __ldg(gb + gidx) : 0., acc[4]);
                 }
                 if (u == 0 && P.inlet) acc[4] = dd_add(acc[4], P.layer_o - __ldg(o + gidx));
 
-                // fluxes, phi force and Ck (3S:761-811); the trial test and the
-                // clamps below without data-dependent branches (so the scheduler
-                // sees one block); the rare bookkeeping (budget terms of changed
-                // cells, failure keys) is one branch after the stores
+                // fluxes, phi force and Ck (3S:761-811)
                 const CoreOut R = cell_core(dv, P, P.o_on != 0, P.ck == 0, P.phi_eta != 0, C, L, pP, leftO, FxCr,
                                             s2u, mO, mC, mo_, mc_, spu, c1, bp, bm, ap, am);
-                double onv = R.onv, crv = R.crv, pnv = R.pnv;
-                const double dO = R.dO, dCr = R.dCr, rightO = R.rightO, rightCr = R.rightCr;
-                const bool nonfinite = !isfinite(onv) || !isfinite(crv) || !isfinite(pnv);
-                double clO = 0., clCr = 0.;
-                bool outside = false;
-                if (P.bounds == 1) {
-                    const double oc = sclamp(onv, 0., 1.), ccr = sclamp(crv, 0., 1.);
-                    if (!nonfinite) {
-                        clO = oc - onv;
-                        clCr = ccr - crv;
-                        clipped += (oc != onv || ccr != crv) ? 1 : 0;
-                        onv = oc;
-                        crv = ccr;
-                        pnv = pnv > .99999 ? 1. : pnv;
-                        pnv = pnv < 1.e-5 ? 0. : pnv;
-                    }
-                } else {
-                    outside = !nonfinite && (onv < -1.e-12 || crv < -1.e-12 || onv + crv > 1. + 1.e-12 ||
-                                             pnv < -1.e-12 || pnv > 1. + 1.e-12);
-                }
-                on[gidx] = onv; crn[gidx] = crv; pn[gidx] = pnv;
-                FxO = rightO; FxCr = rightCr;
-                if (nonfinite || outside || dO != 0. || dCr != 0. || clO != 0. || clCr != 0.) {
-                    if (nonfinite || outside) errkey = min(errkey, (unsigned long long)cell * 4ull + (nonfinite ? 0ull : 1ull));
-                    // adding +-0 to a normalised double-double leaves it unchanged,
-                    // so zero increments (metal cells: h(pn) == h(p) == 0) are skipped
-                    if (dO != 0.) acc[0] = dd_add(acc[0], dO);
-                    if (dCr != 0.) acc[1] = dd_add(acc[1], dCr);
-                    if (clO != 0.) acc[2] = dd_add(acc[2], clO);
-                    if (clCr != 0.) acc[3] = dd_add(acc[3], clCr);
-                }
+                FxO = R.rightO; FxCr = R.rightCr;
+                finish_cell(R, P.bounds == 1, on + gidx, crn + gidx, pn + gidx, acc, clipped, errkey, [&]() {
+                    return ((long long)u * g.na + row) * g.nb + col + (SLAB ? P.cell_off : 0);
+                });
             }
             pP = C.p;
             C = L;
@@ -673,31 +822,20 @@ __device__ __forceinline__ unsigned eta_cell_pass(const StepParams& P, int neta,
         iam = rbase + (long long)(row == 0 ? g.na - 1 : row - 1) * g.pb + col;
         iap = rbase + (long long)(row == g.na - 1 ? 0 : row + 1) * g.pb + col;
     }
-    const double S = __ldg(s2 + idx), phi = __ldg(p + idx);
+    const EtaTrial<DIM, typename DivOf<DM>::T> trial(dv, P, __ldg(s2 + idx), __ldg(p + idx));
     double Sn = 0., pairs = 0.;
-    int first_bad = -1;   // the first field failing the range test
+    bool in_range = true;
     for (int q = 0; q < neta; ++q) {
         const double* e = eta + (long long)q * g.nstore;
-        const double ec = __ldg(e + idx);
-        double lap;
-        if (DIM == 3)
-            lap = dv.dvxx((__ldg(e + ixp) - 2. * ec + __ldg(e + ixm))) + dv.dvaa((__ldg(e + iap) - 2. * ec + __ldg(e + iam)))
-                + dv.dvbb((__ldg(e + ibp) - 2. * ec + __ldg(e + ibm)));
-        else
-            lap = dv.dvxx((__ldg(e + ixp) - 2. * ec + __ldg(e + ixm))) + dv.dvbb((__ldg(e + ibp) - 2. * ec + __ldg(e + ibm)));
-        const double force = grain_deta(ec, S, phi, P.eta_W, P.eta_A) - P.eta_K * lap;
-        const double v = ec - P.dt_etaL * force;
-        const bool fail = !(v >= -1.e-12 && v <= 1. + 1.e-12);   // NaN fails both comparisons
-        first_bad = (fail && first_bad < 0) ? q : first_bad;
+        const double v = trial(__ldg(e + idx), __ldg(e + ixm), __ldg(e + ixp), __ldg(e + iam), __ldg(e + iap),
+                               __ldg(e + ibm), __ldg(e + ibp));
+        in_range = in_range && eta_in_range(v);
         eta_next[(long long)q * g.nstore + idx] = v;
         const double sq = v * v;
         pairs += Sn * sq;
         Sn += sq;
     }
-    // keyed once per cell: the first failing field in reference order
-    if (first_bad >= 0)
-        errkey = min(errkey, ERR_ETA_BASE + (unsigned long long)first_bad * (unsigned long long)P.key_ncells +
-                                 (unsigned long long)cell);
+    if (!in_range) errkey = min(errkey, eta_fail_key(eta_next + idx, neta, g.nstore, P.key_ncells, cell));
     s2_next[idx] = Sn;
     gb_next[idx] = P.eta_scale * smin(1., 16. * pairs);
     return dbad;
@@ -794,31 +932,24 @@ __device__ __forceinline__ unsigned eta_march_pass(const StepParams& P, int n, c
         for (int q = 0; q < NCAP; ++q)
             if (q < n) S += ec[q] * ec[q];
         const long long cell = ((long long)x * g.na + row) * g.nb + col + (SLAB ? P.cell_off : 0);
+        const EtaTrial<DIM, typename DivOf<DM>::T> trial(dv, P, S, phi);
         double Sn = 0., pairs = 0.;
-        unsigned bad = 0;
+        bool in_range = true;
 #pragma unroll
         for (int q = 0; q < NCAP; ++q) {
             if (q >= n) break;
             const double* e = eta + (long long)q * g.nstore + base;
-            const double c0 = ec[q];
-            double lap;
-            if (DIM == 3)
-                lap = dv.dvxx((en[q] - 2. * c0 + ep[q])) + dv.dvaa((__ldg(e + cap) - 2. * c0 + __ldg(e + cam)))
-                    + dv.dvbb((__ldg(e + cbp) - 2. * c0 + __ldg(e + cbm)));
-            else
-                lap = dv.dvxx((en[q] - 2. * c0 + ep[q])) + dv.dvbb((__ldg(e + cbp) - 2. * c0 + __ldg(e + cbm)));
-            const double force = grain_deta(c0, S, phi, P.eta_W, P.eta_A) - P.eta_K * lap;
-            const double v = c0 - P.dt_etaL * force;
-            bad |= !(v >= -1.e-12 && v <= 1. + 1.e-12) ? (1u << q) : 0u;   // NaN fails both comparisons
+            double am = 0., ap = 0.;
+            if (DIM == 3) { am = __ldg(e + cam); ap = __ldg(e + cap); }
+            const double v = trial(ec[q], ep[q], en[q], am, ap, __ldg(e + cbm), __ldg(e + cbp));
+            in_range = in_range && eta_in_range(v);
             eta_next[(long long)q * g.nstore + base + rc] = v;
             const double sq = v * v;
             pairs += Sn * sq;
             Sn += sq;
         }
-        // fields failing the range test, keyed once (the first in reference order)
-        if (bad)
-            errkey = min(errkey, ERR_ETA_BASE + (unsigned long long)(__ffs(bad) - 1) *
-                                     (unsigned long long)(SLAB ? P.key_ncells : g.ncells) + (unsigned long long)cell);
+        if (!in_range)
+            errkey = min(errkey, eta_fail_key(eta_next + base + rc, n, g.nstore, SLAB ? P.key_ncells : g.ncells, cell));
         s2_next[base + rc] = Sn;
         gb_next[base + rc] = P.eta_scale * smin(1., 16. * pairs);
 #pragma unroll
@@ -1150,6 +1281,10 @@ k_eta_tma(const StepParams P, const __grid_constant__ CUtensorMap m_int, const _
             S2 += v * v;
         }
         const long long cell = ((long long)x * g.na + row) * g.nb + col;
+        unsigned dbad = 0;   // the exact policy divides every quotient exactly
+        using Dv = typename DivOf<FAST ? 0 : 2>::T;
+        const Dv dv{P, dbad};
+        const EtaTrial<3, Dv> trial(dv, P, S2, phi);
         double Sn = 0., pairs = 0.;
 #pragma unroll
         for (int q = 0; q < N; ++q) {
@@ -1159,12 +1294,8 @@ k_eta_tma(const StepParams P, const __grid_constant__ CUtensorMap m_int, const _
             const double ap = ta == TA - 1 ? bot[q * TB + tb] : s0[o + c + TB];
             const double bm = tb == 0 ? lft[(q * TA + ta) * 2 + 1] : s0[o + c - 1];
             const double bp = tb == TB - 1 ? rgt[(q * TA + ta) * 2] : s0[o + c + 1];
-            const double lap = fdiv<FAST>((sp[o + c] - 2. * c0 + sm[o + c]), P.v_dxdx)
-                             + fdiv<FAST>((ap - 2. * c0 + am), P.v_dada)
-                             + fdiv<FAST>((bp - 2. * c0 + bm), P.v_dbdb);
-            const double force = grain_deta(c0, S2, phi, P.eta_W, P.eta_A) - P.eta_K * lap;
-            const double v = c0 - P.dt_etaL * force;
-            if (!isfinite(v) || v < -1.e-12 || v > 1. + 1.e-12)
+            const double v = trial(c0, sm[o + c], sp[o + c], am, ap, bm, bp);
+            if (!eta_in_range(v))
                 errkey = min(errkey, ERR_ETA_BASE + (unsigned long long)q * (unsigned long long)g.ncells + (unsigned long long)cell);
             eta_next[(long long)q * g.nstore + base + own] = v;
             const double sq = v * v;
@@ -1312,22 +1443,15 @@ k_eta_stream(const StepParams P, int neta, const double* __restrict__ eta, const
                 const double v = s0[e * S1 + c1];
                 S += v * v;
             }
-            const double phi = __ldg(p + idx);
+            unsigned dbad = 0;   // the exact policy divides every quotient exactly
+            using Dv = typename DivOf<FAST ? 0 : 2>::T;
+            const Dv dv{P, dbad};
+            const EtaTrial<DIM, Dv> trial(dv, P, S, __ldg(p + idx));
             double Sn = 0., pairs = 0.;
             for (int e = 0; e < neta; ++e) {
                 const int o = e * S1;
-                const double ec = s0[o + c1];
-                double lap;
-                if (DIM == 3)
-                    lap = fdiv<FAST>((sp[o + c1] - 2. * ec + sm[o + c1]), P.v_dxdx)
-                        + fdiv<FAST>((s0[o + ap] - 2. * ec + s0[o + am]), P.v_dada)
-                        + fdiv<FAST>((s0[o + bp] - 2. * ec + s0[o + bm]), P.v_dbdb);
-                else
-                    lap = fdiv<FAST>((sp[o + c1] - 2. * ec + sm[o + c1]), P.v_dxdx)
-                        + fdiv<FAST>((s0[o + bp] - 2. * ec + s0[o + bm]), P.v_dbdb);
-                const double force = grain_deta(ec, S, phi, P.eta_W, P.eta_A) - P.eta_K * lap;
-                const double v = ec - P.dt_etaL * force;
-                if (!isfinite(v) || v < -1.e-12 || v > 1. + 1.e-12)
+                const double v = trial(s0[o + c1], sm[o + c1], sp[o + c1], s0[o + am], s0[o + ap], s0[o + bm], s0[o + bp]);
+                if (!eta_in_range(v))
                     errkey = min(errkey, ERR_ETA_BASE + (unsigned long long)e * (unsigned long long)g.ncells + (unsigned long long)cell);
                 eta_next[(long long)e * g.nstore + idx] = v;
                 const double sq = v * v;
