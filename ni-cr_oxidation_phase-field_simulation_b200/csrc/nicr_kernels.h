@@ -80,6 +80,7 @@ struct FastC {
 struct StepParams {
     Grid g;
     double dx, dt;               // spacing along X
+    double dt_s, etaK_s;         // 2^-128 dt and 2^-128 eta_K (after scaled quotients)
     union {                      // by form: the other form's constants are not needed
         DivSet div;              // fast == 0
         FastC f;                 // fast == 1
@@ -105,7 +106,10 @@ struct StepParams {
     // offset by cell_off and eta keys count key_ncells cells per field.
     long long cell_off, key_ncells;
     // Error word of this step: -1 st->err_key, 0/1 st->slot_err[err_slot] (slab form)
-    int err_slot, pad_;
+    int err_slot;
+    // drop-in form: 1 when a divisor or a constant after a scaled quotient
+    // lies outside the certified range, so every chunk is divided by IEEE division
+    unsigned div_gate;
 };
 // The run constants of the configured form (spacings along X, rows, columns);
 // the other scalar members of sp are set already. Returns the exact divisions,
@@ -121,6 +125,10 @@ inline DivSet fill_form_constants(StepParams& sp, int dim, double dx, double da,
     d.dt = make_divc(sp.dt);
     if (!sp.fast) {
         sp.div = d;
+        sp.dt_s = std::ldexp(sp.dt, -128);
+        sp.etaK_s = std::ldexp(sp.eta_K, -128);
+        const bool k_ok = sp.eta_K == 0. || (std::fabs(sp.eta_K) >= std::ldexp(1., -500) && std::fabs(sp.eta_K) <= std::ldexp(1., 500));
+        sp.div_gate = d.dxdx.gate | d.dada.gate | d.dbdb.gate | d.dx.gate | d.da.gate | d.db.gate | d.dt.gate | (k_ok ? 0u : 1u);
         return d;
     }
     FastC f{};

@@ -97,10 +97,10 @@ inline EtaCoef eta_coef(double fwhm, double dx, double W, double kappa, double p
 // The host stores y = RN(1/b) and the double-word reciprocal zh = RD(1/b),
 // zl = RN(1/b - zh) >= 0 (Brisebarre, Muller, Raina, "Accelerating correctly
 // rounded floating-point division when the divisor is known in advance",
-// IEEE Trans. Comput. 53(8), 2004), the latter two scaled by 2^128. For b > 0
-// with 2^-60 <= b <= 2^60 and a numerator a:
+// IEEE Trans. Comput. 53(8), 2004). For b > 0 with 2^-60 <= b <= 2^60 and a
+// numerator a:
 //   as = a * 2^128                  exact for |a| < 2^895, subnormals included,
-//   q0 = RN(a*zh' + RN(a*zl'))      within (1/2 + 2^-51) ulp of as/b,
+//   q0 = RN(as*zh + RN(as*zl))      within (1/2 + 2^-51) ulp of as/b,
 //   e  = q0*b - as                  exact: q0 is within one ulp of as/b, and
 //                                   as/b >= 2^-1006 keeps its bits normal,
 //   qs = RN(q0 - e*y)               = RN(as/b), Markstein's correction theorem
@@ -114,10 +114,13 @@ inline EtaCoef eta_coef(double fwhm, double dx, double W, double kappa, double p
 // final scaling would round a second time), infinite or NaN (infinite, NaN or
 // huge numerators), or any quotient of a divisor outside the range, is
 // flagged. tests/division_check.c restates this on the host and checks it
-// against IEEE division, near-midpoint quotients included.
+// against IEEE division, near-midpoint quotients included. Sums and products
+// of scaled quotients round as the unscaled ones do (a power of two, and sums
+// that reach the subnormal range are exact), so the kernels keep quotients
+// scaled through a sum and fold 2^-128 into the constant that follows it.
 struct DivC {
     double b, rb;      // divisor and y = RN(1/b) (the reciprocal form multiplies by it)
-    double zh, zl;     // 2^128 RD(1/b) and 2^128 RN(1/b - RD(1/b))
+    double zh, zl;     // RD(1/b) and RN(1/b - RD(1/b))
     unsigned gate;     // 0 when b is in range, else 1 (every quotient flagged)
     unsigned pad;
 };
@@ -131,8 +134,8 @@ inline DivC make_divc(double b) {
         zh = std::nextafter(zh, 0.0);
         rem = std::fma(-zh, b, 1.0);
     }
-    d.zh = std::ldexp(zh, 128);
-    d.zl = std::ldexp(rem / b, 128);
+    d.zh = zh;
+    d.zl = rem / b;
     const bool in_range = std::isnormal(b) && b > 0. && b >= std::ldexp(1.0, -60) && b <= std::ldexp(1.0, 60);
     d.gate = in_range ? 0u : 1u;
     d.pad = 0;
@@ -145,11 +148,14 @@ __device__ __noinline__ double ieee_div(double a, double b);
 // The exact quotient; a flagged one (see DivC) sets `bad` (the value returned
 // for it is then not the IEEE quotient), so a caller can test once for a
 // whole group of divisions and recompute the group with IEEE division.
-__device__ __forceinline__ double xdiv_flag(double a, const DivC& d, unsigned& bad) {
-    const double as = __dmul_rn(a, 0x1p128);
-    const double q0 = __fma_rn(a, d.zh, __dmul_rn(a, d.zl));
+// the scaled quotient of a scaled numerator (uncertified)
+__device__ __forceinline__ double xdiv_scaled(double as, const DivC& d) {
+    const double q0 = __fma_rn(as, d.zh, __dmul_rn(as, d.zl));
     const double e = __fma_rn(q0, d.b, -as);
-    const double qs = __fma_rn(-e, d.rb, q0);
+    return __fma_rn(-e, d.rb, q0);
+}
+__device__ __forceinline__ double xdiv_flag(double a, const DivC& d, unsigned& bad) {
+    const double qs = xdiv_scaled(__dmul_rn(a, 0x1p128), d);
     // |qs| in (0, 2^-894): a subnormal quotient; >= 2^1024: infinite or NaN
     const unsigned u = (unsigned)__double2hiint(qs) & 0x7FFFFFFFu;
     bad |= ((u - 1u) < 0x080FFFFFu || u >= 0x7FF00000u || d.gate) ? 1u : 0u;

@@ -158,8 +158,8 @@ struct OnePassStep {
             fused_smem + L::STEP_BYTES + ((128u - (smem_u32(fused_smem + L::STEP_BYTES) & 127u)) & 127u));
 
         if (st->failed) return false;   // a previous step of this batch was rejected
-        unsigned dbad = 0;
-        const typename DivOf<DM>::T dv{P, dbad};
+        unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+        const typename DivOf<DM>::T dv{P, low};
 
         const bool o_on = MODE == 1 ? true : P.o_on != 0;
         const bool ck_legacy = MODE == 1 ? true : P.ck == 0;
@@ -416,7 +416,7 @@ struct OnePassStep {
             __syncthreads();
             return false;
         }
-        if (DM == 1 && __syncthreads_or(dbad != 0)) return true;
+        if (DM == 1 && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
         if (errkey != ERR_NONE) atomicMin(&st->err_key, errkey);
         block_reduce_dd<5>(acc, clipped, sdd, scnt);
         if (tid == 0) {

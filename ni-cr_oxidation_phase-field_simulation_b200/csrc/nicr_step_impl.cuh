@@ -90,43 +90,60 @@ struct Tile {
 
 // Divisions of the cell arithmetic, as policies the shared arithmetic (lead
 // points, cell updates) is written against. Reciprocal (kFast): no divisions;
-// that form's expressions use the folded constants of FastC. DivRun: the exact
-// quotient (xdiv_flag), raising `bad` for the rare quotients it cannot certify
-// (subnormal, infinite or NaN, or a divisor out of range) instead of
-// branching, so the march carries no branch or call per division; a CTA (or
-// thread) that raised it marches again with DivExact before it publishes
+// that form's expressions use the folded constants of FastC. The exact
+// policies return quotients in a carried scale 1/S: up() from an unscaled
+// numerator, same() from one in the carried scale, plain() unscaled from
+// unscaled; the caller folds S into the constant that multiplies a sum.
+//
+// DivRun: quotients carried times 2^128 (xdiv_scaled), so a Laplacian's three
+// quotients and the faces of a divergence are never scaled back (4 to 6 FP64
+// operations per division instead of 6). It keeps in `low` the smallest
+// 2 * (high word) - 1 of the quotients (zero wraps to the largest), from which
+// one comparison at the end of the march tells whether any nonzero quotient
+// was subnormal (two integer operations per division instead of five).
+// Infinite and NaN quotients reach a trial value and fail its test. A CTA (or
+// thread) that saw either marches again with DivExact before it publishes
 // anything, so every result is still the IEEE quotient.
+constexpr unsigned kLowQuotient = 0x101FFFFDu;   // 2 * 0x080FFFFF - 1: scaled quotients below 2^-894
 struct Reciprocal {
     static constexpr bool kFast = true;
     const StepParams& P;
-    unsigned& bad;   // never raised
+    unsigned& low;   // unused
 };
 struct DivRun {
     static constexpr bool kFast = false;
+    static constexpr double S = 0x1p-128;
     const StepParams& P;
-    unsigned& bad;
-    __device__ double q(double v, const DivC& d) const { return xdiv_flag(v, d, bad); }
-    __device__ double dvx(double v) const { return q(v, P.div.dx); }
-    __device__ double dva(double v) const { return q(v, P.div.da); }
-    __device__ double dvb(double v) const { return q(v, P.div.db); }
-    __device__ double dvxx(double v) const { return q(v, P.div.dxdx); }
-    __device__ double dvaa(double v) const { return q(v, P.div.dada); }
-    __device__ double dvbb(double v) const { return q(v, P.div.dbdb); }
-    __device__ double dvt(double v) const { return q(v, P.div.dt); }
+    unsigned& low;
+    __device__ double same(double as, const DivC& d) const {
+        const double qs = xdiv_scaled(as, d);
+        low = min(low, 2u * (unsigned)__double2hiint(qs) - 1u);
+        return qs;
+    }
+    __device__ double up(double a, const DivC& d) const { return same(__dmul_rn(a, 0x1p128), d); }
+    __device__ double plain(double a, const DivC& d) const { return __dmul_rn(up(a, d), 0x1p-128); }
+    // a quotient that no trial value depends on: infinite and NaN are noted here
+    __device__ double plain_checked(double a, const DivC& d) const {
+        const double q = plain(a, d);
+        if (!isfinite(q)) low = 0;
+        return q;
+    }
+    __device__ double dt() const { return P.dt_s; }
+    __device__ double etaK() const { return P.etaK_s; }
 };
 // exact for every numerator: xdiv, with the IEEE division (an out-of-line
-// call) for numerators outside the guarded range
+// call) for numerators outside the guarded range; nothing is scaled
 struct DivExact {
     static constexpr bool kFast = false;
+    static constexpr double S = 1.;
     const StepParams& P;
-    unsigned& bad;   // unused: every result is exact
-    __device__ double dvx(double v) const { return xdiv(v, P.div.dx); }
-    __device__ double dva(double v) const { return xdiv(v, P.div.da); }
-    __device__ double dvb(double v) const { return xdiv(v, P.div.db); }
-    __device__ double dvxx(double v) const { return xdiv(v, P.div.dxdx); }
-    __device__ double dvaa(double v) const { return xdiv(v, P.div.dada); }
-    __device__ double dvbb(double v) const { return xdiv(v, P.div.dbdb); }
-    __device__ double dvt(double v) const { return xdiv(v, P.div.dt); }
+    unsigned& low;   // unused: every result is exact
+    __device__ double same(double a, const DivC& d) const { return xdiv(a, d); }
+    __device__ double up(double a, const DivC& d) const { return xdiv(a, d); }
+    __device__ double plain(double a, const DivC& d) const { return xdiv(a, d); }
+    __device__ double plain_checked(double a, const DivC& d) const { return xdiv(a, d); }
+    __device__ double dt() const { return P.dt; }
+    __device__ double etaK() const { return P.eta_K; }
 };
 // The policy of a march pass: 0 the reciprocal form; 1 the drop-in form's
 // first pass (exact quotients, out-of-range numerators flagged); 2 the drop-in
@@ -166,11 +183,12 @@ struct EtaTrial {
             return c - fma(c, fma(-f.e2, c * c, T), -l);
         } else {
             double lap;
+            const DivSet& d = P.div;
             if (DIM == 3)
-                lap = dv.dvxx((xp - 2. * c + xm)) + dv.dvaa((ap - 2. * c + am)) + dv.dvbb((bp - 2. * c + bm));
+                lap = dv.up(xp - 2. * c + xm, d.dxdx) + dv.up(ap - 2. * c + am, d.dada) + dv.up(bp - 2. * c + bm, d.dbdb);
             else
-                lap = dv.dvxx((xp - 2. * c + xm)) + dv.dvbb((bp - 2. * c + bm));
-            const double force = grain_deta(c, S, phi, P.eta_W, P.eta_A) - P.eta_K * lap;
+                lap = dv.up(xp - 2. * c + xm, d.dxdx) + dv.up(bp - 2. * c + bm, d.dbdb);
+            const double force = grain_deta(c, S, phi, P.eta_W, P.eta_A) - dv.etaK() * lap;
             return c - P.dt_etaL * force;
         }
     }
@@ -356,21 +374,24 @@ struct StepKernel {
             v.mc = cc * fma(hh, Phys::boc - mbc, mbc);
         } else {
             double lapO, lapC;
+            const DivSet& d = k.div;
             if (DIM == 3) {
-                lapO = dv.dvxx((sop[c2] - 2. * oc + som[c2]))
-                     + dv.dvaa((so0[T::i2(a + 1, b)] - 2. * oc + so0[T::i2(a - 1, b)]))
-                     + dv.dvbb((so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)]));
-                lapC = dv.dvxx((scp[c2] - 2. * cc + scm[c2]))
-                     + dv.dvaa((sc0[T::i2(a + 1, b)] - 2. * cc + sc0[T::i2(a - 1, b)]))
-                     + dv.dvbb((sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)]));
+                lapO = dv.up(sop[c2] - 2. * oc + som[c2], d.dxdx)
+                     + dv.up(so0[T::i2(a + 1, b)] - 2. * oc + so0[T::i2(a - 1, b)], d.dada)
+                     + dv.up(so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)], d.dbdb);
+                lapC = dv.up(scp[c2] - 2. * cc + scm[c2], d.dxdx)
+                     + dv.up(sc0[T::i2(a + 1, b)] - 2. * cc + sc0[T::i2(a - 1, b)], d.dada)
+                     + dv.up(sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)], d.dbdb);
             } else {
-                lapO = dv.dvxx((sop[c2] - 2. * oc + som[c2])) + dv.dvbb((so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)]));
-                lapC = dv.dvxx((scp[c2] - 2. * cc + scm[c2])) + dv.dvbb((sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)]));
+                lapO = dv.up(sop[c2] - 2. * oc + som[c2], d.dxdx)
+                     + dv.up(so0[T::i2(a, b + 1)] - 2. * oc + so0[T::i2(a, b - 1)], d.dbdb);
+                lapC = dv.up(scp[c2] - 2. * cc + scm[c2], d.dxdx)
+                     + dv.up(sc0[T::i2(a, b + 1)] - 2. * cc + sc0[T::i2(a, b - 1)], d.dbdb);
             }
             const double hh = h(pc);
             v.hh = hh;
-            v.muO = mu_o_local(oc, cc, hh) - 2. * Phys::ko * lapO;
-            v.muCr = mu_cr_local(oc, cc, hh) - 2. * Phys::kc * lapC;
+            v.muO = mu_o_local(oc, cc, hh) - 2. * Phys::ko * Dv::S * lapO;
+            v.muCr = mu_cr_local(oc, cc, hh) - 2. * Phys::kc * Dv::S * lapC;
             v.mo = o_on ? mobility(oc, hh, gbv, Phys::bmo, Phys::boo, k.gbm1_o) : 0.;
             v.mc = mobility(cc, hh, gbv, Phys::bmc, Phys::boc, k.gbm1_cr);
         }
@@ -432,54 +453,56 @@ struct StepKernel {
             r.crv = crv;
             return r;
         } else {
-        // x faces: the right face of u is the left face of u+1 (same expression)
-        r.rightO = dv.dvx(-.5 * (C.mo + L.mo) * (L.muO - C.muO));
-        r.rightCr = dv.dvx(-.5 * (C.mc + L.mc) * (L.muCr - C.muCr));
+        // x faces: the right face of u is the left face of u+1 (same expression);
+        // the faces stay in the carried scale, the divergence's numerators too
+        const DivSet& d = k.div;
+        r.rightO = dv.up(-.5 * (C.mo + L.mo) * (L.muO - C.muO), d.dx);
+        r.rightCr = dv.up(-.5 * (C.mc + L.mc) * (L.muCr - C.muCr), d.dx);
         double divO = 0., divCr;
         {
             const double mc0 = mc_[c1], mu0 = mC[c1];
-            const double front = dv.dvb(-.5 * (mc0 + mc_[bp]) * (mC[bp] - mu0));
-            const double back = dv.dvb(-.5 * (mc_[bm] + mc0) * (mu0 - mC[bm]));
+            const double front = dv.up(-.5 * (mc0 + mc_[bp]) * (mC[bp] - mu0), d.db);
+            const double back = dv.up(-.5 * (mc_[bm] + mc0) * (mu0 - mC[bm]), d.db);
             if (DIM == 3) {
-                const double top = dv.dva(-.5 * (mc0 + mc_[ap]) * (mC[ap] - mu0));
-                const double bottom = dv.dva(-.5 * (mc_[am] + mc0) * (mu0 - mC[am]));
-                divCr = dv.dvx(leftCr - r.rightCr) + dv.dva(bottom - top) + dv.dvb(back - front);
+                const double top = dv.up(-.5 * (mc0 + mc_[ap]) * (mC[ap] - mu0), d.da);
+                const double bottom = dv.up(-.5 * (mc_[am] + mc0) * (mu0 - mC[am]), d.da);
+                divCr = dv.same(leftCr - r.rightCr, d.dx) + dv.same(bottom - top, d.da) + dv.same(back - front, d.db);
             } else {
-                divCr = dv.dvx(leftCr - r.rightCr) + dv.dvb(back - front);
+                divCr = dv.same(leftCr - r.rightCr, d.dx) + dv.same(back - front, d.db);
             }
         }
         if (o_on) {
             const double m0 = mo_[c1], mu0 = mO[c1];
-            const double front = dv.dvb(-.5 * (m0 + mo_[bp]) * (mO[bp] - mu0));
-            const double back = dv.dvb(-.5 * (mo_[bm] + m0) * (mu0 - mO[bm]));
+            const double front = dv.up(-.5 * (m0 + mo_[bp]) * (mO[bp] - mu0), d.db);
+            const double back = dv.up(-.5 * (mo_[bm] + m0) * (mu0 - mO[bm]), d.db);
             if (DIM == 3) {
-                const double top = dv.dva(-.5 * (m0 + mo_[ap]) * (mO[ap] - mu0));
-                const double bottom = dv.dva(-.5 * (mo_[am] + m0) * (mu0 - mO[am]));
-                divO = dv.dvx(leftO - r.rightO) + dv.dva(bottom - top) + dv.dvb(back - front);
+                const double top = dv.up(-.5 * (m0 + mo_[ap]) * (mO[ap] - mu0), d.da);
+                const double bottom = dv.up(-.5 * (mo_[am] + m0) * (mu0 - mO[am]), d.da);
+                divO = dv.same(leftO - r.rightO, d.dx) + dv.same(bottom - top, d.da) + dv.same(back - front, d.db);
             } else {
-                divO = dv.dvx(leftO - r.rightO) + dv.dvb(back - front);
+                divO = dv.same(leftO - r.rightO, d.dx) + dv.same(back - front, d.db);
             }
         }
         const double oo = C.o, cc = C.cr, pp = C.p;
-        double onv = o_on ? oo + k.dt * divO : oo;
-        double crv = cc + k.dt * divCr;
+        double onv = o_on ? oo + dv.dt() * divO : oo;
+        double crv = cc + dv.dt() * divCr;
         double lapP;
         if (DIM == 3)
-            lapP = dv.dvxx((L.p - 2. * pp + pP)) + dv.dvaa((spu[ap] - 2. * pp + spu[am]))
-                 + dv.dvbb((spu[bp] - 2. * pp + spu[bm]));
+            lapP = dv.up(L.p - 2. * pp + pP, d.dxdx) + dv.up(spu[ap] - 2. * pp + spu[am], d.dada)
+                 + dv.up(spu[bp] - 2. * pp + spu[bm], d.dbdb);
         else
-            lapP = dv.dvxx((L.p - 2. * pp + pP)) + dv.dvbb((spu[bp] - 2. * pp + spu[bm]));
+            lapP = dv.up(L.p - 2. * pp + pP, d.dxdx) + dv.up(spu[bp] - 2. * pp + spu[bm], d.dbdb);
         const double hpv = 30. * pp * pp * (pp - 1.) * (pp - 1.);
         double fp = Phys::W * (4. * pp * pp * pp - 6. * pp * pp + 2. * pp)
-                  + hpv * (foxide(oo, cc) - fmetal(oo, cc)) - 2. * Phys::kp * lapP;
+                  + hpv * (foxide(oo, cc) - fmetal(oo, cc)) - 2. * Phys::kp * Dv::S * lapP;
         if (phi_eta) fp += grain_dphi(s2u, pp, k.eta_W, k.eta_A);
         r.pnv = pp - k.dtL * fp;
         r.dO = 0.;
         r.dCr = 0.;
         if (ck_legacy) {
             const double hn = h(r.pnv);
-            r.dO = dv.dvt(-Phys::ckO * ((Phys::oxideO - onv) * hn - (Phys::oxideO - oo) * C.hh));
-            r.dCr = dv.dvt(-Phys::ckCr * ((Phys::oxideCr - crv) * hn - (Phys::oxideCr - cc) * C.hh));
+            r.dO = dv.plain(-Phys::ckO * ((Phys::oxideO - onv) * hn - (Phys::oxideO - oo) * C.hh), d.dt);
+            r.dCr = dv.plain(-Phys::ckCr * ((Phys::oxideCr - crv) * hn - (Phys::oxideCr - cc) * C.hh), d.dt);
             onv += r.dO;
             crv += r.dCr;
         }
@@ -539,12 +562,12 @@ struct StepKernel {
             if (R.dCr != 0.) acc[1] = dd_add(acc[1], R.dCr);
         }
     }
-    // The X face between two cells as the march carries it: the flux
-    // (exact forms) or, in the reciprocal form, the flux times -2 dx.
+    // The X face between two cells as the march carries it: the flux in the
+    // carried scale (exact forms) or times -2 dx (reciprocal form).
     template <class Dv>
     __device__ static double face_x(const Dv& dv, double m0, double m1, double mu0, double mu1) {
         if constexpr (Dv::kFast) return (m0 + m1) * (mu1 - mu0);
-        else return dv.dvx(-.5 * (m0 + m1) * (mu1 - mu0));
+        else return dv.up(-.5 * (m0 + m1) * (mu1 - mu0), dv.P.div.dx);
     }
     // The surface-mobility closure of the O face at X = 0 with bc=mu
     // (left_flux, 3S:621-628): the carried face, and the budget's increment.
@@ -558,11 +581,12 @@ struct StepKernel {
                 carry = -4. * mf * (P.mu_res - C.muO);
                 lf = (2. * mf * (P.mu_res - C.muO)) * P.f.rdx;
             } else {
-                lf = carry = dv.dvx(2. * mf * (P.mu_res - C.muO));
+                carry = dv.up(2. * mf * (P.mu_res - C.muO), P.div.dx);
+                lf = carry * Dv::S;
             }
         }
         if constexpr (Dv::kFast) inc = (P.dt * lf) * P.f.rdx;
-        else inc = dv.dvx(P.dt * lf);
+        else inc = dv.plain_checked(P.dt * lf, P.div.dx);
         booked = dd_add(booked, inc);
         return carry;
     }
@@ -600,8 +624,8 @@ struct StepKernel {
         unsigned long long errkey = ERR_NONE;
 
         if (st->failed) return false;  // a previous step of this batch was rejected
-        unsigned bad = 0;
-        const typename DivOf<DM>::T dv{P, bad};
+        unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+        const typename DivOf<DM>::T dv{P, low};
 
         auto slot3 = [](int w) { return ((w % 3) + 3) % 3; };
         // o/cr ring of 4 planes: the plane staged at the top of an iteration
@@ -723,7 +747,7 @@ struct StepKernel {
             C = L;
             s2u = s2n;
         }
-        if (DM == 1 && __syncthreads_or(bad != 0)) return true;
+        if (DM == 1 && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
         if (errkey != ERR_NONE) atomicMin(SLAB ? err_word(P, st) : &st->err_key, errkey);
         block_reduce_dd<5>(acc, clipped, sdd, scnt);
         if (threadIdx.x == 0 && threadIdx.y == 0) {
@@ -809,8 +833,8 @@ __device__ __forceinline__ unsigned eta_cell_pass(const StepParams& P, int neta,
                                          double* __restrict__ s2_next, int x, int row, int col,
                                          unsigned long long& errkey) {
     const Grid& g = P.g;
-    unsigned dbad = 0;
-    const typename DivOf<DM>::T dv{P, dbad};
+    unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+    const typename DivOf<DM>::T dv{P, low};
     const long long idx = (long long)x * g.plane + (long long)row * g.pb + col;
     const long long cell = ((long long)x * g.na + row) * g.nb + col + P.cell_off;
     const long long ixm = x > 0 ? idx - g.plane : idx, ixp = x < g.nx - 1 ? idx + g.plane : idx;
@@ -838,7 +862,7 @@ __device__ __forceinline__ unsigned eta_cell_pass(const StepParams& P, int neta,
     if (!in_range) errkey = min(errkey, eta_fail_key(eta_next + idx, neta, g.nstore, P.key_ncells, cell));
     s2_next[idx] = Sn;
     gb_next[idx] = P.eta_scale * smin(1., 16. * pairs);
-    return dbad;
+    return DM == 1 && (low <= kLowQuotient || errkey != ERR_NONE);
 }
 // The cell's eta update with the division policy of the form; in the drop-in
 // form a cell whose numerators left the exact-division range is recomputed
@@ -899,8 +923,8 @@ __device__ __forceinline__ unsigned eta_march_pass(const StepParams& P, int n, c
                                                    double* __restrict__ gb_next, double* __restrict__ s2_next,
                                                    int row, int col, int i0, int i1, unsigned long long& errkey) {
     const Grid& g = P.g;
-    unsigned dbad = 0;
-    const typename DivOf<DM>::T dv{P, dbad};
+    unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+    const typename DivOf<DM>::T dv{P, low};
     const long long rc = (long long)row * g.pb + col;
     const long long cbm = (long long)row * g.pb + (col == 0 ? g.nb - 1 : col - 1);
     const long long cbp = (long long)row * g.pb + (col == g.nb - 1 ? 0 : col + 1);
@@ -956,7 +980,7 @@ __device__ __forceinline__ unsigned eta_march_pass(const StepParams& P, int n, c
         for (int q = 0; q < NCAP; ++q)
             if (q < n) { ep[q] = ec[q]; ec[q] = en[q]; }
     }
-    return dbad;
+    return DM == 1 && (low <= kLowQuotient || errkey != ERR_NONE);
 }
 
 // X-marching form of the eta update for a compile-time number of fields N:
@@ -1281,9 +1305,9 @@ k_eta_tma(const StepParams P, const __grid_constant__ CUtensorMap m_int, const _
             S2 += v * v;
         }
         const long long cell = ((long long)x * g.na + row) * g.nb + col;
-        unsigned dbad = 0;   // the exact policy divides every quotient exactly
+        unsigned low = ~0u;   // the exact policy divides every quotient exactly
         using Dv = typename DivOf<FAST ? 0 : 2>::T;
-        const Dv dv{P, dbad};
+        const Dv dv{P, low};
         const EtaTrial<3, Dv> trial(dv, P, S2, phi);
         double Sn = 0., pairs = 0.;
 #pragma unroll
@@ -1443,9 +1467,9 @@ k_eta_stream(const StepParams P, int neta, const double* __restrict__ eta, const
                 const double v = s0[e * S1 + c1];
                 S += v * v;
             }
-            unsigned dbad = 0;   // the exact policy divides every quotient exactly
+            unsigned low = ~0u;   // the exact policy divides every quotient exactly
             using Dv = typename DivOf<FAST ? 0 : 2>::T;
-            const Dv dv{P, dbad};
+            const Dv dv{P, low};
             const EtaTrial<DIM, Dv> trial(dv, P, S, __ldg(p + idx));
             double Sn = 0., pairs = 0.;
             for (int e = 0; e < neta; ++e) {
