@@ -45,24 +45,19 @@ struct nicr_batch {
     };
     std::vector<PairGraph> graphs;
 
-    void enqueue_step(std::vector<nicr::BatchDomain>& descs, std::vector<nicr::FinalizeDomain>& fins) {
+    void enqueue_step(std::vector<nicr::BatchDomain>& descs) {
         const int n = (int)doms.size();
         for (int i = 0; i < n; ++i) {
             nicr::Model& m = *doms[i]->m;
             m.prepare_step();
             descs[i] = m.step_desc();
+            m.enqueue_eta();   // before the step kernel, whose last CTA per domain commits the step
         }
         launches += nicr::launch_step_batch(descs.data(), n, stream);
-        for (int i = 0; i < n; ++i) {
-            nicr::Model& m = *doms[i]->m;
-            m.complete_step(descs[i].nblocks, false);
-            fins[i] = m.finalize_desc(descs[i].nblocks);
-        }
-        nicr::launch_finalize_batch(fins.data(), n, stream);
-        launches += (n + nicr::kFinalizeMax - 1) / nicr::kFinalizeMax;
+        for (int i = 0; i < n; ++i) doms[i]->m->complete_step();
     }
 
-    void launch_pair(std::vector<nicr::BatchDomain>& descs, std::vector<nicr::FinalizeDomain>& fins) {
+    void launch_pair(std::vector<nicr::BatchDomain>& descs) {
         const int n = (int)doms.size();
         std::vector<int> key((size_t)n);
         for (int i = 0; i < n; ++i) {
@@ -85,8 +80,8 @@ struct nicr_batch {
             for (int i = 0; i < n; ++i) d0[i] = doms[i]->m->launches;
             cudaGraph_t graph = nullptr;
             nicr::check_cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-            enqueue_step(descs, fins);
-            enqueue_step(descs, fins);
+            enqueue_step(descs);
+            enqueue_step(descs);
             nicr::check_cuda(cudaStreamEndCapture(stream, &graph), "cudaStreamEndCapture");
             const cudaError_t e = cudaGraphInstantiate(&q.exec, graph, 0);
             cudaGraphDestroy(graph);
@@ -123,7 +118,10 @@ struct nicr_batch {
         nicr::check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
         nicr::check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
         auto pass = [&] {
-            for (int i = 0; i < n; ++i) descs[i] = doms[i]->m->step_desc();
+            for (int i = 0; i < n; ++i) {
+                descs[i] = doms[i]->m->step_desc();
+                descs[i].budget = nullptr;   // trial launches commit nothing
+            }
             nicr::launch_step_batch(descs.data(), n, stream);
             for (auto* h : doms)
                 if (h->m->advance_eta) h->m->launch_trial_eta();   // the step kernel ran batched above
@@ -160,7 +158,6 @@ struct nicr_batch {
         if (nsteps <= 0) return NICR_OK;
         std::vector<nicr::Model::RunPlan> plans((size_t)n);
         std::vector<nicr::BatchDomain> descs((size_t)n);
-        std::vector<nicr::FinalizeDomain> fins((size_t)n);
         for (int i = 0; i < n; ++i) doms[i]->m->run_begin(plans[i], nsteps, schedule);
         const bool use_graphs = doms[0]->m->graphs_enabled();
         for (int s = 0; s < nsteps;) {
@@ -168,19 +165,23 @@ struct nicr_batch {
             bool pair = use_graphs && s + 1 < nsteps;
             for (int i = 0; pair && i < n; ++i) pair = !doms[i]->m->ksp_due(plans[i], s + 1);
             if (pair) {
-                launch_pair(descs, fins);
+                launch_pair(descs);
                 for (int i = 0; i < n; ++i) doms[i]->m->run_pre_step(plans[i], s + 1);   // schedule entry only
                 s += 2;
             } else {
-                enqueue_step(descs, fins);
+                enqueue_step(descs);
                 ++s;
             }
         }
+        std::vector<nicr::FlushDomain> last((size_t)n);
+        for (int i = 0; i < n; ++i) last[i] = doms[i]->m->flush_desc();
+        nicr::launch_step_flush(last.data(), n, stream);
+        launches += (n + nicr::kFlushMax - 1) / nicr::kFlushMax;
         int rc = NICR_OK;
         err.clear();
         for (int i = 0; i < n; ++i) {
             nicr::Model& m = *doms[i]->m;
-            const int r = m.run_end(plans[i], completed ? completed + i : nullptr);
+            const int r = m.run_end(plans[i], completed ? completed + i : nullptr, false);
             if (r != NICR_OK) {
                 doms[i]->err = m.last_error;
                 if (rc == NICR_OK) {

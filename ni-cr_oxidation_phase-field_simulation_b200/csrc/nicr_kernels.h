@@ -35,10 +35,12 @@ struct Status {
     int timeout;                  // a kernel's bounded wait for its own copies ran out
     long long failed_step;        // index (steps_done) of the rejected step
     long long steps_done;         // accepted steps since creation
-    // Slab form: first failing trial of the step that reads buffer parity q,
-    // in slot q (the slabs of a domain agree on a step's outcome by reading
-    // every slab's slot of that step; see launch_step_finalize_slab).
+    // First failing trial of the step that reads buffer parity q, in slot q.
+    // Slab form: the slabs of a domain agree on a step's outcome by reading
+    // every slab's slot of that step (launch_step_finalize_slab). Whole
+    // domains: the next step's launch reads it (see launch_step_main).
     unsigned long long slot_err[2];
+    int pending[2];               // partials of the step of parity q that await their commit (0: none)
 };
 constexpr unsigned long long ERR_NONE = ~0ull;
 constexpr unsigned long long ERR_ETA_BASE = 1ull << 62;
@@ -54,8 +56,6 @@ struct DevBudget {
 struct StepPartial {
     double s[5][2];
     long long clipped;
-    int redo;   // drop-in form: the CTA's chunk awaits the recomputation kernel
-    int pad;
 };
 
 // Exact divisions by the run constants (drop-in form): dx*dx etc. are the
@@ -105,8 +105,9 @@ struct StepParams {
     // Failing-trial keys in whole-domain reference order: the cell index is
     // offset by cell_off and eta keys count key_ncells cells per field.
     long long cell_off, key_ncells;
-    // Error word of this step: -1 st->err_key, 0/1 st->slot_err[err_slot] (slab form)
+    // Error word of this step: -1 st->err_key, 0/1 st->slot_err[err_slot]
     int err_slot;
+    int slab, pad_;              // an X slab (its plane range and key offsets apply)
     // drop-in form: 1 when a divisor or a constant after a scaled quotient
     // lies outside the certified range, so every chunk is divided by IEEE division
     unsigned div_gate;
@@ -168,13 +169,17 @@ inline void whole_domain_range(StepParams& sp) {
 
 // ---- step --------------------------------------------------------------------
 // Main fused step: mu, M, six-face fluxes, phi, Ck, bounds -> trial buffers.
+// With a budget (P.err_slot = the buffer parity) the commit is deferred: the
+// launch leaves its partials in `partials` as pending, and one extra CTA of it
+// commits the previous step from `prev` (the other parity's partials) beside
+// the step's own CTAs; launch_step_flush commits the last one. Whatever else
+// can fail the step (the eta update) is launched before the step kernel.
+// Without a budget nothing is committed and the caller reads the partials.
 void launch_step_main(const StepParams& P, const double* o, const double* cr, const double* p,
                       const double* gb, const double* s2, double* on, double* crn, double* pn,
-                      StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out);
+                      StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                      cudaStream_t stream, int* nblocks_out);
 int step_main_blocks(const StepParams& P);
-// kernels launch_step_main launches: the drop-in form adds the recomputation
-// kernel of CTAs whose numerators left the exact-division range
-int step_main_kernels(const StepParams& P);
 // Planes per CTA along X for grid g (step and eta kernels), and one chunk for
 // the n domains of a batch. NICR_XCHUNK forces a chunk for tuning runs.
 int choose_xchunk(const Grid& g);
@@ -190,8 +195,9 @@ void step_kernels_prepare(const StepParams& P);
 // The reciprocal form's launchers (nicr_step_fast.cu, compiled with FMA
 // contraction); the generic launchers dispatch to them when P.fast is set.
 void launch_step_main_fast(const StepParams& P, const double* o, const double* cr, const double* p, const double* gb,
-                           const double* s2, double* on, double* crn, double* pn, StepPartial* partials, Status* st,
-                           cudaStream_t stream, int* nblocks_out);
+                           const double* s2, double* on, double* crn, double* pn, StepPartial* partials,
+                           const StepPartial* prev, DevBudget* budget, Status* st, cudaStream_t stream,
+                           int* nblocks_out);
 void launch_eta_update_fast(const StepParams& P, int neta, const double* eta, const double* s2, const double* p,
                             double* eta_next, double* gb_next, double* s2_next, Status* st, cudaStream_t stream);
 void step_kernels_prepare_fast(const StepParams& P);
@@ -211,10 +217,12 @@ struct BatchDomain {
     const double *o, *cr, *p, *gb, *s2;
     double *on, *crn, *pn;
     StepPartial* partials;
+    const StepPartial* prev;
+    DevBudget* budget;
     Status* st;
     int gx, gy, block0, nblocks;
 };
-constexpr int kBatchMax = 48;   // 48 entries: ~24 KB of kernel parameters (limit 32 KB)
+constexpr int kBatchMax = 48;   // 48 entries: ~32,000 bytes of kernel parameters (limit 32,764)
 struct StepBatch {
     int n, pad;
     BatchDomain d[kBatchMax];
@@ -228,13 +236,15 @@ struct BatchSlim {
     Grid g;
     double layer_o;
     long long key_ncells;
-    int x_hi, inlet, gx, gy, block0, pad;
+    int x_hi, inlet, gx, gy, block0, nblocks, err_slot, pad;
     const double *o, *cr, *p, *gb, *s2;
     double *on, *crn, *pn;
     StepPartial* partials;
+    const StepPartial* prev;
+    DevBudget* budget;
     Status* st;
 };
-constexpr int kBatchSlimMax = 160;   // 160 x 168 bytes + the shared parameters: < 27.5 KB of kernel parameters
+constexpr int kBatchSlimMax = 160;   // 160 x 192 bytes + the shared parameters: < 31.5 KB of kernel parameters
 struct StepBatchSlim {
     StepParams base;
     int n, pad;
@@ -269,26 +279,15 @@ void step_eta_prepare_fast(const StepParams& P, int neta);
 bool step_fused_applies(const Grid& g, int neta);
 bool launch_step_fused(const StepParams& P, int neta, const double* o, const double* cr, const double* p,
                        const double* eta, double* on, double* crn, double* pn, double* eta_next,
-                       StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out);
+                       StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                       cudaStream_t stream, int* nblocks_out);
 bool launch_step_fused_fast(const StepParams& P, int neta, const double* o, const double* cr, const double* p,
                             const double* eta, double* on, double* crn, double* pn, double* eta_next,
-                            StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out);
+                            StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                            cudaStream_t stream, int* nblocks_out);
 // kernel attributes of the fused step, set outside any stream capture
 void step_fused_prepare(const StepParams& P, int neta);
 void step_fused_prepare_fast(const StepParams& P, int neta);
-
-struct FinalizeDomain {
-    const StepPartial* partials;
-    int nblocks, pad;
-    DevBudget* budget;
-    Status* st;
-};
-constexpr int kFinalizeMax = 512;
-struct FinalizeBatch {
-    int n, pad;
-    FinalizeDomain d[kFinalizeMax];
-};
-void launch_finalize_batch(const FinalizeDomain* doms, int n, cudaStream_t stream);
 
 // The seven arrays of a 3D VTI frame in file order (X fastest) and type, for
 // the output path (nicr_vti.cu). range gets bit a set when array a holds a
@@ -300,9 +299,19 @@ struct VtiArgs {
 };
 void launch_vti_arrays(const VtiArgs& a, void* out, bool f64, unsigned* range, cudaStream_t stream);
 
-// Commit of one step: reduce partials, commit budget unless a trial failed
-void launch_step_finalize(const StepPartial* partials, int nblocks, DevBudget* budget, Status* st,
-                          int accept_mode, cudaStream_t stream);
+// Commits the pending step, if any: its partials (of parity q at partials +
+// q * cap) reduced, then budget and counters unless a trial failed.
+struct FlushDomain {
+    const StepPartial* partials;
+    DevBudget* budget;
+    Status* st;
+    int cap, pad;
+};
+constexpr int kFlushMax = 512;   // 512 x 32 bytes of kernel parameters
+struct FlushList {
+    FlushDomain d[kFlushMax];
+};
+void launch_step_flush(const FlushDomain* doms, int n, cudaStream_t stream);
 // Slab form of the commit: the step is rejected when any slab's error word
 // of this step (peers[j]->slot_err[slot], read after every slab's step
 // kernels completed) holds a failing trial; the minimum key is recorded in

@@ -120,6 +120,7 @@ Model::Model(const nicr_config& cfg, const SlabSpec* slab) : c(cfg), dim(cfg.dim
         sp.cell_off = (long long)x_off * g.na * g.nb;
         sp.key_ncells = (long long)c.nx * g.na * g.nb;
         sp.err_slot = 0;
+        sp.slab = 1;
     }
     sp.xchunk = choose_xchunk(own_grid());
 
@@ -133,7 +134,7 @@ Model::Model(const nicr_config& cfg, const SlabSpec* slab) : c(cfg), dim(cfg.dim
         grain = dalloc(ns);
         if (dim == 2) { gb_initial = dalloc(ns); if (has_eta) { pairs = dalloc(ns); check_cuda(cudaMemsetAsync(pairs, 0, ns * 8, stream), "memset"); } }
         partial_cap = std::max(step_main_blocks(sp), 148 * 4) + 8;
-        partials = dalloc_t<StepPartial>(partial_cap);
+        partials = dalloc_t<StepPartial>((size_t)2 * partial_cap);   // one half per buffer parity
         st = dalloc_t<Status>(1);
         bud = dalloc_t<DevBudget>(1);
         diag_part = dalloc_t<DiagOut>(148 * 4 + 8);
@@ -141,7 +142,7 @@ Model::Model(const nicr_config& cfg, const SlabSpec* slab) : c(cfg), dim(cfg.dim
         red_out = dalloc_t<StepPartial>(1);
         check_cuda(cudaMallocHost(&h_st, sizeof(Status)), "cudaMallocHost");
         check_cuda(cudaMemsetAsync(bud, 0, sizeof(DevBudget), stream), "memset");
-        Status s0{ERR_NONE, 0, 0, -1, 0, {ERR_NONE, ERR_NONE}};
+        Status s0{ERR_NONE, 0, 0, -1, 0, {ERR_NONE, ERR_NONE}, {0, 0}};
         *h_st = s0;
         check_cuda(cudaMemcpyAsync(st, h_st, sizeof(Status), cudaMemcpyHostToDevice, stream), "memcpy");
 
@@ -766,6 +767,7 @@ void Model::reset_status() {
     h_st->err_key = ERR_NONE;
     h_st->failed = 0;
     h_st->timeout = 0;
+    h_st->pending[0] = h_st->pending[1] = 0;
     h_st->failed_step = -1;
     h_st->steps_done = steps_done;
     h_st->slot_err[0] = h_st->slot_err[1] = ERR_NONE;
@@ -780,7 +782,7 @@ void Model::set_xchunk(int c) {
         cudaFree(partials);
         partials = nullptr;
         partial_cap = need;
-        partials = dalloc_t<StepPartial>(partial_cap);
+        partials = dalloc_t<StepPartial>((size_t)2 * partial_cap);
     }
     for (auto& q : pair_graphs)   // captured launches carry the old grid
         if (q.exec) { cudaGraphExecDestroy(q.exec); q.exec = nullptr; }
@@ -794,9 +796,9 @@ void Model::launch_trial_eta() {
 
 void Model::launch_trial_kernels() {
     int nb = 0;
-    if (onepass_step() && launch_onepass(&nb)) return;
+    if (onepass_step() && launch_onepass(&nb, nullptr)) return;
     const BatchDomain d = step_desc();
-    launch_step_main(sp, d.o, d.cr, d.p, d.gb, d.s2, d.on, d.crn, d.pn, partials, st, stream, &nb);
+    launch_step_main(sp, d.o, d.cr, d.p, d.gb, d.s2, d.on, d.crn, d.pn, partials, nullptr, nullptr, st, stream, &nb);
     launch_trial_eta();
 }
 
@@ -841,39 +843,46 @@ void Model::prepare_step() {
     if (has_eta && eta_dirty) eta_mask_now();
 }
 
+// The parameters of a committed step: its error word is its buffer parity's.
+StepParams Model::step_params() const {
+    StepParams q = sp;
+    q.err_slot = cur;
+    return q;
+}
+
+FlushDomain Model::flush_desc() const { return FlushDomain{partials, bud, st, partial_cap, 0}; }
+
+void Model::flush_commit() {
+    const size_t e = prof_begin();
+    const FlushDomain d = flush_desc();
+    launch_step_flush(&d, 1, stream);
+    prof_end(K_FINALIZE, e, 1);
+}
+
 BatchDomain Model::step_desc() const {
     BatchDomain d{};
     const int nxt = cur ^ 1;
-    d.sp = sp;
+    d.sp = step_params();
     d.o = o_[cur]; d.cr = cr_[cur]; d.p = p_[cur];
     d.gb = gb_[gcur];
     d.s2 = has_eta ? s2_[gcur] : nullptr;
     d.on = o_[nxt]; d.crn = cr_[nxt]; d.pn = p_[nxt];
-    d.partials = partials;
+    d.partials = partials + (size_t)cur * partial_cap;
+    d.prev = partials + (size_t)(cur ^ 1) * partial_cap;
+    d.budget = bud;
     d.st = st;
     return d;
 }
 
-FinalizeDomain Model::finalize_desc(int nb) const {
-    FinalizeDomain f{};
-    f.partials = partials;
-    f.nblocks = nb;
-    f.budget = bud;
-    f.st = st;
-    return f;
+void Model::enqueue_eta() {
+    if (!advance_eta) return;
+    const size_t e = prof_begin();
+    launch_eta_update(step_params(), neta, eta_[ecur], s2_[gcur], p_[cur], eta_[ecur ^ 1], gb_[gcur ^ 1],
+                      s2_[gcur ^ 1], st, stream);
+    prof_end(K_ETA_UPDATE, e, 1);
 }
 
-void Model::complete_step(int nb, bool finalize) {
-    if (advance_eta) {
-        const size_t e = prof_begin();
-        launch_eta_update(sp, neta, eta_[ecur], s2_[gcur], p_[cur], eta_[ecur ^ 1], gb_[gcur ^ 1], s2_[gcur ^ 1], st, stream);
-        prof_end(K_ETA_UPDATE, e, 1);
-    }
-    if (finalize) {
-        const size_t e = prof_begin();
-        launch_step_finalize(partials, nb, bud, st, 0, stream);
-        prof_end(K_FINALIZE, e, 1);
-    }
+void Model::complete_step() {
     cur ^= 1;
     if (advance_eta) { ecur ^= 1; gcur ^= 1; }
 }
@@ -899,10 +908,11 @@ bool Model::onepass_step() const {
            step_fused_applies(g, neta);
 }
 
-bool Model::launch_onepass(int* nb) {
+bool Model::launch_onepass(int* nb, DevBudget* budget) {
     const size_t e = prof_begin();
-    if (!launch_step_fused(sp, neta, o_[cur], cr_[cur], p_[cur], eta_[ecur], o_[cur ^ 1], cr_[cur ^ 1], p_[cur ^ 1],
-                           eta_[ecur ^ 1], partials, st, stream, nb)) {
+    if (!launch_step_fused(budget ? step_params() : sp, neta, o_[cur], cr_[cur], p_[cur], eta_[ecur], o_[cur ^ 1],
+                           cr_[cur ^ 1], p_[cur ^ 1], eta_[ecur ^ 1], partials + (size_t)cur * partial_cap,
+                           partials + (size_t)(cur ^ 1) * partial_cap, budget, st, stream, nb)) {
         onepass_failed = true;
         return false;
     }
@@ -913,13 +923,8 @@ bool Model::launch_onepass(int* nb) {
 void Model::enqueue_step() {
     int nb = 0;
     if (onepass_step()) {
-        if (launch_onepass(&nb)) {
-            const size_t e = prof_begin();
-            launch_step_finalize(partials, nb, bud, st, 0, stream);
-            prof_end(K_FINALIZE, e, 1);
-            cur ^= 1;
-            ecur ^= 1;
-            gcur ^= 1;
+        if (launch_onepass(&nb, bud)) {
+            complete_step();
             eta_dirty = true;   // gb and eta_s2 were not written: rebuilt from eta when read
             return;
         }
@@ -928,22 +933,19 @@ void Model::enqueue_step() {
     const BatchDomain d = step_desc();
     if (fused_step()) {
         if (!ticket) ticket = dalloc_t<unsigned>(1);
-        size_t e = prof_begin();
-        launch_step_eta_fast(sp, neta, d.o, d.cr, d.p, d.gb, d.s2, d.on, d.crn, d.pn, partials, eta_[ecur],
+        flush_commit();   // the previous step: k_step_eta commits nothing
+        const size_t e = prof_begin();
+        launch_step_eta_fast(d.sp, neta, d.o, d.cr, d.p, d.gb, d.s2, d.on, d.crn, d.pn, d.partials, eta_[ecur],
                              eta_[ecur ^ 1], gb_[gcur ^ 1], s2_[gcur ^ 1], ticket, st, stream, &nb);
         prof_end(K_STEP_ETA, e, 1);
-        e = prof_begin();
-        launch_step_finalize(partials, nb, bud, st, 0, stream);
-        prof_end(K_FINALIZE, e, 1);
-        cur ^= 1;
-        ecur ^= 1;
-        gcur ^= 1;
+        complete_step();
         return;
     }
+    enqueue_eta();   // before the step kernel, whose last CTA commits the step
     const size_t e = prof_begin();
-    launch_step_main(sp, d.o, d.cr, d.p, d.gb, d.s2, d.on, d.crn, d.pn, partials, st, stream, &nb);
-    prof_end(K_STEP_MAIN, e, step_main_kernels(sp));
-    complete_step(nb, true);
+    launch_step_main(d.sp, d.o, d.cr, d.p, d.gb, d.s2, d.on, d.crn, d.pn, d.partials, d.prev, bud, st, stream, &nb);
+    prof_end(K_STEP_MAIN, e, 1);
+    complete_step();
 }
 
 std::string Model::describe_failure(unsigned long long key, int nxt) {
@@ -1039,6 +1041,7 @@ void Model::run_pre_step(RunPlan& r, int s) {
     const long long n = r.before + s + 1;
     const double time = double(n) * c.dt;
     if (c.nucleation == NICR_NUC_KSP && time + 1.e-12 * c.nucleation_period >= r.next) {
+        if (s > 0) flush_commit();   // the scan stamps only states of accepted steps
         kd.neta = neta;
         const size_t e = prof_begin();
         launch_ksp_scan(kd, o_[cur], cr_[cur], p_[cur], eta_[ecur], kw, bud, kres, st, stream);
@@ -1049,7 +1052,8 @@ void Model::run_pre_step(RunPlan& r, int s) {
     r.sched[(size_t)s] = r.next;
 }
 
-int Model::run_end(RunPlan& r, int* completed) {
+int Model::run_end(RunPlan& r, int* completed, bool flush) {
+    if (flush && !is_slab) flush_commit();
     if (!r.schedule) return finish_batch(r.before, r.nsteps, nullptr, completed);
     r.sched[(size_t)r.nsteps] = r.next;
     const int rc = finish_batch(r.before, r.nsteps, &r.sched, completed);
@@ -1167,8 +1171,8 @@ int Model::slab_launch() {
     int nb = 0;
     size_t e = prof_begin();
     launch_step_main(P, o_[cur], cr_[cur], p_[cur], gb_[gcur], has_eta ? s2_[gcur] : nullptr, o_[cur ^ 1],
-                     cr_[cur ^ 1], p_[cur ^ 1], partials, st, stream, &nb);
-    prof_end(K_STEP_MAIN, e, step_main_kernels(P));
+                     cr_[cur ^ 1], p_[cur ^ 1], partials, nullptr, nullptr, st, stream, &nb);
+    prof_end(K_STEP_MAIN, e, 1);
     if (advance_eta) {
         e = prof_begin();
         launch_eta_update(P, neta, eta_[ecur], s2_[gcur], p_[cur], eta_[ecur ^ 1], gb_[gcur ^ 1], s2_[gcur ^ 1], st, stream);

@@ -112,8 +112,9 @@ public:
 
     // One step split into phases, for batches that launch the step kernel of
     // many domains at once: prepare_step (eta mask when stale), step_desc (the
-    // step kernel's parameters and buffers), then complete_step (eta update,
-    // optional finalize, buffer parity). run_begin / run_pre_step / run_end are
+    // step kernel's parameters and buffers), enqueue_eta (the eta update, before
+    // the step kernel, whose last CTA commits the step), then complete_step
+    // (buffer parity). run_begin / run_pre_step / run_end are
     // run()'s schedule (Ksp scans) and commit around those steps.
     struct RunPlan {
         long long before = 0;
@@ -135,8 +136,11 @@ public:
     void launch_trial_eta();
     void prepare_step();
     BatchDomain step_desc() const;
-    FinalizeDomain finalize_desc(int nblocks) const;
-    void complete_step(int nblocks, bool finalize);
+    StepParams step_params() const;
+    FlushDomain flush_desc() const;
+    void flush_commit();   // commits the last enqueued step (each step kernel commits the one before)
+    void enqueue_eta();
+    void complete_step();
     // step-pair graphs: whether they are used, whether step s of plan r
     // starts with a Ksp scan, and the buffer parity a captured pair keys on
     bool graphs_enabled() const;
@@ -144,7 +148,7 @@ public:
     int parity_key() const { return cur | (ecur << 1) | (gcur << 2); }
     void run_begin(RunPlan& r, int nsteps, bool schedule);
     void run_pre_step(RunPlan& r, int s);
-    int run_end(RunPlan& r, int* completed);
+    int run_end(RunPlan& r, int* completed, bool flush = true);   // flush: commit the last step first
 
     // The own planes as a grid of their own (a whole domain: g) and their
     // offset in the stored arrays, for reductions over owned cells.
@@ -197,7 +201,7 @@ public:
     bool onepass_step() const;
     bool onepass_failed = false;   // the launcher refused (buffer alignment): split form from then on
     // one step in the one-pass form into the trial buffers; false when it cannot launch
-    bool launch_onepass(int* nb);
+    bool launch_onepass(int* nb, DevBudget* budget);
 
 private:
     friend class SlabGroup;

@@ -54,6 +54,7 @@ __global__ void k_status_clear(nicr::Status* st) {
     st->timeout = 0;
     st->failed_step = -1;
     st->slot_err[0] = st->slot_err[1] = nicr::ERR_NONE;
+    st->pending[0] = st->pending[1] = 0;
 }
 
 // Reduces the per-CTA partials in block order (deterministic) into the
@@ -177,7 +178,7 @@ extern "C" int nicr_step_noalloc(const nicr_config* cfg, const double* o, const 
     k_status_clear<<<1, 1, 0, st>>>(&s->status);
     int nb = 0;
     nicr::launch_step_main(sp, o, cr, p, cfg->grains ? gb : nullptr, eta_s2, o_next, cr_next, p_next, s->partials,
-                           &s->status, st, &nb);
+                           nullptr, nullptr, &s->status, st, &nb);
     k_step_result<<<1, 256, 0, st>>>(s->partials, nb, &s->status, result);
     return cudaGetLastError() == cudaSuccess ? NICR_OK : NICR_ERR_CUDA;
 }

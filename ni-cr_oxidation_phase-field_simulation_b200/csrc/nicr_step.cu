@@ -103,43 +103,14 @@ __global__ void k_check_division(DivC d, long long n, unsigned long long seed, u
     atomicAdd(counts + 1, total);
 }
 
-// Step commit: partial sums in block order (deterministic), then the budget is
-// advanced only when no trial failed (fields swap only on acceptance, 3S:821).
-__device__ __forceinline__ void finalize_body(const StepPartial* __restrict__ partials, int nblocks,
-                                              DevBudget* budget, Status* st, int accept_mode) {
+// CTA b commits domain b's pending step.
+__global__ void k_step_flush(const __grid_constant__ FlushList L) {
     __shared__ DD sdd[32 * 5];
     __shared__ long long scnt[32];
-    if (st->failed) return;
-    DD acc[5] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
-    long long clipped = 0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-        for (int q = 0; q < 5; ++q) acc[q] = dd_add(acc[q], DD{partials[b].s[q][0], partials[b].s[q][1]});
-        clipped += partials[b].clipped;
-    }
-    block_reduce_dd<5>(acc, clipped, sdd, scnt);
-    if (threadIdx.x == 0) {
-        if (st->err_key != ERR_NONE) {
-            st->failed = 1;
-            st->failed_step = st->steps_done;
-            return;
-        }
-        if (accept_mode == 0) {
-            // slots: ckO ckCr clipO clipCr bcO -> budget indices 2 3 4 5 6
-            for (int q = 0; q < 5; ++q) {
-                DD b{budget->v[2 + q][0], budget->v[2 + q][1]};
-                b = dd_add(b, acc[q]);
-                budget->v[2 + q][0] = b.hi;
-                budget->v[2 + q][1] = b.lo;
-            }
-            budget->clipped += clipped;
-            st->steps_done += 1;
-        }
-    }
-}
-
-__global__ void k_step_finalize(const StepPartial* __restrict__ partials, int nblocks, DevBudget* budget,
-                                Status* st, int accept_mode) {
-    finalize_body(partials, nblocks, budget, st, accept_mode);
+    const FlushDomain& d = L.d[blockIdx.x];
+    if (d.st->failed) return;
+    const int q = d.st->pending[0] ? 0 : 1;   // at most one step is pending
+    commit_pending(d.partials + (size_t)q * d.cap, q, d.budget, d.st, sdd, scnt);
 }
 
 // Slab commit: the same reduction; the step's outcome is the failing-trial
@@ -219,12 +190,6 @@ __global__ void k_copy_segments(const CopyList L, const Status* st) {
         const double2 v = *reinterpret_cast<const double2*>(S.src + r * S.src_pitch + c);
         *reinterpret_cast<double2*>(S.dst + r * S.dst_pitch + c) = v;
     }
-}
-
-// Batched commit: block b commits domain b (same arithmetic as k_step_finalize).
-__global__ void k_finalize_batch(const __grid_constant__ FinalizeBatch B) {
-    const FinalizeDomain& d = B.d[blockIdx.x];
-    finalize_body(d.partials, d.nblocks, d.budget, d.st, 0);
 }
 
 // refresh() for output: mu at interior cells, M at interior cells.
@@ -347,25 +312,26 @@ void step_kernels_prepare(const StepParams& P) {
     ensure_smem_attr(k, (int)T::SMEM_BYTES);
 }
 
-int step_main_kernels(const StepParams& P) { return P.fast ? 1 : 2; }
-
 void launch_step_main(const StepParams& P, const double* o, const double* cr, const double* p, const double* gb,
-                      const double* s2, double* on, double* crn, double* pn, StepPartial* partials, Status* st,
-                      cudaStream_t stream, int* nblocks_out) {
-    if (P.fast) launch_step_main_fast(P, o, cr, p, gb, s2, on, crn, pn, partials, st, stream, nblocks_out);
-    else launch_step_form<false>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, stream, nblocks_out);
+                      const double* s2, double* on, double* crn, double* pn, StepPartial* partials,
+                      const StepPartial* prev, DevBudget* budget, Status* st, cudaStream_t stream, int* nblocks_out) {
+    if (P.fast)
+        launch_step_main_fast(P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, stream, nblocks_out);
+    else
+        launch_step_form<false>(P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, stream, nblocks_out);
 }
 
 bool step_fused_applies(const Grid& g, int neta) { return fused_step_applies(g, neta); }
 
 bool launch_step_fused(const StepParams& P, int neta, const double* o, const double* cr, const double* p,
                        const double* eta, double* on, double* crn, double* pn, double* eta_next,
-                       StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out) {
+                       StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                       cudaStream_t stream, int* nblocks_out) {
     if (P.fast)
-        return launch_step_fused_fast(P, neta, o, cr, p, eta, on, crn, pn, eta_next, partials, st, stream,
-                                      nblocks_out);
-    return launch_step_fused_form<false>(P, neta, o, cr, p, eta, on, crn, pn, eta_next, partials, st, stream,
-                                         nblocks_out);
+        return launch_step_fused_fast(P, neta, o, cr, p, eta, on, crn, pn, eta_next, partials, prev, budget, st,
+                                      stream, nblocks_out);
+    return launch_step_fused_form<false>(P, neta, o, cr, p, eta, on, crn, pn, eta_next, partials, prev, budget, st,
+                                         stream, nblocks_out);
 }
 
 void step_fused_prepare(const StepParams& P, int neta) {
@@ -388,9 +354,13 @@ void launch_eta_update(const StepParams& P, int neta, const double* eta, const d
     else launch_eta_form<false>(P, neta, eta, s2, p, eta_next, gb_next, s2_next, st, stream);
 }
 
-void launch_step_finalize(const StepPartial* partials, int nblocks, DevBudget* budget, Status* st, int accept_mode,
-                          cudaStream_t stream) {
-    k_step_finalize<<<1, 256, 0, stream>>>(partials, nblocks, budget, st, accept_mode);
+void launch_step_flush(const FlushDomain* doms, int n, cudaStream_t stream) {
+    for (int i0 = 0; i0 < n; i0 += kFlushMax) {
+        FlushList L;
+        const int m = std::min(n - i0, kFlushMax);
+        std::copy(doms + i0, doms + i0 + m, L.d);
+        k_step_flush<<<m, 256, 0, stream>>>(L);
+    }
 }
 
 void launch_step_finalize_slab(const StepPartial* partials, int nblocks, DevBudget* budget, Status* st,
@@ -416,15 +386,6 @@ void launch_copy_segments(const CopyList& L, const Status* st, cudaStream_t stre
     k_copy_segments<<<dim3(bx, L.count), 256, 0, stream>>>(L, st);
 }
 
-void launch_finalize_batch(const FinalizeDomain* doms, int n, cudaStream_t stream) {
-    for (int i0 = 0; i0 < n; i0 += kFinalizeMax) {
-        FinalizeBatch B{};
-        B.n = n - i0 < kFinalizeMax ? n - i0 : kFinalizeMax;
-        for (int i = 0; i < B.n; ++i) B.d[i] = doms[i0 + i];
-        k_finalize_batch<<<B.n, 256, 0, stream>>>(B);
-    }
-}
-
 // The shared part of a domain's parameters: everything but what BatchSlim carries.
 static StepParams slim_base(StepParams sp) {
     sp.g = Grid{};
@@ -432,6 +393,7 @@ static StepParams slim_base(StepParams sp) {
     sp.inlet = 0;
     sp.x_hi = 0;
     sp.key_ncells = 0;
+    sp.err_slot = -1;
     return sp;
 }
 
@@ -447,7 +409,7 @@ static bool launch_step_batch_slim(BatchDomain* doms, int n, cudaStream_t stream
     const StepParams ref = slim_base(doms[0].sp);
     for (int i = 0; i < n; ++i) {
         const StepParams b = slim_base(doms[i].sp);
-        if (std::memcmp(&b, &ref, sizeof(StepParams)) != 0 || doms[i].sp.x_lo != 0 || doms[i].sp.err_slot >= 0)
+        if (std::memcmp(&b, &ref, sizeof(StepParams)) != 0 || doms[i].sp.x_lo != 0 || doms[i].sp.slab)
             return false;
     }
     const int dim = doms[0].sp.g.dim, fast = doms[0].sp.fast;
@@ -465,13 +427,17 @@ static bool launch_step_batch_slim(BatchDomain* doms, int n, cudaStream_t stream
         s.gx = (int)grid.x;
         s.gy = (int)grid.y;
         s.block0 = nb;
+        s.nblocks = (int)(grid.x * grid.y * grid.z);
+        s.err_slot = d.sp.err_slot;
         s.pad = 0;
         s.o = d.o; s.cr = d.cr; s.p = d.p; s.gb = d.gb; s.s2 = d.s2;
         s.on = d.on; s.crn = d.crn; s.pn = d.pn;
         s.partials = d.partials;
+        s.prev = d.prev;
+        s.budget = d.budget;
         s.st = d.st;
-        doms[i].nblocks = (int)(grid.x * grid.y * grid.z);
-        nb += doms[i].nblocks;
+        doms[i].nblocks = s.nblocks;
+        nb += s.nblocks + (d.budget ? 1 : 0);   // and the CTA that commits the previous step
     }
     if (fast) launch_batch_slim_fast(B, nb, dim, stream);
     else if (dim == 3) launch_batch_slim<3, TA3, TB3, 2, false>(B, nb, stream);
@@ -494,8 +460,9 @@ int launch_step_batch(BatchDomain* doms, int n, cudaStream_t stream) {
             d.gx = (int)grid.x;
             d.gy = (int)grid.y;
             d.block0 = nb;
-            nb += (int)(grid.x * grid.y * grid.z);
-            doms[i].nblocks = (int)(grid.x * grid.y * grid.z);
+            d.nblocks = (int)(grid.x * grid.y * grid.z);
+            nb += d.nblocks + (d.budget ? 1 : 0);   // and the CTA that commits the previous step
+            doms[i].nblocks = d.nblocks;
             B.d[B.n++] = d;
             ++i;
         }

@@ -12,9 +12,10 @@
 namespace nicr {
 
 void launch_step_main_fast(const StepParams& P, const double* o, const double* cr, const double* p, const double* gb,
-                           const double* s2, double* on, double* crn, double* pn, StepPartial* partials, Status* st,
-                           cudaStream_t stream, int* nblocks_out) {
-    launch_step_form<true>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, stream, nblocks_out);
+                           const double* s2, double* on, double* crn, double* pn, StepPartial* partials,
+                           const StepPartial* prev, DevBudget* budget, Status* st, cudaStream_t stream,
+                           int* nblocks_out) {
+    launch_step_form<true>(P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, stream, nblocks_out);
 }
 
 void launch_eta_update_fast(const StepParams& P, int neta, const double* eta, const double* s2, const double* p,
@@ -32,9 +33,10 @@ bool launch_step_eta_fast(const StepParams& P, int neta, const double* o, const 
 
 bool launch_step_fused_fast(const StepParams& P, int neta, const double* o, const double* cr, const double* p,
                             const double* eta, double* on, double* crn, double* pn, double* eta_next,
-                            StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out) {
-    return launch_step_fused_form<true>(P, neta, o, cr, p, eta, on, crn, pn, eta_next, partials, st, stream,
-                                        nblocks_out);
+                            StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                            cudaStream_t stream, int* nblocks_out) {
+    return launch_step_fused_form<true>(P, neta, o, cr, p, eta, on, crn, pn, eta_next, partials, prev, budget, st,
+                                        stream, nblocks_out);
 }
 
 void step_fused_prepare_fast(const StepParams& P, int neta) {

@@ -140,7 +140,7 @@ struct OnePassStep {
                                     const double* __restrict__ cr, const double* __restrict__ p,
                                     double* __restrict__ on, double* __restrict__ crn, double* __restrict__ pn,
                                     double* __restrict__ eta_next, StepPartial* __restrict__ partials, Status* st,
-                                    unsigned long long* bars, int kb) {
+                                    unsigned long long* bars, int kb, int bx, int by, int bz) {
         extern __shared__ __align__(128) unsigned char fused_smem[];
         double* smem = reinterpret_cast<double*>(fused_smem);
         double* so = smem;                 // 4 slots x S2
@@ -157,7 +157,6 @@ struct OnePassStep {
         double* ering = reinterpret_cast<double*>(
             fused_smem + L::STEP_BYTES + ((128u - (smem_u32(fused_smem + L::STEP_BYTES) & 127u)) & 127u));
 
-        if (st->failed) return false;   // a previous step of this batch was rejected
         unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
         const typename DivOf<DM>::T dv{P, low};
 
@@ -166,8 +165,8 @@ struct OnePassStep {
         const bool bounds_legacy = MODE == 1 ? true : P.bounds == 1;
         const Grid& g = P.g;
         const int ta = threadIdx.y, tb = threadIdx.x, tid = tb + TB * ta;
-        const int a0 = blockIdx.y * TA, b0 = blockIdx.x * TB;
-        const int i0 = blockIdx.z * P.xchunk, i1 = min(g.nx, i0 + P.xchunk);
+        const int a0 = by * TA, b0 = bx * TB;
+        const int i0 = bz * P.xchunk, i1 = min(g.nx, i0 + P.xchunk);
         const int row = a0 + ta, col = b0 + tb;
         const typename SK::Offs offs = SK::make_offs(g, a0, b0);
 
@@ -230,9 +229,7 @@ struct OnePassStep {
             ring_o = eta_slot_point<N>(a, b, ring_s);
         }
 
-        DD acc[5] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};  // ckO ckCr clipO clipCr bcO
-        long long clipped = 0;
-        unsigned long long errkey = ERR_NONE;
+        LocalBook book;
 
         auto slot3 = [](int w) { return ((w % 3) + 3) % 3; };
         auto oslot = [&](int w) { return so + (w & 3) * T::S2; };
@@ -286,8 +283,8 @@ struct OnePassStep {
             // the x = 0 face of plane 0 and the inlet's budget term, here rather
             // than in the march: left_flux (3S:621-628), the surface-mobility
             // closure of the O face with bc=mu, replaces the ghost face
-            if (P.bc == 1) FxO = SK::surface_face(dv, P, o_on, C, gbu, acc[4]);
-            if (P.inlet) acc[4] = dd_add(acc[4], P.layer_o - __ldg(o + (long long)row * g.pb + col));
+            if (P.bc == 1) FxO = SK::surface_face(dv, P, o_on, C, gbu, book);
+            if (P.inlet) book.add(4, P.layer_o - __ldg(o + (long long)row * g.pb + col));
         } else {
             SK::load_oc(P, o, cr, i0 - 2, oslot(i0 - 2), cslot(i0 - 2), offs);
             SK::load_oc(P, o, cr, i0 - 1, oslot(i0 - 1), cslot(i0 - 1), offs);
@@ -370,7 +367,7 @@ struct OnePassStep {
                                                              mO, mC, mo_, mc_, spu, c1, bp, bm, ap, am);
                 const double pp = C.p;
                 FxO = R.rightO; FxCr = R.rightCr;
-                SK::finish_cell(R, bounds_legacy, on + gidx, crn + gidx, pn + gidx, acc, clipped, errkey, cell_of);
+                SK::finish_cell(R, bounds_legacy, on + gidx, crn + gidx, pn + gidx, book, cell_of);
 
                 // eta_trial (3S:514-526) at plane u; a failing cell is keyed once, by its
                 // first failing field in reference order
@@ -392,7 +389,7 @@ struct OnePassStep {
                         ep[q] = c0;
                     }
                     if (!in_range)
-                        errkey = min(errkey, eta_fail_key(eta_next + gidx, N, g.nstore, g.ncells, cell_of()));
+                        book.fail(eta_fail_key(eta_next + gidx, N, g.nstore, g.ncells, cell_of()));
                 }
 
                 pP = pp;   // a register: the ring slot of plane u-1 takes plane u+2 next
@@ -416,14 +413,17 @@ struct OnePassStep {
             __syncthreads();
             return false;
         }
+        const unsigned long long errkey = book.key();
         if (DM == 1 && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
-        if (errkey != ERR_NONE) atomicMin(&st->err_key, errkey);
+        if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
+        DD acc[5];
+        long long clipped = book.clipped();
+        for (int q = 0; q < 5; ++q) acc[q] = DD{book.v(2 * q), book.v(2 * q + 1)};
         block_reduce_dd<5>(acc, clipped, sdd, scnt);
         if (tid == 0) {
-            StepPartial& out = partials[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)];
+            StepPartial& out = partials[blockIdx.x];
             for (int q = 0; q < 5; ++q) { out.s[q][0] = acc[q].hi; out.s[q][1] = acc[q].lo; }
             out.clipped = clipped;
-            out.redo = 0;
         }
         return false;
     }
@@ -437,18 +437,33 @@ struct OnePassStep {
                                const CUtensorMap* m_col, const CUtensorMap* m_crn, const double* __restrict__ o,
                                const double* __restrict__ cr, const double* __restrict__ p, double* __restrict__ on,
                                double* __restrict__ crn, double* __restrict__ pn, double* __restrict__ eta_next,
-                               StepPartial* __restrict__ partials, Status* st) {
+                               StepPartial* __restrict__ partials, const StepPartial* __restrict__ prev,
+                               DevBudget* budget, Status* st, int gx, int gy, int nblocks) {
+        const int t = blockIdx.x;
+        if (budget) {
+            if (t == nblocks) {   // this CTA commits the previous step
+                extern __shared__ __align__(128) unsigned char fused_smem[];
+                DD* sdd = reinterpret_cast<DD*>(reinterpret_cast<double*>(fused_smem) + T::SMEM_DOUBLES);
+                commit_pending(prev, P.err_slot ^ 1, budget, st, sdd, reinterpret_cast<long long*>(sdd + 32 * 5));
+                return;
+            }
+            if (step_blocked(P, st)) return;
+            if (t == 0 && threadIdx.x == 0 && threadIdx.y == 0) st->pending[P.err_slot] = nblocks;
+        } else if (st->failed) {
+            return;
+        }
+        const int bx = t % gx, by = (t / gx) % gy, bz = t / (gx * gy);
         // the staging ring's mbarriers: one array for both marches (declared in
         // a march, each instantiation would have its own)
         __shared__ unsigned long long bars[L::RING];
         if (FAST) {
-            run_body<0>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials, st, bars, 0);
+            run_body<0>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials, st, bars, 0, bx, by, bz);
         } else if (run_body<1>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials, st, bars,
-                               0)) {
-            const int i0 = blockIdx.z * P.xchunk, i1 = min(P.g.nx, i0 + P.xchunk);
+                               0, bx, by, bz)) {
+            const int i0 = bz * P.xchunk, i1 = min(P.g.nx, i0 + P.xchunk);
             __syncthreads();
             run_body<2>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials, st, bars,
-                        i1 - i0 + 2);
+                        i1 - i0 + 2, bx, by, bz);
         }
     }
 };
@@ -459,8 +474,10 @@ k_step_fused(const StepParams P, const __grid_constant__ CUtensorMap m_int, cons
              const __grid_constant__ CUtensorMap m_col, const __grid_constant__ CUtensorMap m_crn,
              const double* __restrict__ o, const double* __restrict__ cr, const double* __restrict__ p,
              double* __restrict__ on, double* __restrict__ crn, double* __restrict__ pn,
-             double* __restrict__ eta_next, StepPartial* __restrict__ partials, Status* st) {
-    OnePassStep<FAST, N, MODE>::run(P, &m_int, &m_row, &m_col, &m_crn, o, cr, p, on, crn, pn, eta_next, partials, st);
+             double* __restrict__ eta_next, StepPartial* __restrict__ partials, const StepPartial* __restrict__ prev,
+             DevBudget* budget, Status* st, int gx, int gy, int nblocks) {
+    OnePassStep<FAST, N, MODE>::run(P, &m_int, &m_row, &m_col, &m_crn, o, cr, p, on, crn, pn, eta_next, partials, prev,
+                                    budget, st, gx, gy, nblocks);
 }
 
 // The flag combination k_step_fused instantiates with the flags folded (MODE 1).
@@ -475,24 +492,23 @@ inline bool fused_step_applies(const Grid& g, int n) {
 template <bool FAST, int N>
 static bool launch_step_fused_n(const StepParams& P, const double* o, const double* cr, const double* p,
                                 const double* eta, double* on, double* crn, double* pn, double* eta_next,
-                                StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out) {
+                                StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                                cudaStream_t stream, int* nblocks_out) {
     const Grid& g = P.g;
     CUtensorMap mi, mr, mc, mk;
     if (!encode_eta_map(&mi, g, N, eta, FTB, FTA, 1) || !encode_eta_map(&mr, g, N, eta, FTB, 1, 1) ||
         !encode_eta_map(&mc, g, N, eta, 2, FTA, 1) || !encode_eta_map(&mk, g, N, eta, 2, 1, N))
         return false;
     using L = FusedLayout<N>;
-    const dim3 grid(g.nb / FTB, g.na / FTA, (g.nx + P.xchunk - 1) / P.xchunk);
-    if (fused_common_mode(P)) {
-        ensure_smem_attr((const void*)k_step_fused<FAST, N, 1>, (int)L::BYTES);
-        k_step_fused<FAST, N, 1><<<grid, dim3(FTB, FTA), L::BYTES, stream>>>(P, mi, mr, mc, mk, o, cr, p, on, crn,
-                                                                            pn, eta_next, partials, st);
-    } else {
-        ensure_smem_attr((const void*)k_step_fused<FAST, N, 0>, (int)L::BYTES);
-        k_step_fused<FAST, N, 0><<<grid, dim3(FTB, FTA), L::BYTES, stream>>>(P, mi, mr, mc, mk, o, cr, p, on, crn,
-                                                                            pn, eta_next, partials, st);
-    }
-    if (nblocks_out) *nblocks_out = (int)(grid.x * grid.y * grid.z);
+    const int gx = g.nb / FTB, gy = g.na / FTA, nblocks = gx * gy * ((g.nx + P.xchunk - 1) / P.xchunk);
+    auto launch = [&](auto kernel) {
+        ensure_smem_attr((const void*)kernel, (int)L::BYTES);
+        kernel<<<nblocks + (budget ? 1 : 0), dim3(FTB, FTA), L::BYTES, stream>>>(
+            P, mi, mr, mc, mk, o, cr, p, on, crn, pn, eta_next, partials, prev, budget, st, gx, gy, nblocks);
+    };
+    if (fused_common_mode(P)) launch(k_step_fused<FAST, N, 1>);
+    else launch(k_step_fused<FAST, N, 0>);
+    if (nblocks_out) *nblocks_out = nblocks;
     return true;
 }
 
@@ -501,12 +517,13 @@ static bool launch_step_fused_n(const StepParams& P, const double* o, const doub
 template <bool FAST>
 static bool launch_step_fused_form(const StepParams& P, int n, const double* o, const double* cr, const double* p,
                                    const double* eta, double* on, double* crn, double* pn, double* eta_next,
-                                   StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out) {
-    if (!fused_step_applies(P.g, n) || P.err_slot >= 0) return false;
+                                   StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                                   cudaStream_t stream, int* nblocks_out) {
+    if (!fused_step_applies(P.g, n) || P.slab) return false;
     if ((reinterpret_cast<unsigned long long>(eta) & 15ull) != 0) return false;
     switch (n) {
 #define NICR_FUSED_STEP_CASE(k) \
-    case k: return launch_step_fused_n<FAST, k>(P, o, cr, p, eta, on, crn, pn, eta_next, partials, st, stream, nblocks_out);
+    case k: return launch_step_fused_n<FAST, k>(P, o, cr, p, eta, on, crn, pn, eta_next, partials, prev, budget, st, stream, nblocks_out);
         NICR_FUSED_STEP_CASE(1) NICR_FUSED_STEP_CASE(2) NICR_FUSED_STEP_CASE(3) NICR_FUSED_STEP_CASE(4)
         NICR_FUSED_STEP_CASE(5) NICR_FUSED_STEP_CASE(6) NICR_FUSED_STEP_CASE(7) NICR_FUSED_STEP_CASE(8)
 #undef NICR_FUSED_STEP_CASE

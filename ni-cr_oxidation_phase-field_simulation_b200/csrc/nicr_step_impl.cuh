@@ -50,23 +50,82 @@ __device__ void block_reduce_dd(DD (&v)[N], long long& cnt, DD* sdd, long long* 
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
     const int nthreads = blockDim.x * blockDim.y * blockDim.z;
     const int w = tid >> 5, nw = (nthreads + 31) >> 5;
+    // Most CTAs of a step book nothing, and few warps of the others do: warps
+    // without a nonzero value skip their shuffles, CTAs without one everything
+    // (a double-double sum with zeros is exact, so the result is the same).
+    bool nz = cnt != 0;
+    for (int q = 0; q < N; ++q) nz = nz || v[q].hi != 0. || v[q].lo != 0.;
+    if (!__syncthreads_or(nz)) return;
     // lanes of a warp are consecutive linear thread ids because blockDim.x is a multiple of 32
-    for (int off = 16; off > 0; off >>= 1) {
-        for (int q = 0; q < N; ++q) v[q] = dd_add(v[q], shfl_dd(v[q], off));
-        cnt += __shfl_down_sync(0xffffffffu, cnt, off);
-    }
+    const bool any = __any_sync(0xffffffffu, nz);
+    if (any)
+        for (int off = 16; off > 0; off >>= 1) {
+            for (int q = 0; q < N; ++q) v[q] = dd_add(v[q], shfl_dd(v[q], off));
+            cnt += __shfl_down_sync(0xffffffffu, cnt, off);
+        }
     if (lane == 0) {
         for (int q = 0; q < N; ++q) sdd[w * N + q] = v[q];
-        scnt[w] = cnt;
+        scnt[w] = any ? cnt : -1;   // -1: nothing from this warp
     }
     __syncthreads();
     if (tid == 0) {
-        for (int q = 0; q < N; ++q) v[q] = sdd[q];
-        cnt = scnt[0];
-        for (int ww = 1; ww < nw; ++ww) {
+        for (int q = 0; q < N; ++q) v[q] = DD{0., 0.};
+        cnt = 0;
+        for (int ww = 0; ww < nw; ++ww) {
+            if (scnt[ww] < 0) continue;
             for (int q = 0; q < N; ++q) v[q] = dd_add(v[q], sdd[ww * N + q]);
             cnt += scnt[ww];
         }
+    }
+}
+
+// Whether this step must not run: a step of this batch was rejected, or the
+// previous one just was (its commit has not run yet).
+__device__ __forceinline__ bool step_blocked(const StepParams& P, const Status* st) {
+    return st->failed || (!P.slab && P.err_slot >= 0 && st->slot_err[P.err_slot ^ 1] != ERR_NONE);
+}
+
+// Commits the pending step of parity q, if any, by one CTA: partial sums
+// (thread t: partials t, t + nthreads, ...; deterministic), then the budget is
+// advanced only when no trial failed (fields swap only on acceptance, 3S:821).
+// sdd, scnt: block_reduce_dd's scratch.
+__device__ __forceinline__ void commit_pending(const StepPartial* __restrict__ partials, int q_par, DevBudget* budget,
+                                               Status* st, DD* sdd, long long* scnt) {
+    const int tid = threadIdx.x + blockDim.x * threadIdx.y, nthreads = blockDim.x * blockDim.y;
+    const int nblocks = st->pending[q_par];
+    if (nblocks == 0) return;
+    const unsigned long long key = st->slot_err[q_par];
+    __syncthreads();
+    if (key != ERR_NONE) {
+        if (tid == 0) {
+            st->err_key = key;
+            st->failed = 1;
+            st->failed_step = st->steps_done;
+            st->pending[q_par] = 0;
+        }
+        return;
+    }
+    DD acc[5] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
+    long long clipped = 0;
+    for (int b = tid; b < nblocks; b += nthreads) {
+        for (int q = 0; q < 5; ++q) {
+            const DD v{partials[b].s[q][0], partials[b].s[q][1]};
+            if (v.hi != 0. || v.lo != 0.) acc[q] = dd_add(acc[q], v);
+        }
+        clipped += partials[b].clipped;
+    }
+    block_reduce_dd<5>(acc, clipped, sdd, scnt);
+    if (tid == 0) {
+        // slots: ckO ckCr clipO clipCr bcO -> budget indices 2 3 4 5 6
+        for (int q = 0; q < 5; ++q) {
+            DD b{budget->v[2 + q][0], budget->v[2 + q][1]};
+            b = dd_add(b, acc[q]);
+            budget->v[2 + q][0] = b.hi;
+            budget->v[2 + q][1] = b.lo;
+        }
+        budget->clipped += clipped;
+        st->steps_done += 1;
+        st->pending[q_par] = 0;
     }
 }
 
@@ -80,8 +139,9 @@ struct Tile {
     static constexpr int S2 = RA2 * RB2, S1 = RA1 * RB1;
     // shared memory: o[4], cr[4] (halo 2); p[3] (halo 1); muO, muCr, mo, mc [2] (halo 1)
     static constexpr int SMEM_DOUBLES = 8 * S2 + 3 * S1 + 8 * S1;
-    static constexpr size_t SMEM_BYTES = SMEM_DOUBLES * sizeof(double) + 64 * (5 * 16 + 8);
     static constexpr int NT = TA * TB;
+    static constexpr int SCRATCH_DOUBLES = 32 * (5 * 2 + 1);   // the block reduction's (32 warps x 5 DD + counts)
+    static constexpr size_t SMEM_BYTES = (SMEM_DOUBLES + SCRATCH_DOUBLES + 12 * NT) * sizeof(double);   // and the books
     // every thread stages at most two points of each halo tile
     static_assert(2 * NT >= S2 && 2 * NT >= S1, "tile halo larger than two points per thread");
     __device__ static int i2(int a, int b) { return (a + HA2) * RB2 + (b + 2); }
@@ -201,6 +261,53 @@ __device__ __forceinline__ unsigned long long eta_fail_key(const double* eta_nex
             return ERR_ETA_BASE + (unsigned long long)q * (unsigned long long)key_ncells + (unsigned long long)cell;
     return ERR_NONE;
 }
+
+// A thread's budget sums (ckO ckCr clipO clipCr bcO, hi and lo), clipped cells
+// and first failing trial, kept out of the registers: few cells touch them,
+// and 24 registers across the march made the exact forms spill. Slot q of the
+// 12 words lies NT words after slot q - 1, so the threads' slots of one kind
+// are neighbours. SharedBook: in shared memory (the step kernel). LocalBook:
+// in local memory (the one-pass kernel, whose tile fills shared memory and
+// whose chunks are long enough to hide it; in the step kernel its traffic cost
+// 8% on the 151 x 101 x 101 grid).
+template <int NT>
+struct SharedBook {
+    double* w;
+    __device__ explicit SharedBook(double* base) : w(base) {
+        for (int q = 0; q < 11; ++q) w[q * NT] = 0.;   // the clipped count's zero bits too
+        key() = ERR_NONE;
+    }
+    __device__ double& v(int q) { return w[q * NT]; }
+    __device__ long long& clipped() { return *reinterpret_cast<long long*>(w + 10 * NT); }
+    __device__ unsigned long long& key() { return *reinterpret_cast<unsigned long long*>(w + 11 * NT); }
+    __device__ void add(int q, double b) {
+        const DD r = dd_add(DD{v(2 * q), v(2 * q + 1)}, b);
+        v(2 * q) = r.hi;
+        v(2 * q + 1) = r.lo;
+    }
+    __device__ void clip() { clipped() += 1; }
+    __device__ void fail(unsigned long long k) { key() = min(key(), k); }
+};
+struct LocalBook {
+    volatile double w[10];
+    volatile long long n;
+    volatile unsigned long long k0;
+    __device__ LocalBook() {
+        for (int q = 0; q < 10; ++q) w[q] = 0.;
+        n = 0;
+        k0 = ERR_NONE;
+    }
+    __device__ double v(int q) { return w[q]; }
+    __device__ long long clipped() { return n; }
+    __device__ unsigned long long key() { return k0; }
+    __device__ void add(int q, double b) {
+        const DD r = dd_add(DD{w[2 * q], w[2 * q + 1]}, b);
+        w[2 * q] = r.hi;
+        w[2 * q + 1] = r.lo;
+    }
+    __device__ void clip() { n = n + 1; }
+    __device__ void fail(unsigned long long k) { k0 = min((unsigned long long)k0, k); }
+};
 
 struct CenterVals {
     double o, cr, p, hh, muO, muCr, mo, mc;   // hh = h(p), reused by Ck
@@ -518,9 +625,9 @@ struct StepKernel {
     // others, and cells with Ck increments, take the branch after the stores,
     // which stores again what the clamps change. cell(): the cell's index in
     // reference loop order.
-    template <class CellFn>
+    template <class Book, class CellFn>
     __device__ static void finish_cell(const CoreOut& R, bool bounds_legacy, double* on, double* crn, double* pn,
-                                       DD (&acc)[5], long long& clipped, unsigned long long& errkey, CellFn cell) {
+                                       Book& book, CellFn cell) {
         const unsigned ho = (unsigned)__double2hiint(R.onv), hc = (unsigned)__double2hiint(R.crv),
                        hp = (unsigned)__double2hiint(R.pnv);
         double pnv = R.pnv;
@@ -544,22 +651,22 @@ struct StepKernel {
                 const double oc = sclamp(R.onv, 0., 1.), ccr = sclamp(R.crv, 0., 1.);
                 const double clO = oc - R.onv, clCr = ccr - R.crv;
                 if (oc != R.onv || ccr != R.crv) {
-                    ++clipped;
+                    book.clip();
                     *on = oc;
                     *crn = ccr;
                 }
                 // adding +-0 to a normalised double-double leaves it unchanged,
                 // so zero increments are skipped
-                if (clO != 0.) acc[2] = dd_add(acc[2], clO);
-                if (clCr != 0.) acc[3] = dd_add(acc[3], clCr);
+                if (clO != 0.) book.add(2, clO);
+                if (clCr != 0.) book.add(3, clCr);
             } else {
                 outside = R.onv < -1.e-12 || R.crv < -1.e-12 || R.onv + R.crv > 1. + 1.e-12 || R.pnv < -1.e-12 ||
                           R.pnv > 1. + 1.e-12;
             }
             if (nonfinite || outside)
-                errkey = min(errkey, (unsigned long long)cell() * 4ull + (nonfinite ? 0ull : 1ull));
-            if (R.dO != 0.) acc[0] = dd_add(acc[0], R.dO);
-            if (R.dCr != 0.) acc[1] = dd_add(acc[1], R.dCr);
+                book.fail((unsigned long long)cell() * 4ull + (nonfinite ? 0ull : 1ull));
+            if (R.dO != 0.) book.add(0, R.dO);
+            if (R.dCr != 0.) book.add(1, R.dCr);
         }
     }
     // The X face between two cells as the march carries it: the flux in the
@@ -571,9 +678,9 @@ struct StepKernel {
     }
     // The surface-mobility closure of the O face at X = 0 with bc=mu
     // (left_flux, 3S:621-628): the carried face, and the budget's increment.
-    template <class Dv>
+    template <class Dv, class Book>
     __device__ static double surface_face(const Dv& dv, const StepParams& P, bool o_on, const CenterVals& C, double gb0,
-                                          DD& booked) {
+                                          Book& book) {
         double lf = 0., carry = 0., inc;
         if (o_on) {
             const double mf = mobility(P.surface_c_ref, h(C.p), gb0, Phys::bmo, Phys::boo, P.gbm1_o);
@@ -587,7 +694,7 @@ struct StepKernel {
         }
         if constexpr (Dv::kFast) inc = (P.dt * lf) * P.f.rdx;
         else inc = dv.plain_checked(P.dt * lf, P.div.dx);
-        booked = dd_add(booked, inc);
+        book.add(4, inc);
         return carry;
     }
     // One march over the CTA's chunk with the division policy of DM (DivOf).
@@ -619,11 +726,8 @@ struct StepKernel {
         const bool active = (DIM == 3 ? row < g.na : true) && col < g.nb;
         const Offs offs = make_offs(g, a0, b0);
 
-        DD acc[5] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};  // ckO ckCr clipO clipCr bcO
-        long long clipped = 0;
-        unsigned long long errkey = ERR_NONE;
+        SharedBook<T::NT> book(smem + T::SMEM_DOUBLES + T::SCRATCH_DOUBLES + ta * TB + tb);
 
-        if (st->failed) return false;  // a previous step of this batch was rejected
         unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
         const typename DivOf<DM>::T dv{P, low};
 
@@ -731,15 +835,15 @@ struct StepKernel {
                 const long long gidx = (long long)u * g.plane + (long long)row * g.pb + col;
                 double leftO = FxO;
                 if (u == 0 && P.bc == 1) {
-                    leftO = surface_face(dv, P, P.o_on != 0, C, P.grains ? __ldg(gb + gidx) : 0., acc[4]);
+                    leftO = surface_face(dv, P, P.o_on != 0, C, P.grains ? __ldg(gb + gidx) : 0., book);
                 }
-                if (u == 0 && P.inlet) acc[4] = dd_add(acc[4], P.layer_o - __ldg(o + gidx));
+                if (u == 0 && P.inlet) book.add(4, P.layer_o - __ldg(o + gidx));
 
                 // fluxes, phi force and Ck (3S:761-811)
                 const CoreOut R = cell_core(dv, P, P.o_on != 0, P.ck == 0, P.phi_eta != 0, C, L, pP, leftO, FxCr,
                                             s2u, mO, mC, mo_, mc_, spu, c1, bp, bm, ap, am);
                 FxO = R.rightO; FxCr = R.rightCr;
-                finish_cell(R, P.bounds == 1, on + gidx, crn + gidx, pn + gidx, acc, clipped, errkey, [&]() {
+                finish_cell(R, P.bounds == 1, on + gidx, crn + gidx, pn + gidx, book, [&]() {
                     return ((long long)u * g.na + row) * g.nb + col + (SLAB ? P.cell_off : 0);
                 });
             }
@@ -747,39 +851,51 @@ struct StepKernel {
             C = L;
             s2u = s2n;
         }
+        const unsigned long long errkey = book.key();
         if (DM == 1 && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
-        if (errkey != ERR_NONE) atomicMin(SLAB ? err_word(P, st) : &st->err_key, errkey);
+        if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
+        DD acc[5];
+        long long clipped = book.clipped();
+        for (int q = 0; q < 5; ++q) acc[q] = DD{book.v(2 * q), book.v(2 * q + 1)};
         block_reduce_dd<5>(acc, clipped, sdd, scnt);
         if (threadIdx.x == 0 && threadIdx.y == 0) {
             StepPartial& out = partials[blin];
             for (int q = 0; q < 5; ++q) { out.s[q][0] = acc[q].hi; out.s[q][1] = acc[q].lo; }
             out.clipped = clipped;
-            out.redo = 0;
         }
         return false;
     }
 
-    // One CTA's chunk. In the drop-in form a chunk whose numerators left the
-    // guarded range is marched again with every quotient exact (IEEE division
-    // for those), rewriting its trial values, before keys and partials are
-    // published: here (DEFER false), or by k_step_redo after the launch
-    // (DEFER true: the CTA only marks its partial slot), which keeps the
-    // second march and its division calls out of the hot kernel.
-    template <bool DEFER = false>
+    // One CTA's chunk of a step of nblocks CTAs (this one at blin); with a
+    // budget, CTA nblocks commits the previous step instead: a commit in its
+    // own launch, or by the step's last CTA, cost 5 us per step between steps
+    // of 8 (2D 128^2) to 30 us (64^3). In the drop-in form a chunk whose quotients
+    // could not all be certified is marched again with every quotient exact
+    // (IEEE division for those), rewriting its trial values, before keys and
+    // partials are published.
     __device__ static void run(const StepParams& P, const double* __restrict__ o, const double* __restrict__ cr,
                                const double* __restrict__ p, const double* __restrict__ gb,
                                const double* __restrict__ s2, double* __restrict__ on,
                                double* __restrict__ crn, double* __restrict__ pn,
-                               StepPartial* __restrict__ partials, Status* st, int bx, int by, int bz, int blin) {
+                               StepPartial* __restrict__ partials, const StepPartial* __restrict__ prev,
+                               DevBudget* budget, Status* st, int bx, int by, int bz, int blin, int nblocks) {
+        if (!SLAB && budget) {
+            if (blin == nblocks) {
+                extern __shared__ __align__(16) double smem[];
+                DD* sdd = reinterpret_cast<DD*>(smem + T::SMEM_DOUBLES);
+                commit_pending(prev, P.err_slot ^ 1, budget, st, sdd, reinterpret_cast<long long*>(sdd + 32 * 5));
+                return;
+            }
+            if (step_blocked(P, st)) return;
+            if (blin == 0 && threadIdx.x == 0 && threadIdx.y == 0) st->pending[P.err_slot] = nblocks;
+        } else if (st->failed) {
+            return;
+        }
         if (FAST) {
             run_body<0>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
         } else if (run_body<1>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin)) {
-            if (DEFER) {
-                if (threadIdx.x == 0 && threadIdx.y == 0) partials[blin].redo = 1;
-            } else {
-                __syncthreads();
-                run_body<2>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
-            }
+            __syncthreads();
+            run_body<2>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
         }
     }
 };
@@ -789,29 +905,11 @@ __global__ void __launch_bounds__(TA * TB, MINB)
 k_step_main(const StepParams P, const double* __restrict__ o, const double* __restrict__ cr,
             const double* __restrict__ p, const double* __restrict__ gb, const double* __restrict__ s2,
             double* __restrict__ on, double* __restrict__ crn, double* __restrict__ pn,
-            StepPartial* __restrict__ partials, Status* st) {
-    StepKernel<DIM, TA, TB, FAST, SLAB>::template run<true>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, blockIdx.x,
-                                                            blockIdx.y, blockIdx.z,
-                                                            blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
-}
-
-// The drop-in form's recomputation of the chunks k_step_main marked (numerators
-// outside the exact-division range, which its march only flags): each CTA
-// takes marked chunks of the step grid (gx x gy x gz CTAs) in turn and marches
-// them with every quotient exact, rewriting trial values, key and partials.
-template <int DIM, int TA, int TB, bool SLAB = false>
-__global__ void __launch_bounds__(TA * TB, 1)
-k_step_redo(const StepParams P, const double* __restrict__ o, const double* __restrict__ cr,
-            const double* __restrict__ p, const double* __restrict__ gb, const double* __restrict__ s2,
-            double* __restrict__ on, double* __restrict__ crn, double* __restrict__ pn,
-            StepPartial* __restrict__ partials, Status* st, int gx, int gy, int nblocks) {
-    for (int blin = blockIdx.x; blin < nblocks; blin += gridDim.x) {
-        if (!partials[blin].redo) continue;   // the same word for the whole CTA
-        __syncthreads();                      // the previous chunk's shared-memory reads are done
-        StepKernel<DIM, TA, TB, false, SLAB>::template run_body<2>(P, o, cr, p, gb, s2, on, crn, pn, partials, st,
-                                                                   blin % gx, (blin / gx) % gy, blin / (gx * gy),
-                                                                   blin);
-    }
+            StepPartial* __restrict__ partials, const StepPartial* __restrict__ prev, DevBudget* budget, Status* st,
+            int gx, int gy, int nblocks) {
+    const int t = blockIdx.x;
+    StepKernel<DIM, TA, TB, FAST, SLAB>::run(P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, t % gx,
+                                             (t / gx) % gy, t / (gx * gy), t, nblocks);
 }
 
 constexpr int TA3 = 8, TB3 = 32;    // 3D tile: 8 rows x 32 columns, 256 threads
@@ -894,7 +992,7 @@ __global__ void __launch_bounds__(256, 5) k_eta_update(const StepParams P, int n
                              const double* __restrict__ s2, const double* __restrict__ p,
                              double* __restrict__ eta_next, double* __restrict__ gb_next,
                              double* __restrict__ s2_next, Status* st) {
-    if (st->failed) return;
+    if (step_blocked(P, st)) return;
     const Grid& g = P.g;
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = DIM == 3 ? blockIdx.y * blockDim.y + threadIdx.y : 0;
@@ -1001,7 +1099,7 @@ __device__ __forceinline__ void eta_march_body(const StepParams& P, int n, const
                                                const double* __restrict__ p, double* __restrict__ eta_next,
                                                double* __restrict__ gb_next, double* __restrict__ s2_next,
                                                Status* st, int bx, int by, int bz) {
-    if (st->failed) return;
+    if (step_blocked(P, st)) return;
     const Grid& g = P.g;
     const int col = bx * blockDim.x + threadIdx.x;
     const int row = DIM == 3 ? by * blockDim.y + threadIdx.y : 0;
@@ -1015,7 +1113,7 @@ __device__ __forceinline__ void eta_march_body(const StepParams& P, int n, const
         errkey = ERR_NONE;
         eta_march_pass<DIM, 2, NCAP, SLAB>(P, n, eta, p, eta_next, gb_next, s2_next, row, col, i0, i1, errkey);
     }
-    if (errkey != ERR_NONE) atomicMin(SLAB ? err_word(P, st) : &st->err_key, errkey);
+    if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
 }
 
 // 2 CTAs/SM stated in the bounds: the register count stays <= 128 either way,
@@ -1034,7 +1132,7 @@ static void launch_eta_march(const StepParams& P, const double* eta, const doubl
     const Grid& g = P.g;
     if (DIM == 3) {
         const dim3 grid((g.nb + 31) / 32, (g.na + 7) / 8, (P.x_hi - P.x_lo + P.xchunk - 1) / P.xchunk);
-        if (P.err_slot >= 0)   // an X slab (3D only)
+        if (P.slab)   // 3D only
             k_eta_march<3, FAST, N, true><<<grid, dim3(32, 8), 0, stream>>>(P, eta, p, eta_next, gb_next, s2_next, st);
         else
             k_eta_march<3, FAST, N><<<grid, dim3(32, 8), 0, stream>>>(P, eta, p, eta_next, gb_next, s2_next, st);
@@ -1085,8 +1183,10 @@ k_step_eta(const StepParams P, const FusedStep F, const double* __restrict__ o, 
     }
     if (role == 0) {
         const int bx = idx % F.gx_s, r = idx / F.gx_s;
-        StepKernel<3, TA3, TB3, FAST>::run(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, r % F.gy_s,
-                                           r / F.gy_s, idx);
+        // this launch commits nothing: it leaves its step pending (the one before was flushed)
+        if (idx == 0 && threadIdx.x == 0 && threadIdx.y == 0 && !st->failed) st->pending[P.err_slot] = F.n_step;
+        StepKernel<3, TA3, TB3, FAST>::run(P, o, cr, p, gb, s2, on, crn, pn, partials, nullptr, nullptr, st, bx,
+                                           r % F.gy_s, r / F.gy_s, idx, F.n_step);
     } else {
         const int bx = idx % F.gx_e, r = idx / F.gx_e;
         eta_march_body<3, FAST, N>(P, N, eta, p, eta_next, gb_next, s2_next, st, bx, r % F.gy_e, r / F.gy_e);
@@ -1134,7 +1234,7 @@ static bool launch_step_eta_form(const StepParams& P, int neta, const double* o,
                                  StepPartial* partials, const double* eta, double* eta_next, double* gb_next,
                                  double* s2_next, unsigned* ticket, Status* st, cudaStream_t stream,
                                  int* nblocks_out) {
-    if (P.g.dim != 3 || P.err_slot >= 0) return false;
+    if (P.g.dim != 3 || P.slab) return false;
     switch (neta) {
 #define NICR_FUSED_CASE(n)                                                                                   \
     case n:                                                                                                  \
@@ -1232,7 +1332,7 @@ k_eta_tma(const StepParams P, const __grid_constant__ CUtensorMap m_int, const _
     constexpr int TA = S::TA, TB = S::TB;
     extern __shared__ unsigned char tma_smem_raw[];
     __shared__ unsigned long long bars[kTmaRing];
-    if (st->failed) return;
+    if (step_blocked(P, st)) return;
     const Grid& g = P.g;
     double* ring = reinterpret_cast<double*>(((unsigned long long)tma_smem_raw + 127ull) & ~127ull);
     const int ta = threadIdx.y, tb = threadIdx.x, tid = tb + TB * ta;
@@ -1343,7 +1443,7 @@ k_eta_tma(const StepParams P, const __grid_constant__ CUtensorMap m_int, const _
         __syncthreads();
         return;
     }
-    if (errkey != ERR_NONE) atomicMin(&st->err_key, errkey);
+    if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (the
@@ -1423,7 +1523,7 @@ k_eta_stream(const StepParams P, int neta, const double* __restrict__ eta, const
     constexpr int HA = DIM == 3 ? 1 : 0;
     constexpr int RA = TA + 2 * HA, RB = TB + 2, S1 = RA * RB, NT = TA * TB;
     extern __shared__ __align__(16) double ring[];   // [3][neta][S1], then S1 int offsets
-    if (st->failed) return;
+    if (step_blocked(P, st)) return;
     const Grid& g = P.g;
     const int ta = DIM == 3 ? threadIdx.y : 0, tb = threadIdx.x;
     const int a0 = DIM == 3 ? blockIdx.y * TA : 0, b0 = blockIdx.x * TB;
@@ -1487,7 +1587,7 @@ k_eta_stream(const StepParams P, int neta, const double* __restrict__ eta, const
         }
         __syncthreads();   // slot(u-1) is refilled with plane u+2 next
     }
-    if (errkey != ERR_NONE) atomicMin(&st->err_key, errkey);
+    if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
 }
 
 // Batched step: one launch advances up to kBatchMax domains of one
@@ -1514,10 +1614,11 @@ __global__ void __launch_bounds__(TA * TB, MINB) k_step_batch_slim(const __grid_
     P.inlet = D.inlet;
     P.x_hi = D.x_hi;
     P.key_ncells = D.key_ncells;
+    P.err_slot = D.err_slot;
     const int t = (int)blockIdx.x - D.block0;
     const int bx = t % D.gx, r = t / D.gx, by = r % D.gy, bz = r / D.gy;
-    StepKernel<DIM, TA, TB, FAST>::run(P, D.o, D.cr, D.p, D.gb, D.s2, D.on, D.crn, D.pn, D.partials, D.st, bx, by,
-                                       bz, t);
+    StepKernel<DIM, TA, TB, FAST>::run(P, D.o, D.cr, D.p, D.gb, D.s2, D.on, D.crn, D.pn, D.partials, D.prev,
+                                       D.budget, D.st, bx, by, bz, t, D.nblocks);
 }
 
 template <int DIM, int TA, int TB, int MINB, bool FAST>
@@ -1531,8 +1632,8 @@ __global__ void __launch_bounds__(TA * TB, MINB) k_step_batch(const __grid_const
     const BatchDomain& D = B.d[lo];
     const int t = (int)blockIdx.x - D.block0;
     const int bx = t % D.gx, r = t / D.gx, by = r % D.gy, bz = r / D.gy;
-    StepKernel<DIM, TA, TB, FAST>::run(D.sp, D.o, D.cr, D.p, D.gb, D.s2, D.on, D.crn, D.pn, D.partials, D.st, bx, by,
-                                       bz, t);
+    StepKernel<DIM, TA, TB, FAST>::run(D.sp, D.o, D.cr, D.p, D.gb, D.s2, D.on, D.crn, D.pn, D.partials,
+                                       D.prev, D.budget, D.st, bx, by, bz, t, D.nblocks);
 }
 
 }  // namespace
@@ -1558,58 +1659,39 @@ static int step_minb() {
 }
 static int step_minb_for(const StepParams& P) { return P.minb == 2 || P.minb == 3 ? P.minb : step_minb(); }
 
-// CTAs per SM of the recomputation kernel (its grid strides over the step grid)
-constexpr int kRedoCtasPerSm = 2;
-
-template <int MINB, bool FAST>
-static void launch_step3(const StepParams& P, const double* o, const double* cr, const double* p, const double* gb,
-                         const double* s2, double* on, double* crn, double* pn, StepPartial* partials, Status* st,
-                         cudaStream_t stream, int* nblocks_out) {
-    using T = Tile<3, TA3, TB3>;
-    const dim3 grid = step_grid<3, TA3, TB3>(P);
+template <int DIM, int TA, int TB, int MINB, bool FAST, bool SLAB>
+static void launch_step_n(const StepParams& P, const double* o, const double* cr, const double* p, const double* gb,
+                          const double* s2, double* on, double* crn, double* pn, StepPartial* partials,
+                          const StepPartial* prev, DevBudget* budget, Status* st, cudaStream_t stream,
+                          int* nblocks_out) {
+    using T = Tile<DIM, TA, TB>;
+    const dim3 grid = step_grid<DIM, TA, TB>(P);
     const int nblocks = (int)(grid.x * grid.y * grid.z);
-    const int gredo = std::min(nblocks, kRedoCtasPerSm * 148);
-    if (P.err_slot >= 0) {   // an X slab
-        ensure_smem_attr((const void*)k_step_main<3, TA3, TB3, MINB, FAST, true>, (int)T::SMEM_BYTES);
-        k_step_main<3, TA3, TB3, MINB, FAST, true><<<grid, dim3(TB3, TA3), T::SMEM_BYTES, stream>>>(
-            P, o, cr, p, gb, s2, on, crn, pn, partials, st);
-        if constexpr (!FAST) {
-            ensure_smem_attr((const void*)k_step_redo<3, TA3, TB3, true>, (int)T::SMEM_BYTES);
-            k_step_redo<3, TA3, TB3, true><<<gredo, dim3(TB3, TA3), T::SMEM_BYTES, stream>>>(
-                P, o, cr, p, gb, s2, on, crn, pn, partials, st, (int)grid.x, (int)grid.y, nblocks);
-        }
-    } else {
-        ensure_smem_attr((const void*)k_step_main<3, TA3, TB3, MINB, FAST>, (int)T::SMEM_BYTES);
-        k_step_main<3, TA3, TB3, MINB, FAST><<<grid, dim3(TB3, TA3), T::SMEM_BYTES, stream>>>(P, o, cr, p, gb, s2, on,
-                                                                                             crn, pn, partials, st);
-        if constexpr (!FAST) {
-            ensure_smem_attr((const void*)k_step_redo<3, TA3, TB3>, (int)T::SMEM_BYTES);
-            k_step_redo<3, TA3, TB3><<<gredo, dim3(TB3, TA3), T::SMEM_BYTES, stream>>>(
-                P, o, cr, p, gb, s2, on, crn, pn, partials, st, (int)grid.x, (int)grid.y, nblocks);
-        }
-    }
+    ensure_smem_attr((const void*)k_step_main<DIM, TA, TB, MINB, FAST, SLAB>, (int)T::SMEM_BYTES);
+    k_step_main<DIM, TA, TB, MINB, FAST, SLAB><<<nblocks + (budget ? 1 : 0), dim3(TB, TA), T::SMEM_BYTES, stream>>>(
+        P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, (int)grid.x, (int)grid.y, nblocks);
     if (nblocks_out) *nblocks_out = nblocks;
 }
 
 template <bool FAST>
 static void launch_step_form(const StepParams& P, const double* o, const double* cr, const double* p,
                              const double* gb, const double* s2, double* on, double* crn, double* pn,
-                             StepPartial* partials, Status* st, cudaStream_t stream, int* nblocks_out) {
+                             StepPartial* partials, const StepPartial* prev, DevBudget* budget, Status* st,
+                             cudaStream_t stream, int* nblocks_out) {
+#define NICR_STEP_FORM_ARGS P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, stream, nblocks_out
     if (P.g.dim == 3) {
-        if (step_minb_for(P) == 3) launch_step3<3, FAST>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, stream, nblocks_out);
-        else launch_step3<2, FAST>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, stream, nblocks_out);
+        const bool m3 = step_minb_for(P) == 3;
+        if (P.slab) {
+            if (m3) launch_step_n<3, TA3, TB3, 3, FAST, true>(NICR_STEP_FORM_ARGS);
+            else launch_step_n<3, TA3, TB3, 2, FAST, true>(NICR_STEP_FORM_ARGS);
+        } else {
+            if (m3) launch_step_n<3, TA3, TB3, 3, FAST, false>(NICR_STEP_FORM_ARGS);
+            else launch_step_n<3, TA3, TB3, 2, FAST, false>(NICR_STEP_FORM_ARGS);
+        }
     } else {
-        using T = Tile<2, TA2, TB2>;
-        const dim3 grid = step_grid<2, TA2, TB2>(P);
-        k_step_main<2, TA2, TB2, 4, FAST><<<grid, dim3(TB2, TA2), T::SMEM_BYTES, stream>>>(P, o, cr, p, gb, s2, on,
-                                                                                          crn, pn, partials, st);
-        const int nblocks = (int)(grid.x * grid.y * grid.z);
-        if constexpr (!FAST)
-            k_step_redo<2, TA2, TB2><<<std::min(nblocks, kRedoCtasPerSm * 148), dim3(TB2, TA2), T::SMEM_BYTES,
-                                       stream>>>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, (int)grid.x,
-                                                 (int)grid.y, nblocks);
-        if (nblocks_out) *nblocks_out = nblocks;
+        launch_step_n<2, TA2, TB2, 4, FAST, false>(NICR_STEP_FORM_ARGS);
     }
+#undef NICR_STEP_FORM_ARGS
 }
 
 template <bool FAST>
@@ -1630,7 +1712,7 @@ static void launch_eta_form(const StepParams& P, int neta, const double* eta, co
         march = e ? (e[0] == 'm' ? 1 : 0) : -2;
         tma = (e && e[0] == 't') ? 1 : 0;
     }
-    const bool slab = P.err_slot >= 0;   // X slabs use the march or the per-cell kernel
+    const bool slab = P.slab != 0;   // X slabs use the march or the per-cell kernel
     if (tma && !slab && launch_eta_tma<FAST>(neta, P, eta, p, eta_next, gb_next, s2_next, st, stream)) return;
     if (march == 1 || (march == -2 && FAST)) {
         const bool done = g.dim == 3 ? eta_march_dispatch<3, FAST>(neta, P, eta, p, eta_next, gb_next, s2_next, st, stream)
