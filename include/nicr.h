@@ -470,8 +470,8 @@ int nicr_conv3d_fwd_act(const void* x, const void* w, const float* bias, int act
                         int cin, int cout, void* stream);
 /* The same from a staged halo block (Cout <= 64 and rows of at least 128
  * voxels, else NICR_ERR_INVALID_ARG); nicr_conv3d_fwd_act and
- * nicr_conv3d_fwd use it for Cout <= 32 with Cin x Cout <= 768, where it is
- * the faster form. */
+ * nicr_conv3d_fwd use it for Cout <= 32 with Cin x Cout <= 768 where
+ * nicr_conv3d_fwd_shift does not apply. */
 int nicr_conv3d_fwd_halo(const void* x, const void* w, const float* bias, int act, void* y, int n, int d, int h, int w_,
                          int cin, int cout, void* stream);
 /* The halo-block forward marching along y (a CTA keeps its input lines and
@@ -480,6 +480,25 @@ int nicr_conv3d_fwd_halo(const void* x, const void* w, const float* bias, int ac
  * nicr_conv3d_fwd use it for Cin 16, where it is the fastest form. */
 int nicr_conv3d_fwd_march(const void* x, const void* w, const float* bias, int act, void* y, int n, int d, int h,
                           int w_, int cin, int cout, void* stream);
+/* The forward that stages each input line once for its output lines and its
+ * three x taps (Cout <= 64, else NICR_ERR_INVALID_ARG), with the same sums in
+ * the same order as the form nicr_conv3d_fwd_act used for the shape before. */
+int nicr_conv3d_fwd_shift(const void* x, const void* w, const float* bias, int act, void* y, int n, int d, int h, int w_,
+                          int cin, int cout, void* stream);
+/* Elementwise passes around the convolutions, one kernel each (16-byte aligned
+ * arrays, channels a multiple of 8; NICR_ERR_INVALID_ARG otherwise):
+ *   act_bwd   g = gy * (y > 0) as BF16 (y NULL: g = gy) and gb[c] = the column
+ *             sums of g (FP32, partial: nicr_conv3d_act_bwd_blocks() x c floats
+ *             of scratch); gy and y BF16 or FP32, c <= 2048
+ *   avgpool2  2x2x2 average of BF16 NDHWC (even d, h, w of the input)
+ *   upcat     [nearest 2x of a, b] along the channels, BF16 (d, h, w of the output)
+ *   pad16     FP32 rows of f <= 16 values as 16 BF16 channels, zero-filled */
+int nicr_conv3d_act_bwd_blocks(void);
+int nicr_conv3d_act_bwd(const void* gy, int gy_bf16, const void* y, int y_bf16, void* g, float* partial, float* gb,
+                        long long rows, int c, void* stream);
+int nicr_avgpool2_ndhwc(const void* x, void* y, int n, int d, int h, int w, int c, void* stream);
+int nicr_upcat_ndhwc(const void* a, const void* b, void* y, int n, int d, int h, int w, int ca, int cb, void* stream);
+int nicr_pad16(const float* x, void* y, long long rows, int f, void* stream);
 int nicr_conv3d_fwd_gather(const void* x, const void* w, float* y, int n, int d, int h, int w_, int cin, int cout,
                            void* stream);
 int nicr_conv3d_fwd_mma_sync(const void* x, const void* w, float* y, int n, int d, int h, int w_, int cin, int cout,

@@ -14,6 +14,7 @@
 // Every tcgen05 form keeps its accumulator in TMEM. Forward forms, chosen by
 // shape in nicr_conv3d_fwd_act from measured rates:
 //   k_conv3d_fwd_march  Cin 16, rows >= 128: halo lines kept on chip along y
+//   k_conv3d_fwd_shift  narrow outputs: input lines staged once, x taps as row shifts
 //   k_conv3d_fwd_halo   narrow outputs, rows >= 128: one halo block per chunk
 //   k_conv3d_fwd_tma    everything else: per-tap TMA boxes
 //   k_conv3d_fwd_tc     where the driver refuses a tensor map: cp.async gathers
@@ -172,6 +173,29 @@ __device__ __forceinline__ uint64_t umma_sdesc(uint32_t saddr, uint32_t lbo, uin
 __host__ __device__ constexpr uint32_t umma_idesc(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
+
+// One MMA (kind::f16, BF16 operands) and one commit of the warp's MMAs, issued
+// by the warp's elected lane. The whole warp runs the issuing loops, so that
+// descriptors, addresses and loop counters are warp-uniform and stay in uniform
+// registers, which the instruction takes its operands from (a one-thread branch
+// moves them there for every MMA: 3 to 11% of the whole layer at 128^3). One
+// CTA issues an M = 128, K = 16 MMA every 40 (N = 16, 32) to 64 cycles (N =
+// 128) this way. elect.sync elects the same lane each time, as the commit
+// requires.
+__device__ __forceinline__ void umma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p, e;\n .reg .b32 r;\n elect.sync r|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    asm volatile(
+        "{\n .reg .pred e;\n .reg .b32 r;\n elect.sync r|e, 0xffffffff;\n"
+        " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
+        : "memory");
+}
+// the warp's index as a warp-uniform value
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0));
@@ -371,7 +395,7 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_tma(const __grid_constant__ 
     const uint32_t raw = smem_u32(tma_smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;   // swizzled stages start on 1024-byte boundaries
     unsigned char* gen = tma_smem_raw + (base - raw);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
     const int S = C.stages;
     uint64_t* full = reinterpret_cast<uint64_t*>(gen + S * C.stage_bytes);
     uint64_t* empty = full + S;
@@ -426,34 +450,26 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_tma(const __grid_constant__ 
             tma_3d(st + C.a_bytes, &wmap, c0, tap, n0, smem_u32(full + s));
             *issued = it + 1;
         }
-    } else if (t == 32) {   // MMA issuer
+    } else if (warp == 1) {   // MMA issuer (the whole warp: see umma_f16)
         const uint32_t idesc = umma_idesc(TC_M, N);
         const uint32_t row = (uint32_t)C.swz_bytes;
         int it = 0;
         for (; it < iters; ++it) {
             const int s = it % S;
-            if (!mbar_wait(smem_u32(full + s), (uint32_t)((it / S) & 1))) {
-                atomicExch(failed, 1);
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(full + s), (uint32_t)((it / S) & 1)))) {
+                if (lane == 0) atomicExch(failed, 1);
                 break;
             }
-            *consumed = it + 1;
+            if (lane == 0) *consumed = it + 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = base + s * C.stage_bytes;
-            for (int k = 0; k < C.kc / 16; ++k) {
-                const uint64_t ad = umma_sdesc_sw(st + k * 32, row);
-                const uint64_t bd = umma_sdesc_sw(st + C.a_bytes + k * 32, row);
-                const uint32_t acc = (it > 0 || k > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(empty + s)));
+            const uint64_t ad = umma_sdesc_sw(st, row), bd = umma_sdesc_sw(st + C.a_bytes, row);
+            for (int k = 0; k < C.kc / 16; ++k)   // 16 channels: 32 bytes, 2 in the descriptor's address
+                umma_f16(tmem, ad + 2 * k, bd + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
+            umma_commit(smem_u32(empty + s));
         }
         // arrives once every MMA issued so far has completed (also after a timeout)
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_u32(acc_full)));
+        umma_commit(smem_u32(acc_full));
     }
     __syncwarp();
     bool ok = mbar_wait(smem_u32(acc_full), 0);
@@ -588,7 +604,7 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_halo(const __grid_constant__
     const uint32_t raw = smem_u32(hb_smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* gen = hb_smem_raw + (base - raw);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
     const int S = H.stages;
     uint64_t* full = reinterpret_cast<uint64_t*>(gen + S * H.stage_bytes);
     uint64_t* empty = full + S;
@@ -642,8 +658,8 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_halo(const __grid_constant__
         asm volatile("cp.async.wait_group 0;");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (t == 0) {
-            ok = mbar_wait(smem_u32(full + s), (uint32_t)((c / S) & 1));
+        if (warp == 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(full + s), (uint32_t)((c / S) & 1)));
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int tap = 0; tap < 27; ++tap) {
@@ -651,20 +667,15 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_halo(const __grid_constant__
                     const uint64_t ad = umma_sdesc(st + row * 16, H.a_plane, 128);
                     const uint64_t bd = umma_sdesc(st + H.a_bytes + (uint32_t)(tap * 2 * N) * 16, (uint32_t)N * 16, 128);
                     const uint32_t accum = (c > 0 || tap > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                        "l"(ad), "l"(bd), "r"(idesc), "r"(accum));
+                    umma_f16(tmem, ad, bd, idesc, accum);
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                    smem_u32(empty + s)));
+                umma_commit(smem_u32(empty + s));
             }
         }
         if (__syncthreads_or(!ok)) break;
         committed = c + 1;
     }
-    if (t == 0) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(acc_full)));
+    if (warp == 0) umma_commit(smem_u32(acc_full));
     if (committed > 0 || !ok) {
         const bool done = mbar_wait(smem_u32(acc_full), 0);
         ok = ok && done;
@@ -769,7 +780,7 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_march(const __grid_constant_
     const uint32_t raw = smem_u32(mc_smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* gen = mc_smem_raw + (base - raw);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
     uint64_t* full = reinterpret_cast<uint64_t*>(gen + M.w_off + M.w_bytes);   // 4 slots
     uint64_t* accf = full + 4;                                                 // 2 accumulators
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accf + 2);
@@ -874,11 +885,11 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_march(const __grid_constant_
     bool ok = true;
     int issued = 0;   // output lines whose MMAs were issued
     for (int yo = y0; yo < y1 && ok; ++yo) {
-        if (t == 0) {
+        if (warp == 0) {
             // lines yo-1 and yo landed in earlier iterations (or the prologue); wait for yo + 1
             for (int L = (yo == y0 ? yo - 1 : yo + 1); L <= yo + 1 && ok; ++L) {
                 const int k = L - (y0 - 1);
-                ok = mbar_wait(smem_u32(full + (k & 3)), (uint32_t)((k >> 2) & 1));
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(full + (k & 3)), (uint32_t)((k >> 2) & 1)));
             }
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -896,13 +907,9 @@ __global__ void __launch_bounds__(128) k_conv3d_fwd_march(const __grid_constant_
                             umma_sdesc(base + M.w_off + (uint32_t)((c * 27 + tap) * 2 * N) * 16, (uint32_t)N * 16, 128);
                         const uint32_t accum = first ? 0u : 1u;
                         first = 0;
-                        asm volatile(
-                            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dacc),
-                            "l"(ad), "l"(bd), "r"(idesc), "r"(accum));
+                        umma_f16(dacc, ad, bd, idesc, accum);
                     }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                    smem_u32(accf + (j & 1))));
+                umma_commit(smem_u32(accf + (j & 1)));
             }
         }
         if (__syncthreads_or(!ok)) {
@@ -960,6 +967,321 @@ bool march_plan(const Vol& V, int cin, int cout, MarchConv& M) {
     return M.smem <= 227u * 1024u;
 }
 
+// ---------------------------------------------------------------- forward with the x taps as row shifts
+// For narrow outputs (Cout <= 64), where the per-tap form is bound by the 27
+// operand boxes that each 128-voxel tile reads through L2. A CTA owns T output
+// lines y0 .. y0+T-1 of plane (b, z), 128 voxels of x each, and steps through
+// the input lines instead of the taps: input line (z+dz, y) is staged once, as
+// W = 130 voxel rows from x0 - 1 (zero fill: the padding), and serves up to
+// three output lines and all three x taps, whose A operand is the same line
+// starting at voxel row dx + 1. A plane's T + 2 lines and its weights (one
+// block of three taps per dy) pass through two rings of slots; per output line
+// that is 3 (T + 2) / T line loads instead of 27.
+// The rows of a swizzled line start anywhere in the swizzle pattern: the
+// pattern is a function of the shared-memory address (slots are aligned to its
+// repeat), so a descriptor's start address moves by whole rows.
+// Every output element takes its products in the order of the form that its
+// shape used before, so results are the same bits: tap by tap with the
+// channels inside (order 0, the per-tap form), or 16 channels at a time with
+// the 27 taps inside (order 1, the halo block).
+// Step (p, dy) of plane p (a dz, or a channel chunk and a dz) issues T x 3 x
+// Cin/16 MMAs and commits them to the done barrier of its weight slot; a line
+// is free once the last step that reads it is done. The CTAs are persistent:
+// warp 4 loads, warp 5 issues, warps 0-3 store an item from one of two sets of
+// accumulators while the next item's MMAs fill the other, so loads, MMAs and
+// stores of successive items overlap (as one item per CTA they took turns:
+// 32->32 at 128^3 257 us). Waits are bounded as in k_conv3d_fwd_tma; a role
+// that gives up sets `failed`, and the others run out of their own waits.
+struct ShiftConv {
+    int order, kc, chunks, row_bytes, T, nr, nb, tiles_x, groups_y, cols, box_w, items, ctas;
+    uint32_t line_chunk, line_slot, line_tx, b_tap, b_slot, b_tx;
+    uint32_t b_off, bar_off;
+    size_t smem;
+};
+constexpr int SH_ROWS = 130, SH_THREADS = 192;
+
+template <int KS, int T>   // K steps of 16 channels per box (1, 2 or 4), output lines per item (1, 2 or 4)
+__global__ void __launch_bounds__(SH_THREADS) k_conv3d_fwd_shift(const __grid_constant__ CUtensorMap xmap,
+                                                                  const __grid_constant__ CUtensorMap wmap,
+                                                                  void* __restrict__ y, const float* __restrict__ bias,
+                                                                  int act, const Vol V, int cout, const ShiftConv C) {
+    extern __shared__ unsigned char sh_smem_raw[];
+    const uint32_t raw = smem_u32(sh_smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    unsigned char* gen = sh_smem_raw + (base - raw);
+    const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
+    uint64_t* lfull = reinterpret_cast<uint64_t*>(gen + C.bar_off);   // nr: line landed
+    uint64_t* bfull = lfull + C.nr;                                   // nb: weights landed
+    uint64_t* done = bfull + C.nb;                                    // nb: the step's MMAs completed
+    uint64_t* acc_full = done + C.nb;                                 // 2: an item's sums are complete
+    uint64_t* acc_empty = acc_full + 2;                               // 2: they were stored
+    uint64_t* last_mma = acc_empty + 2;                               // every MMA issued has completed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last_mma + 1);
+    int* failed = reinterpret_cast<int*>(tmem_slot + 1);
+    int* lines_in = failed + 1;    // lines whose loads were issued
+    int* steps_in = failed + 2;    // steps whose weights' loads were issued
+    int* last_step = failed + 3;   // nr: the last step that reads the slot's line
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(C.cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (t == 32) {
+        for (int q = 0; q < C.nr + 2 * C.nb + 5; ++q) {
+            const uint32_t bar = smem_u32(lfull + q);
+            const uint32_t count = q >= C.nr + 2 * C.nb + 2 && q < C.nr + 2 * C.nb + 4 ? 4u : 1u;   // acc_empty: 4 warps
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;");
+        *failed = *lines_in = *steps_in = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    const int N = cout;
+    const int boxes = C.order ? 1 : C.chunks;   // channel boxes per line
+    struct Item {
+        int x0, y0, z, b, dz0, ndz, planes;
+    };
+    // item i; planes in accumulation order: planes outside the grid hold
+    // zeros, which leave a sum as it is, and are skipped (dz = 0 is inside)
+    auto item = [&](int i) {
+        Item m;
+        m.x0 = i % C.tiles_x * TC_M;
+        i /= C.tiles_x;
+        m.y0 = i % C.groups_y * T;
+        i /= C.groups_y;
+        m.z = i % V.d;
+        m.b = i / V.d;
+        m.dz0 = m.z > 0 ? -1 : 0;
+        m.ndz = (m.z < V.d - 1 ? 1 : 0) - m.dz0 + 1;
+        m.planes = C.order ? C.chunks * m.ndz : m.ndz;
+        return m;
+    };
+
+    if (warp == 4) {
+        if (lane == 0) {   // producer
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
+            int finished = 0;   // steps known to have completed (they complete in order)
+            int line = 0, step = 0;   // issued so far
+            bool ok = true;
+            auto wait_steps = [&](int upto) {
+                while (ok && finished < upto) {
+                    ok = mbar_wait(smem_u32(done + finished % C.nb), (uint32_t)((finished / C.nb) & 1));
+                    if (ok) ++finished;
+                }
+            };
+            for (int i = blockIdx.x; i < C.items && ok; i += gridDim.x) {
+                const Item m = item(i);
+                for (int p = 0; p < m.planes && ok; ++p) {
+                    const int dz = m.dz0 + p % m.ndz, c0 = C.order ? p / m.ndz * C.kc : 0;
+                    for (int r = 0, dy = 0; dy < 3 && ok; ++dy, ++step) {
+                        // the lines step (p, dy) adds: 0 .. T-1, then one per step
+                        for (; r < T + dy && ok; ++r) {
+                            const int sl = line % C.nr;
+                            if (line >= C.nr) wait_steps(last_step[sl] + 1);
+                            if (!ok) break;
+                            last_step[sl] = step - dy + min(r, 2);
+                            const uint32_t st = base + (uint32_t)sl * C.line_slot, bar = smem_u32(lfull + sl);
+                            mbar_expect(bar, C.line_tx);   // the boxes' full bytes arrive, zero-filled parts included
+                            for (int c = 0; c < boxes; ++c)
+                                tma_5d(st + c * C.line_chunk, &xmap, c0 + c * C.kc, m.x0 - 1, m.y0 - 1 + r, m.z + dz, m.b, bar);
+                            *lines_in = ++line;
+                        }
+                        wait_steps(step - C.nb + 1);
+                        if (!ok) break;
+                        const uint32_t st = base + C.b_off + (uint32_t)(step % C.nb) * C.b_slot, bar = smem_u32(bfull + step % C.nb);
+                        mbar_expect(bar, C.b_tx);
+                        for (int c = 0; c < boxes; ++c)
+                            for (int dx = 0; dx < 3; ++dx)
+                                tma_3d(st + (uint32_t)(c * 3 + dx) * C.b_tap, &wmap, c0 + c * C.kc, (dz + 1) * 9 + dy * 3 + dx, 0, bar);
+                        *steps_in = step + 1;
+                    }
+                }
+            }
+            if (!ok) atomicExch(failed, 1);
+        }
+        __syncwarp();
+    } else if (warp == 5) {   // MMA issuer (the whole warp: see umma_f16)
+        const uint32_t idesc = umma_idesc(TC_M, N);
+        constexpr uint32_t row = KS * 32;   // bytes of a voxel row in a box
+        const uint32_t line16 = C.line_chunk >> 4, b_tap16 = C.b_tap >> 4, line_slot16 = C.line_slot >> 4, b_slot16 = C.b_slot >> 4;
+        const uint64_t adesc = umma_sdesc_sw(base, row), bdesc = umma_sdesc_sw(base + C.b_off, row);
+        bool ok = true;
+        int step = 0, l0 = 0, seen = 0, n = 0;   // steps, the plane's first line, lines seen, items
+        for (int i = blockIdx.x; i < C.items && ok; i += gridDim.x, ++n) {
+            const Item m = item(i);
+            const uint32_t d0 = tmem + (uint32_t)((n & 1) * T * N);
+            // the accumulators' last item must have been stored
+            if (n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_empty + (n & 1)), (uint32_t)((n / 2 - 1) & 1)));
+            uint32_t fresh = 1;
+            for (int p = 0; p < m.planes && ok; ++p, l0 += T + 2)
+                for (int dy = 0; dy < 3 && ok; ++dy, ++step) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bfull + step % C.nb), (uint32_t)((step / C.nb) & 1)));
+                    for (; seen < l0 + T + dy && ok; ++seen)
+                        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(lfull + seen % C.nr), (uint32_t)((seen / C.nr) & 1)));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    // a descriptor's address field counts 16 bytes in its low
+                    // word, so operands are reached by additions
+                    const uint64_t b0 = bdesc + (uint32_t)(step % C.nb) * b_slot16;
+                    uint64_t a0[T];
+#pragma unroll
+                    for (int q = 0; q < T; ++q) a0[q] = adesc + (uint32_t)((l0 + q + dy) % C.nr) * line_slot16;
+#pragma unroll
+                    for (int dx = 0; dx < 3; ++dx)
+                        for (int c = 0; c < boxes; ++c) {
+                            const uint64_t bd = b0 + (uint32_t)(c * 3 + dx) * b_tap16;
+                            const uint32_t ao = (uint32_t)c * line16 + ((uint32_t)(dx * row) >> 4);
+#pragma unroll
+                            for (int k = 0; k < KS; ++k) {
+#pragma unroll
+                                for (int q = 0; q < T; ++q)
+                                    umma_f16(d0 + (uint32_t)(q * N), a0[q] + ao + 2 * k, bd + 2 * k, idesc, fresh ^ 1u);
+                                fresh = 0;
+                            }
+                        }
+                    umma_commit(smem_u32(done + step % C.nb));
+                }
+            if (ok) umma_commit(smem_u32(acc_full + (n & 1)));
+        }
+        if (!ok && lane == 0) atomicExch(failed, 1);
+        umma_commit(smem_u32(last_mma));   // arrives once every MMA issued so far has completed (also after a timeout)
+    } else {   // epilogue
+        bool ok = true;
+        int n = 0;
+        for (int i = blockIdx.x; i < C.items && ok; i += gridDim.x, ++n) {
+            const Item m = item(i);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_full + (n & 1)), (uint32_t)((n >> 1) & 1)));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int xx = m.x0 + warp * 32 + lane;
+            for (int q = 0; q < T; ++q) {
+                const int yy = m.y0 + q;
+                const bool store = xx < V.w && yy < V.h;
+                const long long o0 = ((((long long)m.b * V.d + m.z) * V.h + yy) * V.w + xx) * cout;
+                for (int c = 0; c < N; c += 16) {
+                    uint32_t r[16];
+                    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(((n & 1) * T + q) * N + c);
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                        : "r"(taddr));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4) {
+                        const float4 bj = bias ? *reinterpret_cast<const float4*>(bias + c + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        v[j] = __uint_as_float(r[j]) + bj.x;
+                        v[j + 1] = __uint_as_float(r[j + 1]) + bj.y;
+                        v[j + 2] = __uint_as_float(r[j + 2]) + bj.z;
+                        v[j + 3] = __uint_as_float(r[j + 3]) + bj.w;
+                    }
+                    if (act & ACT_RELU) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.f);
+                    }
+                    if (!store) continue;
+                    if (act & ACT_BF16) {
+                        uint32_t h[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            h[j] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v[2 * j])) |
+                                   ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v[2 * j + 1])) << 16);
+                        uint4* out = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(y) + o0 + c);
+                        out[0] = make_uint4(h[0], h[1], h[2], h[3]);
+                        out[1] = make_uint4(h[4], h[5], h[6], h[7]);
+                    } else {
+                        float* out = static_cast<float*>(y) + o0 + c;
+#pragma unroll
+                        for (int j = 0; j < 16; j += 4)
+                            *reinterpret_cast<float4*>(out + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    }
+                }
+            }
+            // the accumulators are read: the item after next may overwrite them
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + (n & 1))) : "memory");
+        }
+        if (!ok && lane == 0) atomicExch(failed, 1);
+    }
+    __syncthreads();
+    const bool drained = mbar_wait(smem_u32(last_mma), 0);
+    if (t == 0 && (*failed != 0 || !drained)) {
+        atomicExch(&g_conv_error, 1);
+        // loads still in flight land in this CTA's shared memory: wait (bounded) for the last ones issued
+        for (int q = max(0, *lines_in - C.nr); q < *lines_in; ++q)
+            mbar_wait(smem_u32(lfull + q % C.nr), (uint32_t)((q / C.nr) & 1));
+        for (int q = max(0, *steps_in - C.nb); q < *steps_in; ++q)
+            mbar_wait(smem_u32(bfull + q % C.nb), (uint32_t)((q / C.nb) & 1));
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C.cols));
+}
+
+// The halo block's shapes (its accumulation order is order 1 above).
+bool halo_shape(const Vol& V, int cin, int cout) { return cout <= 32 && cin * cout <= 768 && V.w >= TC_M; }
+
+// The row-shift plan, or false outside its shapes (Cout <= 64).
+bool shift_plan(const Vol& V, int cin, int cout, ShiftConv& C) {
+    if (cout > 64 || cin % 16 != 0 || cout % 16 != 0) return false;
+    C = ShiftConv{};
+    C.order = halo_shape(V, cin, cout) ? 1 : 0;
+    C.kc = C.order ? 16 : cin % 64 == 0 ? 64 : cin % 32 == 0 ? 32 : 16;
+    C.chunks = cin / C.kc;
+    C.row_bytes = C.kc * 2;
+    const int boxes = C.order ? 1 : C.chunks;
+    C.box_w = V.w + 2 < SH_ROWS ? V.w + 2 : SH_ROWS;
+    // slots start on the swizzle's repeat (8 rows, at most 1024 bytes)
+    C.line_chunk = ((uint32_t)SH_ROWS * C.row_bytes + 1023u) & ~1023u;
+    C.line_slot = C.line_chunk * boxes;
+    C.line_tx = (uint32_t)C.box_w * C.row_bytes * boxes;
+    C.b_tap = ((uint32_t)cout * C.row_bytes + 1023u) & ~1023u;
+    C.b_slot = C.b_tap * 3 * boxes;
+    C.b_tx = (uint32_t)cout * C.row_bytes * 3 * boxes;
+    C.tiles_x = (V.w + TC_M - 1) / TC_M;
+    // lines per item: 4, or fewer where the rings do not fit or there would be
+    // less than two items per SM; two CTAs per SM where they fit
+    for (int T : {4, 2, 1}) {
+        if (T > 1 && ((long long)C.tiles_x * ((V.h + T - 1) / T) * V.d * V.n < 148 * 2 || T > V.h)) continue;
+        if (2 * T * cout > 512) continue;
+        for (size_t limit : {(size_t)112 * 1024, (size_t)226 * 1024}) {
+            const size_t fixed = 1024 + 1024;   // alignment, barriers and counters
+            if (limit < (size_t)200 * 1024 && 2 * T * cout > 256) continue;   // two CTAs share 512 TMEM columns
+            C.nb = 3;
+            if (fixed + (size_t)3 * C.b_slot + (size_t)(T + 3) * C.line_slot > limit) continue;
+            C.T = T;
+            C.nr = T + 3;
+            // the rest of the limit: lines and weights ahead, evenly
+            while (C.nr < 2 * (T + 2) && fixed + (size_t)C.nb * C.b_slot + (size_t)(C.nr + 1) * C.line_slot <= limit) {
+                ++C.nr;
+                if (C.nb < 6 && fixed + (size_t)(C.nb + 1) * C.b_slot + (size_t)C.nr * C.line_slot <= limit) ++C.nb;
+            }
+            C.b_off = C.nr * C.line_slot;
+            C.bar_off = C.b_off + C.nb * C.b_slot;
+            C.smem = (size_t)C.bar_off + (C.nr + 2 * C.nb + 5) * 8 + 16 + C.nr * 4 + 1024;
+            C.groups_y = (V.h + T - 1) / T;
+            const long long items = (long long)C.tiles_x * C.groups_y * V.d * V.n;
+            if (items > 0x7fffffffLL) return false;
+            C.items = (int)items;
+            const int per_sm = limit < (size_t)200 * 1024 ? 2 : 1;
+            C.ctas = (int)(items < 148LL * per_sm ? items : 148LL * per_sm);
+            C.cols = 32;
+            while (C.cols < 2 * T * cout) C.cols <<= 1;
+            if (C.smem < (size_t)C.cols * 400) C.smem = (size_t)C.cols * 400;
+            return true;
+        }
+    }
+    return false;
+}
+
 // ---------------------------------------------------------------- weight gradient, tcgen05 + TMA
 // dw[co][tap][ci] = sum_u dy[u - off(tap)][co] * x[u][ci] (u runs over the
 // voxels of x; dy is zero outside the grid): one GEMM with M = (tap, co)
@@ -999,7 +1321,7 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tma(const __grid_constant_
     const uint32_t raw = smem_u32(wg_smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* gen = wg_smem_raw + (base - raw);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x, warp = uniform_warp(), lane = t & 31;
     const int S = G.stages;
     uint64_t* full = reinterpret_cast<uint64_t*>(gen + S * G.stage_bytes);
     uint64_t* empty = full + S;
@@ -1064,32 +1386,27 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tma(const __grid_constant_
                 tma_5d(st + G.a_bytes + (uint32_t)j * G.b_box, &xmap, n0 + j * G.wsb, x0, y0, z, b, bar);
             *issued = it + 1;
         }
-    } else if (t == 32) {   // MMA issuer
+    } else if (warp == 1) {   // MMA issuer (the whole warp: see umma_f16)
         const uint32_t idesc = umma_idesc(TC_M, N) | (1u << 15) | (1u << 16);   // A and B MN-major
         const uint32_t ra = (uint32_t)G.wsa * 2, rb = (uint32_t)G.wsb * 2;
         for (int it = 0; it < iters; ++it) {
             const int s = it % S;
-            if (!mbar_wait(smem_u32(full + s), (uint32_t)((it / S) & 1))) {
-                atomicExch(failed, 1);
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(full + s), (uint32_t)((it / S) & 1)))) {
+                if (lane == 0) atomicExch(failed, 1);
                 break;
             }
-            *consumed = it + 1;
+            if (lane == 0) *consumed = it + 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = base + s * G.stage_bytes;
             for (int k = 0; k < G.kt / 16; ++k) {   // two 8-row groups per MMA
                 const uint64_t ad = umma_sdesc_mn(st + k * 16 * ra, ra, G.a_box);
                 const uint64_t bd = umma_sdesc_mn(st + G.a_bytes + k * 16 * rb, rb, G.b_box);
                 const uint32_t acc = (it > 0 || k > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+                umma_f16(tmem, ad, bd, idesc, acc);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(empty + s)));
+            umma_commit(smem_u32(empty + s));
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_u32(acc_full)));
+        umma_commit(smem_u32(acc_full));
     }
     __syncwarp();
     bool ok = iters > 0 ? mbar_wait(smem_u32(acc_full), 0) : true;
@@ -1213,27 +1530,288 @@ int check_args(long long voxels, int cin, int cout) {
     return NICR_OK;
 }
 
+// ---------------------------------------------------------------- elementwise passes around the convolutions
+__device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        v[2 * j] = __uint_as_float(w[j] << 16);
+        v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+    }
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        w[j] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v[2 * j])) |
+               ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v[2 * j + 1])) << 16);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// 8 consecutive channels as FP32 from a BF16 or FP32 array
+template <bool BF16>
+__device__ __forceinline__ void load8(const void* p, long long i, float (&v)[8]) {
+    if (BF16) {
+        unpack8(*reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p) + i), v);
+    } else {
+        const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i);
+        const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+}
+
+// Backward of act(. + bias): g = gy * (y > 0) (y null: g = gy) as BF16, and
+// per-CTA column sums of g in FP32 (the bias gradient, k_bias_grad adds them).
+// One pass over gy and y instead of a conversion, a comparison, a product, a
+// reduction and a conversion (290 us at 16 channels of 128^3; 39 us here):
+// HBM bound, 8 channels per thread, a thread's rows strided by the grid.
+constexpr int kActBwdBlocks = 148 * 4;
+template <bool GB, int YT>   // GB: gy is BF16; YT: 0 no y, 1 BF16, 2 FP32
+__global__ void __launch_bounds__(256) k_act_bwd(const void* __restrict__ gy, const void* __restrict__ y,
+                                                  __nv_bfloat16* __restrict__ g, float* __restrict__ partial,
+                                                  long long rows, int c) {
+    __shared__ float sums[256 * 8];
+    const int vecs = c / 8, rpb = blockDim.x / vecs;   // rows per pass of the CTA
+    const int v = threadIdx.x % vecs, r0 = threadIdx.x / vecs;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (long long r = (long long)blockIdx.x * rpb + r0; r < rows; r += (long long)gridDim.x * rpb) {
+        const long long i = r * c + v * 8;
+        float a[8];
+        load8<GB>(gy, i, a);
+        if (YT) {
+            float m[8];
+            load8<YT == 1>(y, i, m);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[j] *= m[j] > 0.f ? 1.f : 0.f;   // a product, so NaN and Inf pass as they did
+        }
+        *reinterpret_cast<uint4*>(g + i) = pack8(a);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += a[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sums[threadIdx.x * 8 + j] = acc[j];
+    __syncthreads();
+    for (int q = threadIdx.x; q < c; q += blockDim.x) {
+        double s = 0.;
+        for (int k = 0; k < rpb; ++k) s += (double)sums[(k * vecs) * 8 + q];
+        partial[(long long)blockIdx.x * c + q] = (float)s;
+    }
+}
+// gb[q] = the sum of the partials of column q: warp per column, FP64
+__global__ void k_bias_grad(const float* __restrict__ partial, float* __restrict__ gb, int blocks, int c) {
+    const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (q >= c) return;
+    double s = 0.;
+    for (int k = lane; k < blocks; k += 32) s += (double)partial[(long long)k * c + q];
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+    if (lane == 0) gb[q] = (float)s;
+}
+
+// 2x2x2 average of BF16 NDHWC, summed in FP32 (8 channels per thread), in the
+// order of the torch reduction it stands for (four running sums of two, added
+// in turn): a sum rounded elsewhere flips a BF16 value now and then, which the
+// layers below spread
+__global__ void __launch_bounds__(256) k_avgpool2(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
+                                                   Vol V, int c, long long total) {
+    const int vecs = c / 8;
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+        const int v = (int)(i % vecs);
+        long long r = i / vecs;
+        const int xo = (int)(r % V.w); r /= V.w;
+        const int yo = (int)(r % V.h); r /= V.h;
+        const int zo = (int)(r % V.d);
+        const long long b = r / V.d;
+        float e[8][8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {   // k = 4 z + 2 y + x
+            const long long src = (((b * 2 * V.d + 2 * zo + (k >> 2)) * 2 * V.h + 2 * yo + ((k >> 1) & 1)) * 2 * V.w + 2 * xo + (k & 1));
+            load8<true>(x, src * c + v * 8, e[k]);
+        }
+        float s[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            s[j] = ((((e[0][j] + e[4][j]) + (e[1][j] + e[5][j])) + (e[2][j] + e[6][j])) + (e[3][j] + e[7][j])) * 0.125f;
+        *reinterpret_cast<uint4*>(y + i * 8) = pack8(s);
+    }
+}
+
+// out = [nearest 2x of a, b] along the channels, BF16 NDHWC; V is the fine grid
+__global__ void __launch_bounds__(256) k_upcat(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
+                                                __nv_bfloat16* __restrict__ y, Vol V, int ca, int cb, long long total) {
+    const int va = ca / 8, vecs = (ca + cb) / 8;
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+        const int v = (int)(i % vecs);
+        const long long vox = i / vecs;
+        const __nv_bfloat16* src;
+        if (v < va) {
+            long long r = vox;
+            const int x = (int)(r % V.w); r /= V.w;
+            const int yy = (int)(r % V.h); r /= V.h;
+            const int z = (int)(r % V.d);
+            const long long n = r / V.d;
+            src = a + (((n * (V.d / 2) + z / 2) * (V.h / 2) + yy / 2) * (V.w / 2) + x / 2) * ca + v * 8;
+        } else {
+            src = b + vox * cb + (v - va) * 8;
+        }
+        *reinterpret_cast<uint4*>(y + i * 8) = *reinterpret_cast<const uint4*>(src);
+    }
+}
+
+// FP32 rows of f <= 16 values as 16 BF16 channels, the rest zero
+__global__ void __launch_bounds__(256) k_pad16(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long rows,
+                                                int f) {
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < rows * 2; i += (long long)gridDim.x * 256) {
+        const long long r = i >> 1;
+        const int c0 = (int)(i & 1) * 8;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = c0 + j < f ? x[r * f + c0 + j] : 0.f;
+        *reinterpret_cast<uint4*>(y + i * 8) = pack8(v);
+    }
+}
+int elementwise_blocks(long long items) {
+    const long long want = (items + 255) / 256;
+    return (int)(want < 148 * 16 ? (want > 0 ? want : 1) : 148 * 16);
+}
+bool aligned16(const void* p) { return (reinterpret_cast<unsigned long long>(p) & 15ull) == 0; }
+
 }  // namespace
 
 extern "C" {
+
+int nicr_conv3d_act_bwd_blocks(void) { return kActBwdBlocks; }
+
+int nicr_conv3d_act_bwd(const void* gy, int gy_bf16, const void* y, int y_bf16, void* g, float* partial, float* gb,
+                        long long rows, int c, void* stream) {
+    if (!gy || !g || !partial || !gb || rows <= 0 || c <= 0 || c % 8 != 0 || c > 2048 || !aligned16(gy) || !aligned16(g) ||
+        (y && !aligned16(y)))
+        return NICR_ERR_INVALID_ARG;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int threads = 256 / (c / 8) * (c / 8);
+    auto* out = static_cast<__nv_bfloat16*>(g);
+#define NICR_ACT_BWD(GB, YT) k_act_bwd<GB, YT><<<kActBwdBlocks, threads, 0, s>>>(gy, y, out, partial, rows, c)
+    if (gy_bf16) {
+        if (!y) NICR_ACT_BWD(true, 0);
+        else if (y_bf16) NICR_ACT_BWD(true, 1);
+        else NICR_ACT_BWD(true, 2);
+    } else {
+        if (!y) NICR_ACT_BWD(false, 0);
+        else if (y_bf16) NICR_ACT_BWD(false, 1);
+        else NICR_ACT_BWD(false, 2);
+    }
+#undef NICR_ACT_BWD
+    k_bias_grad<<<(c + 7) / 8, 256, 0, s>>>(partial, gb, kActBwdBlocks, c);
+    return cudaGetLastError() == cudaSuccess ? NICR_OK : NICR_ERR_CUDA;
+}
+
+int nicr_avgpool2_ndhwc(const void* x, void* y, int n, int d, int h, int w, int c, void* stream) {
+    if (!x || !y || n <= 0 || d <= 0 || h <= 0 || w <= 0 || (d | h | w) % 2 != 0 || c <= 0 || c % 8 != 0 || !aligned16(x) ||
+        !aligned16(y))
+        return NICR_ERR_INVALID_ARG;
+    const Vol V{n, d / 2, h / 2, w / 2};
+    const long long total = V.voxels() * (c / 8);
+    k_avgpool2<<<elementwise_blocks(total), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), V, c, total);
+    return cudaGetLastError() == cudaSuccess ? NICR_OK : NICR_ERR_CUDA;
+}
+
+int nicr_upcat_ndhwc(const void* a, const void* b, void* y, int n, int d, int h, int w, int ca, int cb, void* stream) {
+    if (!a || !b || !y || n <= 0 || d <= 0 || h <= 0 || w <= 0 || (d | h | w) % 2 != 0 || ca <= 0 || cb <= 0 ||
+        (ca | cb) % 8 != 0 || !aligned16(a) || !aligned16(b) || !aligned16(y))
+        return NICR_ERR_INVALID_ARG;
+    const Vol V{n, d, h, w};
+    const long long total = V.voxels() * ((ca + cb) / 8);
+    k_upcat<<<elementwise_blocks(total), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b), static_cast<__nv_bfloat16*>(y), V, ca,
+        cb, total);
+    return cudaGetLastError() == cudaSuccess ? NICR_OK : NICR_ERR_CUDA;
+}
+
+int nicr_pad16(const float* x, void* y, long long rows, int f, void* stream) {
+    if (!x || !y || rows <= 0 || f <= 0 || f > 16 || !aligned16(y)) return NICR_ERR_INVALID_ARG;
+    k_pad16<<<elementwise_blocks(rows * 2), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        x, static_cast<__nv_bfloat16*>(y), rows, f);
+    return cudaGetLastError() == cudaSuccess ? NICR_OK : NICR_ERR_CUDA;
+}
 
 int nicr_conv3d_fwd_tma(const void* x, const void* w, float* y, int n, int d, int h, int w_, int cin, int cout,
                         void* stream) {
     return launch_fwd_tma(x, w, nullptr, 0, y, n, d, h, w_, cin, cout, stream);
 }
 
+int nicr_conv3d_fwd_shift(const void* x, const void* w, const float* bias, int act, void* y, int n, int d, int h,
+                          int w_, int cin, int cout, void* stream) {
+    const Vol V{n, d, h, w_};
+    const int rc = check_args(V.voxels(), cin, cout);
+    ShiftConv C;
+    if (rc != NICR_OK || !x || !w || !y || (act & ~(ACT_RELU | ACT_BF16)) != 0 || !shift_plan(V, cin, cout, C))
+        return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
+    const auto enc = conv_map_encoder();
+    if (!enc) return NICR_ERR_CUDA;
+    const CUtensorMapSwizzle swz = C.kc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                   : C.kc == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    CUtensorMap xmap, wmap;
+    {   // x: (c, w, h, d, n), boxes {KC, W + 2, 1, 1, 1}
+        const cuuint64_t dims[5] = {(cuuint64_t)cin, (cuuint64_t)w_, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
+        const cuuint64_t str[4] = {(cuuint64_t)cin * 2, (cuuint64_t)w_ * cin * 2, (cuuint64_t)h * w_ * cin * 2,
+                                   (cuuint64_t)d * h * w_ * cin * 2};
+        const cuuint32_t box[5] = {(cuuint32_t)C.kc, (cuuint32_t)C.box_w, 1, 1, 1};
+        if (enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(x), dims, str, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return NICR_ERR_INVALID_ARG;
+    }
+    {   // w: (ci, tap, co), boxes {KC, 1, Cout}
+        const cuuint64_t dims[3] = {(cuuint64_t)cin, 27, (cuuint64_t)cout};
+        const cuuint64_t str[2] = {(cuuint64_t)cin * 2, (cuuint64_t)27 * cin * 2};
+        const cuuint32_t box[3] = {(cuuint32_t)C.kc, 1, (cuuint32_t)cout};
+        if (enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, str, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return NICR_ERR_INVALID_ARG;
+    }
+    auto launch = [&](auto kernel) -> int {
+        if (ensure_smem((const void*)kernel, C.smem) != NICR_OK) return NICR_ERR_CUDA;
+        kernel<<<C.ctas, SH_THREADS, C.smem, static_cast<cudaStream_t>(stream)>>>(xmap, wmap, y, bias, act, V, cout, C);
+        return cudaGetLastError() == cudaSuccess ? NICR_OK : NICR_ERR_CUDA;
+    };
+    switch (C.kc / 16 * 8 + C.T) {
+        case 8 + 1: return launch(k_conv3d_fwd_shift<1, 1>);
+        case 8 + 2: return launch(k_conv3d_fwd_shift<1, 2>);
+        case 8 + 4: return launch(k_conv3d_fwd_shift<1, 4>);
+        case 16 + 1: return launch(k_conv3d_fwd_shift<2, 1>);
+        case 16 + 2: return launch(k_conv3d_fwd_shift<2, 2>);
+        case 16 + 4: return launch(k_conv3d_fwd_shift<2, 4>);
+        case 32 + 1: return launch(k_conv3d_fwd_shift<4, 1>);
+        case 32 + 2: return launch(k_conv3d_fwd_shift<4, 2>);
+        case 32 + 4: return launch(k_conv3d_fwd_shift<4, 4>);
+        default: return NICR_ERR_INVALID_ARG;
+    }
+}
+
 int nicr_conv3d_fwd_act(const void* x, const void* w, const float* bias, int act, void* y, int n, int d, int h, int w_,
                         int cin, int cout, void* stream) {
-    // measured at 128^3 (TFLOP/s): march / halo block / per-tap TMA
-    //   16->16 170 / 145 / 91, 16->32 238 / 167 / 135, 48->16 128 / 138 / 104,
-    //   32->32 200 / 131 / 225, 64->64 - / 214 / 677
+    // measured (us), row shifts / the form before:
+    //   at 128^3, BF16 output: 16->16 145 / 113 (march), 16->32 159 / 163 (march),
+    //     32->16 273 / 425 (halo block), 48->16 401 / 590 (halo block),
+    //     32->32 195 / 485, 96->32 660 / 1246, 64->64 484 / 640 (per tap)
+    //   at 96^3: 32->32 133 / 270, 48->16 214 / 459 (per tap)
+    //   at 64^3, where a line fills half a tile and the per-tap form packs two:
+    //     16->16 44 / 58, 32->32 61 / 71, 96->32 173 / 171, 32->64 94 / 82, 64->64 129 / 91
+    // so: the march for Cin 16 on rows of at least 128 voxels; row shifts up to
+    // Cout 64 on rows that the per-tap form gives a tile of their own, and for
+    // the narrowest layers on rows of half a tile; else per tap
     MarchConv M;
     if (cin == 16 && march_plan(Vol{n, d, h, w_}, cin, cout, M)) {
         const int rc = nicr_conv3d_fwd_march(x, w, bias, act, y, n, d, h, w_, cin, cout, stream);
         if (rc != NICR_ERR_INVALID_ARG) return rc;
     }
+    if (w_ > TC_M / 2 || (w_ > TC_M / 4 && cout <= 32 && cin * cout <= 1024)) {
+        const int rc = nicr_conv3d_fwd_shift(x, w, bias, act, y, n, d, h, w_, cin, cout, stream);
+        if (rc != NICR_ERR_INVALID_ARG) return rc;
+    }
     HaloConv H;
-    if (cout <= 32 && cin * cout <= 768 && halo_plan(Vol{n, d, h, w_}, cin, cout, H)) {
+    if (halo_shape(Vol{n, d, h, w_}, cin, cout) && halo_plan(Vol{n, d, h, w_}, cin, cout, H)) {
         const int rc = nicr_conv3d_fwd_halo(x, w, bias, act, y, n, d, h, w_, cin, cout, stream);
         if (rc != NICR_ERR_INVALID_ARG) return rc;
     }

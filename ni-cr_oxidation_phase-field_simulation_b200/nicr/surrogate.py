@@ -33,6 +33,12 @@ def _lib():
         L.nicr_conv3d_fwd_act.argtypes = [vp, vp, vp, i, vp, i, i, i, i, i, i, vp]
         L.nicr_conv3d_fwd_halo.argtypes = [vp, vp, vp, i, vp, i, i, i, i, i, i, vp]
         L.nicr_conv3d_fwd_march.argtypes = [vp, vp, vp, i, vp, i, i, i, i, i, i, vp]
+        L.nicr_conv3d_fwd_shift.argtypes = [vp, vp, vp, i, vp, i, i, i, i, i, i, vp]
+        ll = ctypes.c_longlong
+        L.nicr_conv3d_act_bwd.argtypes = [vp, i, vp, i, vp, vp, vp, ll, i, vp]
+        L.nicr_avgpool2_ndhwc.argtypes = [vp, vp, i, i, i, i, i, vp]
+        L.nicr_upcat_ndhwc.argtypes = [vp, vp, vp, i, i, i, i, i, i, vp]
+        L.nicr_pad16.argtypes = [vp, vp, ll, i, vp]
         L.nicr_conv3d_error.argtypes = [ctypes.POINTER(ctypes.c_int)]
         L._conv_bound = True
     return L
@@ -45,15 +51,15 @@ def _check(rc, what):
 
 def conv3d_raw(x, w_bf16, form: str = "tcgen05"):
     """y = conv(x, w): x (n, d, h, w, cin) BF16, w (cout, 27, cin) BF16 -> FP32.
-    form: "tcgen05" (nicr_conv3d_fwd: y-march, halo block, TMA-staged or
-    gathered as the shapes allow), "march", "halo", "tma", "gather" (the
-    tcgen05 forms alone) or "mma_sync"."""
+    form: "tcgen05" (nicr_conv3d_fwd: the fastest form the shapes allow),
+    "shift", "march", "halo", "tma", "gather" (the tcgen05 forms alone) or
+    "mma_sync"."""
     import torch
     n, d, h, wd, cin = x.shape
     cout = w_bf16.shape[0]
     y = torch.empty((n, d, h, wd, cout), dtype=torch.float32, device=x.device)
     stream = torch.cuda.current_stream(x.device).cuda_stream
-    if form in ("halo", "march"):
+    if form in ("halo", "march", "shift"):
         f = f"nicr_conv3d_fwd_{form}"
         _check(getattr(_lib(), f)(x.data_ptr(), w_bf16.data_ptr(), None, 0, y.data_ptr(), n, d, h, wd, cin, cout,
                                   stream), f)
@@ -100,6 +106,35 @@ def conv3d_wgrad_raw(x, dy, form: str = "tcgen05"):
     _check(getattr(_lib(), f)(x.data_ptr(), dy.data_ptr(), dw.data_ptr(), n, d, h, wd, cin, cout,
                               torch.cuda.current_stream(x.device).cuda_stream), f)
     return dw
+
+
+def _stream(t):
+    import torch
+    return torch.cuda.current_stream(t.device).cuda_stream
+
+
+def _act_backward(gy, y):
+    """(g, gb): g = gy * (y > 0) as BF16 (y None: gy), gb its FP32 sum per
+    channel, in one pass (nicr_conv3d_act_bwd)."""
+    import torch
+    gy = gy.contiguous()
+    c = gy.shape[-1]
+    L = _lib()
+    if gy.dtype in (torch.bfloat16, torch.float32):
+        g = torch.empty(gy.shape, dtype=torch.bfloat16, device=gy.device)
+        part = torch.empty((L.nicr_conv3d_act_bwd_blocks(), c), dtype=torch.float32, device=gy.device)
+        gb = torch.empty(c, dtype=torch.float32, device=gy.device)
+        rc = L.nicr_conv3d_act_bwd(gy.data_ptr(), int(gy.dtype == torch.bfloat16), y.data_ptr() if y is not None else None,
+                                   int(y is not None and y.dtype == torch.bfloat16), g.data_ptr(), part.data_ptr(),
+                                   gb.data_ptr(), gy.numel() // c, c, _stream(gy))
+        if rc == 0:
+            return g, gb
+        if rc != 1:   # NICR_ERR_INVALID_ARG: a layout the kernel does not take
+            _check(rc, "nicr_conv3d_act_bwd")
+    g = gy.float()
+    if y is not None:
+        g = g * (y > 0)
+    return g.to(torch.bfloat16).contiguous(), g.sum(dim=tuple(range(g.dim() - 1)))
 
 
 def _data_gradient(gyb, wt, dtype):
@@ -159,13 +194,10 @@ def _make_fn():
         @staticmethod
         def backward(ctx, gy):
             xb, wb, y = ctx.saved_tensors
-            g = gy.float()
-            if ctx.relu:
-                g = g * (y > 0)
-            gb = g.sum(dim=tuple(range(g.dim() - 1)))
-            gyb = g.to(torch.bfloat16).contiguous()
-            wt = wb.flip(1).permute(2, 1, 0).contiguous()
-            gx = _data_gradient(gyb, wt, xb.dtype)
+            gyb, gb = _act_backward(gy, y)
+            gx = None
+            if ctx.needs_input_grad[0]:   # not for the network's first layer
+                gx = _data_gradient(gyb, wb.flip(1).permute(2, 1, 0).contiguous(), xb.dtype)
             gw = conv3d_wgrad_raw(xb, gyb)
             return gx, gw, gb, None, None
 
@@ -209,10 +241,35 @@ def _module_classes():
 
     def pool(x):   # 2x2x2 average, NDHWC
         n, d, h, w, c = x.shape
+        if fused(x):
+            y = torch.empty((n, d // 2, h // 2, w // 2, c), dtype=x.dtype, device=x.device)
+            if _lib().nicr_avgpool2_ndhwc(x.data_ptr(), y.data_ptr(), n, d, h, w, c, _stream(x)) == 0:
+                return y
         return x.float().view(n, d // 2, 2, h // 2, 2, w // 2, 2, c).mean(dim=(2, 4, 6)).to(torch.bfloat16)
 
     def up(x):     # nearest 2x, NDHWC
         return x.repeat_interleave(2, 1).repeat_interleave(2, 2).repeat_interleave(2, 3)
+
+    def upcat(a, b):   # [up(a), b] along the channels
+        n, d, h, w, cb = b.shape
+        if fused(a) and fused(b) and tuple(a.shape[:4]) == (n, d // 2, h // 2, w // 2):
+            y = torch.empty((n, d, h, w, a.shape[-1] + cb), dtype=b.dtype, device=b.device)
+            if _lib().nicr_upcat_ndhwc(a.data_ptr(), b.data_ptr(), y.data_ptr(), n, d, h, w, a.shape[-1], cb,
+                                       _stream(b)) == 0:
+                return y
+        return torch.cat([up(a), b], dim=-1)
+
+    def padded(x):     # FP32 fields -> PAD BF16 channels
+        if not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.float32 and x.is_contiguous():
+            y = torch.empty(x.shape[:-1] + (PAD,), dtype=torch.bfloat16, device=x.device)
+            if _lib().nicr_pad16(x.data_ptr(), y.data_ptr(), x.numel() // x.shape[-1], x.shape[-1], _stream(x)) == 0:
+                return y
+        pad = torch.zeros(x.shape[:-1] + (PAD - x.shape[-1],), dtype=x.dtype, device=x.device)
+        return torch.cat([x, pad], dim=-1).to(torch.bfloat16)
+
+    def fused(x):
+        """The library's one-kernel passes serve inference; training keeps torch's, which record gradients."""
+        return not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous()
 
     class UNet3d(nn.Module):
         """3 levels, `base` channels at full resolution (x2 per level)."""
@@ -230,13 +287,11 @@ def _module_classes():
 
         def forward(self, x):
             """x: (n, d, h, w, fields) FP32, normalised -> the predicted change (same shape)."""
-            pad = torch.zeros(x.shape[:-1] + (PAD - x.shape[-1],), dtype=x.dtype, device=x.device)
-            h0 = torch.cat([x, pad], dim=-1).to(torch.bfloat16)
-            e1 = self.enc1(h0)
+            e1 = self.enc1(padded(x))
             e2 = self.enc2(pool(e1))
             m = self.mid(pool(e2))
-            d2 = self.dec2(torch.cat([up(m), e2], dim=-1))
-            d1 = self.dec1(torch.cat([up(d2), e1], dim=-1))
+            d2 = self.dec2(upcat(m, e2))
+            d1 = self.dec1(upcat(d2, e1))
             return self.head(d1).float()[..., : self.fields]
 
     return Conv, UNet3d
