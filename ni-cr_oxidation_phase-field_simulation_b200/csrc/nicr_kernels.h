@@ -41,6 +41,10 @@ struct Status {
     // domains: the next step's launch reads it (see launch_step_main).
     unsigned long long slot_err[2];
     int pending[2];               // partials of the step of parity q that await their commit (0: none)
+    // a launch of many steps (launch_steps2d): grid barrier arrivals, accepted
+    // steps and the key that ended it, for its commit
+    unsigned long long barrier, multi_key;
+    int multi_steps, pad_;
 };
 constexpr unsigned long long ERR_NONE = ~0ull;
 constexpr unsigned long long ERR_ETA_BASE = 1ull << 62;
@@ -301,6 +305,22 @@ void launch_vti_arrays(const VtiArgs& a, void* out, bool f64, unsigned* range, c
 
 // Commits the pending step, if any: its partials (of parity q at partials +
 // q * cap) reduced, then budget and counters unless a trial failed.
+// Many steps of a small 2D domain in one cooperative launch and its commit
+// (nicr_steps2d.cuh): steps2d_tile gives the tile's planes TX for which the
+// domain's CTAs of TX x 32 cells are resident one per SM (0: too large, or no
+// cooperative launches on the device). The buffers are read at parities par,
+// gpar, epar and written at the others, toggling with each accepted step (gpar
+// and epar only with evolving eta, neta > 0).
+struct Steps2DArgs {
+    double *o[2], *cr[2], *p[2], *gb[2], *s2[2], *eta[2];
+    StepPartial* partials;
+    int neta, nsteps, par, gpar, epar, pad;
+};
+constexpr int kSteps2DMost = 4096;   // steps per launch (tens of milliseconds)
+int steps2d_tile(const Grid& g, int* ctas);
+bool launch_steps2d(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, DevBudget* budget, Status* st,
+                    cudaStream_t stream);
+bool launch_steps2d_fast(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, Status* st, cudaStream_t stream);
 struct FlushDomain {
     const StepPartial* partials;
     DevBudget* budget;

@@ -142,7 +142,7 @@ Model::Model(const nicr_config& cfg, const SlabSpec* slab) : c(cfg), dim(cfg.dim
         red_out = dalloc_t<StepPartial>(1);
         check_cuda(cudaMallocHost(&h_st, sizeof(Status)), "cudaMallocHost");
         check_cuda(cudaMemsetAsync(bud, 0, sizeof(DevBudget), stream), "memset");
-        Status s0{ERR_NONE, 0, 0, -1, 0, {ERR_NONE, ERR_NONE}, {0, 0}};
+        Status s0{ERR_NONE, 0, 0, -1, 0, {ERR_NONE, ERR_NONE}, {0, 0}, 0, ERR_NONE, 0, 0};
         *h_st = s0;
         check_cuda(cudaMemcpyAsync(st, h_st, sizeof(Status), cudaMemcpyHostToDevice, stream), "memcpy");
 
@@ -768,6 +768,9 @@ void Model::reset_status() {
     h_st->failed = 0;
     h_st->timeout = 0;
     h_st->pending[0] = h_st->pending[1] = 0;
+    h_st->barrier = 0;
+    h_st->multi_key = ERR_NONE;
+    h_st->multi_steps = 0;
     h_st->failed_step = -1;
     h_st->steps_done = steps_done;
     h_st->slot_err[0] = h_st->slot_err[1] = ERR_NONE;
@@ -1130,12 +1133,54 @@ int Model::group_length(const RunPlan& r, int s, int nsteps) const {
     return 1;
 }
 
+// n steps (no Ksp scan due after the first) of a 2D domain that fits the
+// resident tiles, in launches of up to kSteps2DMost; false when it does not
+// apply. Not used while profiling (one event pair per kernel launch).
+bool Model::enqueue_steps2d(int n) {
+    if (dim != 2 || is_slab || prof_on || steps2d_failed) return false;
+    int ctas = 0;
+    const int tx = steps2d_tile(g, &ctas);
+    if (!tx || ctas > partial_cap) return false;
+    prepare_step();
+    Steps2DArgs A{};
+    for (int q = 0; q < 2; ++q) {
+        A.o[q] = o_[q]; A.cr[q] = cr_[q]; A.p[q] = p_[q];
+        A.gb[q] = gb_[advance_eta ? q : gcur];
+        A.s2[q] = s2_[advance_eta ? q : gcur];
+        A.eta[q] = eta_[advance_eta ? q : ecur];
+    }
+    A.partials = partials;
+    A.neta = advance_eta ? neta : 0;
+    for (int left = n; left > 0;) {
+        A.nsteps = std::min(left, kSteps2DMost);
+        A.par = cur; A.gpar = gcur; A.epar = ecur;
+        if (!launch_steps2d(sp, A, tx, ctas, bud, st, stream)) {
+            if (left < n) check_cuda(cudaGetLastError(), "cooperative step launch");
+            cudaGetLastError();       // the launch was refused: nothing ran, the stepwise kernels do
+            steps2d_failed = true;
+            return false;
+        }
+        launches += 2;
+        if (A.nsteps & 1) complete_step();   // the parity after n toggles
+        left -= A.nsteps;
+    }
+    return true;
+}
+
+// Steps from s on that no Ksp scan interrupts (a scan before step s itself has run).
+int Model::free_steps(const RunPlan& r, int s, int nsteps) const {
+    int n = 1;
+    while (s + n < nsteps && !ksp_due(r, s + n)) ++n;
+    return n;
+}
+
 int Model::step(int nsteps, int* completed) {
     if (is_slab) throw Error(NICR_ERR_STATE, "a slab is advanced by its slab group");
     if (completed) *completed = 0;
     if (nsteps <= 0) return NICR_OK;
     RunPlan r;
     run_begin(r, nsteps, false);
+    if (enqueue_steps2d(nsteps)) return run_end(r, completed, false);
     const bool graphs = graphs_enabled();
     for (int s = 0; s < nsteps;) {
         const int g = graphs ? group_length(r, s, nsteps) : 1;
@@ -1153,15 +1198,20 @@ int Model::run(int nsteps, int* completed) {
     RunPlan r;
     run_begin(r, nsteps, true);
     const bool graphs = graphs_enabled();
+    bool stepwise = false;   // the last step's commit is pending
     for (int s = 0; s < nsteps;) {
         run_pre_step(r, s);
-        const int g = graphs ? group_length(r, s, nsteps) : 1;
-        if (g > 1) launch_step_group(g);
-        else enqueue_step();
+        int g = free_steps(r, s, nsteps);
+        if (!enqueue_steps2d(g)) {
+            stepwise = true;
+            g = graphs ? group_length(r, s, nsteps) : 1;
+            if (g > 1) launch_step_group(g);
+            else enqueue_step();
+        }
         for (int j = 1; j < g; ++j) run_pre_step(r, s + j);   // no scan is due: schedule entries only
         s += g;
     }
-    return run_end(r, completed);
+    return run_end(r, completed, stepwise);
 }
 
 int Model::slab_launch() {

@@ -138,6 +138,9 @@ public:
     BatchDomain step_desc() const;
     StepParams step_params() const;
     FlushDomain flush_desc() const;
+    bool enqueue_steps2d(int n);
+    int free_steps(const RunPlan& r, int s, int nsteps) const;
+    bool steps2d_failed = false;   // a cooperative launch was refused on this handle
     void flush_commit();   // commits the last enqueued step (each step kernel commits the one before)
     void enqueue_eta();
     void complete_step();

@@ -18,9 +18,11 @@
 // Neumann copies in X for o, cr, phi, gb and for the computed mu and M
 // (refresh copies mu(1) into the ghost, 3S:613-615), periodic rows/columns.
 #include <cstring>
+#include <map>
 
 #include "nicr_step_impl.cuh"
 #include "nicr_step_fused.cuh"
+#include "nicr_steps2d.cuh"
 
 namespace nicr {
 
@@ -111,6 +113,40 @@ __global__ void k_step_flush(const __grid_constant__ FlushList L) {
     if (d.st->failed) return;
     const int q = d.st->pending[0] ? 0 : 1;   // at most one step is pending
     commit_pending(d.partials + (size_t)q * d.cap, q, d.budget, d.st, sdd, scnt);
+}
+
+// Commit of a k_steps2d launch: the accepted steps' budget and count, and the
+// rejection that ended it.
+__global__ void k_steps2d_commit(const StepPartial* __restrict__ partials, int nblocks, DevBudget* budget, Status* st) {
+    __shared__ DD sdd[32 * 5];
+    __shared__ long long scnt[32];
+    if (st->failed || st->timeout) return;
+    DD acc[5] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
+    long long clipped = 0;
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
+        for (int q = 0; q < 5; ++q) {
+            const DD v{partials[b].s[q][0], partials[b].s[q][1]};
+            if (v.hi != 0. || v.lo != 0.) acc[q] = dd_add(acc[q], v);
+        }
+        clipped += partials[b].clipped;
+    }
+    block_reduce_dd<5>(acc, clipped, sdd, scnt);
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 5; ++q) {
+            DD b{budget->v[2 + q][0], budget->v[2 + q][1]};
+            b = dd_add(b, acc[q]);
+            budget->v[2 + q][0] = b.hi;
+            budget->v[2 + q][1] = b.lo;
+        }
+        budget->clipped += clipped;
+        st->steps_done += st->multi_steps;
+        st->barrier = 0;
+        if (st->multi_key != ERR_NONE) {
+            st->err_key = st->multi_key;
+            st->failed = 1;
+            st->failed_step = st->steps_done;
+        }
+    }
 }
 
 // Slab commit: the same reduction; the step's outcome is the failing-trial
@@ -352,6 +388,45 @@ void launch_eta_update(const StepParams& P, int neta, const double* eta, const d
                        double* eta_next, double* gb_next, double* s2_next, Status* st, cudaStream_t stream) {
     if (P.fast) launch_eta_update_fast(P, neta, eta, s2, p, eta_next, gb_next, s2_next, st, stream);
     else launch_eta_form<false>(P, neta, eta, s2, p, eta_next, gb_next, s2_next, st, stream);
+}
+
+int steps2d_tile(const Grid& g, int* ctas) {
+    if (g.dim != 2 || g.ncells > 148LL * 8 * 32) return 0;
+    static std::mutex mu;
+    static std::map<int, std::pair<int, int>> device;   // cooperative launches, SMs
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::pair<int, int> d;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = device.find(dev);
+        if (it == device.end()) {
+            int coop = 0, sms = 0;
+            if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+                return 0;
+            it = device.emplace(dev, std::make_pair(coop, sms)).first;
+        }
+        d = it->second;
+    }
+    if (!d.first) return 0;
+    // the smallest tile whose CTAs fit one per SM: a step's time is its latency,
+    // and more CTAs shorten the halo reads and stores of each
+    for (int tx : {2, 4, 8}) {
+        const long long n = (long long)((g.nx + tx - 1) / tx) * ((g.nb + 31) / 32);
+        if (n <= d.second) {
+            *ctas = (int)n;
+            return tx;
+        }
+    }
+    return 0;
+}
+
+bool launch_steps2d(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, DevBudget* budget, Status* st,
+                    cudaStream_t stream) {
+    const bool ok = P.fast ? launch_steps2d_fast(P, A, tx, ctas, st, stream) : launch_steps2d_form<false>(P, A, tx, ctas, st, stream);
+    if (ok) k_steps2d_commit<<<1, 256, 0, stream>>>(A.partials, ctas, budget, st);
+    return ok;
 }
 
 void launch_step_flush(const FlushDomain* doms, int n, cudaStream_t stream) {

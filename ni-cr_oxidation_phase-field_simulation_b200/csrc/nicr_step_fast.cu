@@ -8,6 +8,7 @@
 // nicr_step_impl.cuh, instantiated with FAST = true.
 #include "nicr_step_impl.cuh"
 #include "nicr_step_fused.cuh"
+#include "nicr_steps2d.cuh"
 
 namespace nicr {
 
@@ -37,6 +38,10 @@ bool launch_step_fused_fast(const StepParams& P, int neta, const double* o, cons
                             cudaStream_t stream, int* nblocks_out) {
     return launch_step_fused_form<true>(P, neta, o, cr, p, eta, on, crn, pn, eta_next, partials, prev, budget, st,
                                         stream, nblocks_out);
+}
+
+bool launch_steps2d_fast(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, Status* st, cudaStream_t stream) {
+    return launch_steps2d_form<true>(P, A, tx, ctas, st, stream);
 }
 
 void step_fused_prepare_fast(const StepParams& P, int neta) {
