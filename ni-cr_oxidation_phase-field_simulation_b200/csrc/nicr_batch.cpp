@@ -3,8 +3,8 @@
 // Ksp schedule, budgets and failure handling, all identical to a single
 // handle); what the batch changes is the launch structure of a step: one
 // k_step_batch launch per group of up to kBatchMax domains instead of one
-// step launch per domain, and one finalize launch for all domains, all on the
-// batch's stream. Small domains (32^3..96^3) would otherwise leave the GPU
+// step launch per domain, and one commit launch for all domains at the end of
+// a call, all on the batch's stream. Small domains (32^3..96^3) would otherwise leave the GPU
 // launch-bound and mostly idle.
 #include <algorithm>
 #include <new>

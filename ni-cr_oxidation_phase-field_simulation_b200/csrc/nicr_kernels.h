@@ -319,15 +319,16 @@ struct Steps2DArgs {
 constexpr int kSteps2DMost = 4096;   // steps per launch (tens of milliseconds)
 int steps2d_tile(const Grid& g, int* ctas);
 bool launch_steps2d(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, DevBudget* budget, Status* st,
-                    cudaStream_t stream);
+                    Status* host, cudaStream_t stream);
 bool launch_steps2d_fast(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, Status* st, cudaStream_t stream);
 struct FlushDomain {
     const StepPartial* partials;
     DevBudget* budget;
     Status* st;
+    Status* host;   // pinned host memory that receives the status
     int cap, pad;
 };
-constexpr int kFlushMax = 512;   // 512 x 32 bytes of kernel parameters
+constexpr int kFlushMax = 512;   // 512 x 40 bytes of kernel parameters
 struct FlushList {
     FlushDomain d[kFlushMax];
 };

@@ -140,7 +140,12 @@ Model::Model(const nicr_config& cfg, const SlabSpec* slab) : c(cfg), dim(cfg.dim
         diag_part = dalloc_t<DiagOut>(148 * 4 + 8);
         diag_out = dalloc_t<DiagOut>(1);
         red_out = dalloc_t<StepPartial>(1);
-        check_cuda(cudaMallocHost(&h_st, sizeof(Status)), "cudaMallocHost");
+        // pinned host memory: the status word and, for small fields, their staging
+        const size_t stage = g.ncells <= kStageCells ? (size_t)g.ncells * 8 : 0;
+        void* pinned = nullptr;
+        check_cuda(cudaMallocHost(&pinned, kStatusBytes + stage), "cudaMallocHost");
+        h_st = static_cast<Status*>(pinned);
+        h_stage = stage ? reinterpret_cast<double*>(static_cast<char*>(pinned) + kStatusBytes) : nullptr;
         check_cuda(cudaMemsetAsync(bud, 0, sizeof(DevBudget), stream), "memset");
         Status s0{ERR_NONE, 0, 0, -1, 0, {ERR_NONE, ERR_NONE}, {0, 0}, 0, ERR_NONE, 0, 0};
         *h_st = s0;
@@ -208,16 +213,25 @@ void Model::release() {
     std::memset(gb_, 0, sizeof gb_); std::memset(s2_, 0, sizeof s2_); std::memset(eta_, 0, sizeof eta_);
     grain = pairs = gb_initial = muO = muCr = mo = mc = nullptr;
     partials = nullptr; st = nullptr; bud = nullptr; diag_part = diag_out = nullptr; red_out = nullptr; kres = nullptr;
-    d_shadow = d_ball = nullptr; d_hyp = nullptr; kw = KspWork{}; h_st = nullptr; stream = nullptr; agree = nullptr; ticket = nullptr;
+    d_shadow = d_ball = nullptr; d_hyp = nullptr; kw = KspWork{}; h_st = nullptr; h_stage = nullptr; stream = nullptr; agree = nullptr; ticket = nullptr;
     gw = GrainWork{}; g_out = nullptr; g_amount = nullptr; g_cells = nullptr;
 }
 
 void Model::sync() { check_cuda(cudaStreamSynchronize(stream), "stream"); }
 
 void Model::copy_out(const double* d, double* host) {
-    check_cuda(cudaMemcpy2DAsync(host, (size_t)g.nb * 8, d, (size_t)g.pb * 8, (size_t)g.nb * 8, (size_t)g.nx * g.na,
-                                 cudaMemcpyDeviceToHost, stream), "D2H");
+    // A small field bound for pageable memory goes through pinned staging: the
+    // driver's own pageable path costs more than the copy (61^2 cells 26 -> 16
+    // us, 180^2 37 -> 29 us; above that the host-side copy takes the gain).
+    bool staged = h_stage != nullptr;
+    if (staged) {
+        cudaPointerAttributes at{};
+        staged = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+    }
+    check_cuda(cudaMemcpy2DAsync(staged ? h_stage : host, (size_t)g.nb * 8, d, (size_t)g.pb * 8, (size_t)g.nb * 8,
+                                 (size_t)g.nx * g.na, cudaMemcpyDeviceToHost, stream), "D2H");
     sync();
+    if (staged) std::memcpy(host, h_stage, (size_t)g.ncells * 8);
 }
 void Model::copy_in(double* d, const double* host) {
     check_cuda(cudaMemcpy2DAsync(d, (size_t)g.pb * 8, host, (size_t)g.nb * 8, (size_t)g.nb * 8, (size_t)g.nx * g.na,
@@ -763,6 +777,11 @@ void Model::get_field(int field, int index, double* host) { copy_out(field_ptr(f
 
 // ------------------------------------------------------------------ stepping
 void Model::reset_status() {
+    // after an accepted run the device's word is what this would write (its
+    // copy on the host says so): nothing to send
+    const bool clean = !is_slab && status_clean && h_st->steps_done == steps_done;
+    status_clean = false;   // until the next accepted run
+    if (clean) return;
     // keep steps_done; clear the failure state for a new batch
     h_st->err_key = ERR_NONE;
     h_st->failed = 0;
@@ -808,6 +827,7 @@ void Model::launch_trial_kernels() {
 void Model::tune(int reps, int* xchunk, int* minb) {
     reps = std::max(1, reps);
     if (!onepass_step()) prepare_step();
+    status_clean = false;   // trial launches use the error word
     reset_status();   // trial kernels of a failing state must not stop the timing runs
     cudaEvent_t e0, e1;
     check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
@@ -853,7 +873,7 @@ StepParams Model::step_params() const {
     return q;
 }
 
-FlushDomain Model::flush_desc() const { return FlushDomain{partials, bud, st, partial_cap, 0}; }
+FlushDomain Model::flush_desc() const { return FlushDomain{partials, bud, st, h_st, partial_cap, 0}; }
 
 void Model::flush_commit() {
     const size_t e = prof_begin();
@@ -997,13 +1017,17 @@ std::string Model::describe_failure(unsigned long long key, int nxt) {
 }
 
 int Model::finish_batch(long long before, int enqueued, const std::vector<double>* nuc_sched, int* completed) {
-    check_cuda(cudaMemcpyAsync(h_st, st, sizeof(Status), cudaMemcpyDeviceToHost, stream), "D2H");
+    // a whole domain's last commit has written the status word to h_st
+    if (is_slab) check_cuda(cudaMemcpyAsync(h_st, st, sizeof(Status), cudaMemcpyDeviceToHost, stream), "D2H");
     sync();
     check_cuda(cudaGetLastError(), "step kernels");
     profile_collect();
     if (h_st->timeout)
         throw Error(NICR_ERR_CUDA, "a step kernel's bounded wait for its own copies ran out; the step results are not valid");
     if (!h_st->failed) {
+        if (!is_slab && h_st->steps_done != before + enqueued)
+            throw Error(NICR_ERR_CUDA, "the step kernels did not complete their steps; the step results are not valid");
+        status_clean = !is_slab;
         steps_done = before + enqueued;
         if (completed) *completed = enqueued;
         return NICR_OK;
@@ -1154,7 +1178,7 @@ bool Model::enqueue_steps2d(int n) {
     for (int left = n; left > 0;) {
         A.nsteps = std::min(left, kSteps2DMost);
         A.par = cur; A.gpar = gcur; A.epar = ecur;
-        if (!launch_steps2d(sp, A, tx, ctas, bud, st, stream)) {
+        if (!launch_steps2d(sp, A, tx, ctas, bud, st, h_st, stream)) {
             if (left < n) check_cuda(cudaGetLastError(), "cooperative step launch");
             cudaGetLastError();       // the launch was refused: nothing ran, the stepwise kernels do
             steps2d_failed = true;

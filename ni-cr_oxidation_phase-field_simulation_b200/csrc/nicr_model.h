@@ -257,6 +257,10 @@ private:
     long long* g_cells = nullptr;
     // pinned host staging for small results
     Status* h_st = nullptr;
+    double* h_stage = nullptr;            // pinned staging of one small field (behind h_st)
+    bool status_clean = false;            // the device's status word is h_st's, as an accepted run leaves it
+    static constexpr size_t kStatusBytes = 256;
+    static constexpr long long kStageCells = 32768;
     // profiling
     bool prof_on = false;
     std::vector<cudaEvent_t> prof_pool;

@@ -105,21 +105,31 @@ __global__ void k_check_division(DivC d, long long n, unsigned long long seed, u
     atomicAdd(counts + 1, total);
 }
 
-// CTA b commits domain b's pending step.
+// The status word into pinned host memory, as a run's last device write: the
+// host reads it after the stream, without a copy of its own.
+__device__ __forceinline__ void report_status(const Status* st, Status* host) {
+    __syncthreads();
+    if (threadIdx.x < sizeof(Status) / 4)
+        reinterpret_cast<volatile unsigned*>(host)[threadIdx.x] = reinterpret_cast<const volatile unsigned*>(st)[threadIdx.x];
+    __threadfence_system();
+}
+
+// CTA b commits domain b's pending step and reports its status.
 __global__ void k_step_flush(const __grid_constant__ FlushList L) {
     __shared__ DD sdd[32 * 5];
     __shared__ long long scnt[32];
     const FlushDomain& d = L.d[blockIdx.x];
-    if (d.st->failed) return;
-    const int q = d.st->pending[0] ? 0 : 1;   // at most one step is pending
-    commit_pending(d.partials + (size_t)q * d.cap, q, d.budget, d.st, sdd, scnt);
+    if (!d.st->failed) {
+        const int q = d.st->pending[0] ? 0 : 1;   // at most one step is pending
+        commit_pending(d.partials + (size_t)q * d.cap, q, d.budget, d.st, sdd, scnt);
+    }
+    report_status(d.st, d.host);
 }
 
 // Commit of a k_steps2d launch: the accepted steps' budget and count, and the
 // rejection that ended it.
-__global__ void k_steps2d_commit(const StepPartial* __restrict__ partials, int nblocks, DevBudget* budget, Status* st) {
-    __shared__ DD sdd[32 * 5];
-    __shared__ long long scnt[32];
+__device__ __forceinline__ void steps2d_commit_body(const StepPartial* __restrict__ partials, int nblocks,
+                                                    DevBudget* budget, Status* st, DD* sdd, long long* scnt) {
     if (st->failed || st->timeout) return;
     DD acc[5] = {{0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}, {0., 0.}};
     long long clipped = 0;
@@ -147,6 +157,13 @@ __global__ void k_steps2d_commit(const StepPartial* __restrict__ partials, int n
             st->failed_step = st->steps_done;
         }
     }
+}
+__global__ void k_steps2d_commit(const StepPartial* __restrict__ partials, int nblocks, DevBudget* budget, Status* st,
+                                 Status* host) {
+    __shared__ DD sdd[32 * 5];
+    __shared__ long long scnt[32];
+    steps2d_commit_body(partials, nblocks, budget, st, sdd, scnt);
+    report_status(st, host);
 }
 
 // Slab commit: the same reduction; the step's outcome is the failing-trial
@@ -423,9 +440,9 @@ int steps2d_tile(const Grid& g, int* ctas) {
 }
 
 bool launch_steps2d(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, DevBudget* budget, Status* st,
-                    cudaStream_t stream) {
+                    Status* host, cudaStream_t stream) {
     const bool ok = P.fast ? launch_steps2d_fast(P, A, tx, ctas, st, stream) : launch_steps2d_form<false>(P, A, tx, ctas, st, stream);
-    if (ok) k_steps2d_commit<<<1, 256, 0, stream>>>(A.partials, ctas, budget, st);
+    if (ok) k_steps2d_commit<<<1, 256, 0, stream>>>(A.partials, ctas, budget, st, host);
     return ok;
 }
 

@@ -224,6 +224,7 @@ class Solver:
         self.info_ = self.info()
         self.shape = (cfg.nx, cfg.ny, cfg.nz) if cfg.dim == 3 else (cfg.nx, cfg.ny)
         self.n = int(np.prod(self.shape))
+        self._device = f"cuda:{cfg.device}"
 
     @classmethod
     def _borrowed(cls, handle: int, cfg: NicrConfig, owner):
@@ -425,20 +426,22 @@ class Solver:
         if name.startswith("eta") and name[3:].isdigit():
             index, name = int(name[3:]) - 1, "eta"
         ptr, pitch = ctypes.c_void_p(), ctypes.c_longlong()
-        self._check(lib().nicr_field_device(self.h, FIELD[name], index, int(writable), ctypes.byref(ptr),
-                                            ctypes.byref(pitch)))
-        i = self.info()
-        rows = i.ny if i.dim == 3 else 1
-        cols = i.nz if i.dim == 3 else i.ny
+        rc = lib().nicr_field_device(self.h, FIELD[name], index, int(writable), ctypes.byref(ptr),
+                                      ctypes.byref(pitch))
+        if rc:
+            self._check(rc)
+        three = len(self.shape) == 3
+        rows = self.shape[1] if three else 1
+        p8 = pitch.value * 8
         # torch takes no read-only CUDA arrays: a read view must not be written
-        view = _DeviceArray(ptr.value, (i.nx, rows, cols), (rows * pitch.value * 8, pitch.value * 8, 8))
-        t = torch.as_tensor(view, device=f"cuda:{self.cfg.device}")
-        return t if i.dim == 3 else t[:, 0, :]
+        view = _DeviceArray(ptr.value, (self.shape[0], rows, self.shape[-1]), (rows * p8, p8, 8))
+        t = torch.as_tensor(view, device=self._device)
+        return t if three else t[:, 0, :]
 
 
 class Batch:
     """Independent domains on one GPU advanced together (nicr_batch_*): one
-    step launch per group of up to 48 domains, one commit launch per step.
+    step launch per group of up to 48 domains, one commit launch per call.
     ``domains[i]`` is a Solver view of domain i (owned by the batch)."""
 
     def __init__(self, cfgs):
