@@ -119,8 +119,13 @@ def _act_backward(gy, y):
     import torch
     gy = gy.contiguous()
     c = gy.shape[-1]
-    L = _lib()
-    if gy.dtype in (torch.bfloat16, torch.float32):
+    # torch's operations serve what the kernel cannot: host tensors, a gradient
+    # of this gradient, activations that a saved-tensor hook has handed back
+    # in another layout
+    if (gy.is_cuda and gy.dtype in (torch.bfloat16, torch.float32) and not torch.is_grad_enabled()
+            and (y is None or (y.device == gy.device and y.shape == gy.shape and y.is_contiguous()
+                               and y.dtype in (torch.bfloat16, torch.float32)))):
+        L = _lib()
         g = torch.empty(gy.shape, dtype=torch.bfloat16, device=gy.device)
         part = torch.empty((L.nicr_conv3d_act_bwd_blocks(), c), dtype=torch.float32, device=gy.device)
         gb = torch.empty(c, dtype=torch.float32, device=gy.device)
@@ -260,7 +265,7 @@ def _module_classes():
         return torch.cat([up(a), b], dim=-1)
 
     def padded(x):     # FP32 fields -> PAD BF16 channels
-        if not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.float32 and x.is_contiguous():
+        if eager(x) and x.dtype == torch.float32 and x.is_contiguous():
             y = torch.empty(x.shape[:-1] + (PAD,), dtype=torch.bfloat16, device=x.device)
             if _lib().nicr_pad16(x.data_ptr(), y.data_ptr(), x.numel() // x.shape[-1], x.shape[-1], _stream(x)) == 0:
                 return y
@@ -269,7 +274,11 @@ def _module_classes():
 
     def fused(x):
         """The library's one-kernel passes serve inference; training keeps torch's, which record gradients."""
-        return not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous()
+        return eager(x) and x.dtype == torch.bfloat16 and x.is_contiguous()
+
+    def eager(x):
+        """No gradients and no trace to be recorded: a trace would hold a pass of the library as a constant."""
+        return not torch.is_grad_enabled() and x.is_cuda and not torch.jit.is_tracing()
 
     class UNet3d(nn.Module):
         """3 levels, `base` channels at full resolution (x2 per level)."""

@@ -22,7 +22,8 @@ def test_act_backward(require_gpu, c, rows, gy_dtype, y_dtype):
     g = torch.Generator(device="cuda").manual_seed(c + rows)
     gy = torch.randn((rows, c), generator=g, device="cuda").to(gy_dtype)
     y = None if y_dtype is None else torch.randn((rows, c), generator=g, device="cuda").relu().to(y_dtype)
-    got, gb = surrogate._act_backward(gy, y)
+    with torch.no_grad():   # as the backward without a graph of its own runs
+        got, gb = surrogate._act_backward(gy, y)
     ref = gy.float() if y is None else gy.float() * (y > 0)
     assert torch.equal(got, ref.to(torch.bfloat16))
     exact, size = ref.double().sum(0), ref.double().abs().sum(0)
@@ -35,7 +36,8 @@ def test_act_backward_passes_nonfinite_values(require_gpu):
     y = torch.ones((64, 16), device="cuda", dtype=torch.bfloat16)
     y[4, 5] = 0.0        # inf x 0 is NaN, as in the torch product
     y[6, 6] = float("nan")
-    got, gb = surrogate._act_backward(gy, y)
+    with torch.no_grad():
+        got, gb = surrogate._act_backward(gy, y)
     ref = gy * (y > 0)
     assert torch.equal(torch.nan_to_num(got.float(), nan=7.0), torch.nan_to_num(ref.to(torch.bfloat16).float(), nan=7.0))
     assert torch.equal(torch.isnan(gb), torch.isnan(ref.sum(0)))
@@ -67,3 +69,28 @@ def test_first_layer_needs_no_input_gradient(require_gpu):
     gx2, gw2, gb2 = torch.autograd.grad(y2.float().square().sum(), (xg, w, b))
     assert gx2.shape == x.shape and torch.equal(gb, gb2)
     assert np.allclose(gw.cpu(), gw2.cpu(), rtol=1e-5, atol=1e-5 * float(gw.abs().max()))   # FP32 atomics: order of sums
+
+
+def test_bias_gradient_is_differentiable(require_gpu):
+    """A backward that records a graph keeps torch's operations: the bias
+    gradient's derivative along the output gradient is the ReLU's mask."""
+    x = torch.randn((1, 4, 8, 16, 16), device="cuda").bfloat16()
+    w = (0.1 * torch.randn((16, 27, 16), device="cuda")).requires_grad_()
+    b = torch.zeros(16, device="cuda", requires_grad=True)
+    y = surrogate.conv3d_act(x, w, b, True, False)
+    dy = torch.randn_like(y).requires_grad_()
+    gb, = torch.autograd.grad(y, (b,), dy, create_graph=True)
+    mask, = torch.autograd.grad(gb.sum(), (dy,))
+    assert torch.equal(mask, (y > 0).float())
+
+
+@pytest.mark.parametrize("y", [None, torch.float32, torch.bfloat16])
+def test_act_backward_of_other_layouts(require_gpu, y):
+    """Stored activations in another stride order take torch's operations."""
+    gy = torch.randn((6, 4, 16), device="cuda")
+    act = None if y is None else torch.randn((4, 6, 16), device="cuda").relu().to(y).transpose(0, 1)
+    with torch.no_grad():
+        got, gb = surrogate._act_backward(gy, act)
+    ref = gy if act is None else gy * (act > 0)
+    assert torch.equal(got, ref.to(torch.bfloat16))
+    assert bool(((gb - ref.sum((0, 1))).abs() <= 2e-6 * ref.abs().sum((0, 1))).all())
