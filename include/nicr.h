@@ -538,6 +538,8 @@ long long nicr_kernel_launches(const nicr_handle* h);
  * of results that differ (0 expected) or -1 on a CUDA error; *tested receives
  * the number of finite numerators checked. No counterpart in the reference. */
 long long nicr_check_division(double b, long long n, unsigned long long seed, long long* tested);
+/* 1 when two operations divide exactly by b, whatever the numerator (decided on the host). */
+int nicr_division_in_two(double b);
 
 #ifdef __cplusplus
 }

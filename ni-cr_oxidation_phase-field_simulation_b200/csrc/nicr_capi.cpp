@@ -213,6 +213,7 @@ const char* nicr_profile_kernel_name(int kernel) { return nicr::Model::kernel_na
 
 long long nicr_kernel_launches(const nicr_handle* h) { return (h && h->m) ? h->m->launches : -1; }
 
+int nicr_division_in_two(double b) { return nicr::division_in_two(b) ? 1 : 0; }
 long long nicr_check_division(double b, long long n, unsigned long long seed, long long* tested) {
     return nicr::check_division(b, n, seed, tested);
 }

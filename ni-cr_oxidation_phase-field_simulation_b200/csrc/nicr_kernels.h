@@ -65,7 +65,8 @@ struct StepPartial {
 // Exact divisions by the run constants (drop-in form): dx*dx etc. are the
 // Laplacian denominators (3S:193-195); X, rows (a), columns (b).
 struct DivSet {
-    DivC dxdx, dada, dbdb, dx, da, db, dt;
+    DivC dxdx, dada, dbdb, dt;
+    DivF dx, da, db;
 };
 // The reciprocal form's run constants, folded on the host so that the kernels
 // spend one multiply-add per neighbour pair and no separate scaling.
@@ -113,7 +114,8 @@ struct StepParams {
     int err_slot;
     int slab, pad_;              // an X slab (its plane range and key offsets apply)
     // drop-in form: 1 when a divisor or a constant after a scaled quotient
-    // lies outside the certified range, so every chunk is divided by IEEE division
+    // lies outside the certified range, so every chunk is divided by IEEE
+    // division; 2 when two operations divide by each of them (division_in_two)
     unsigned div_gate;
 };
 // The run constants of the configured form (spacings along X, rows, columns);
@@ -133,7 +135,12 @@ inline DivSet fill_form_constants(StepParams& sp, int dim, double dx, double da,
         sp.dt_s = std::ldexp(sp.dt, -128);
         sp.etaK_s = std::ldexp(sp.eta_K, -128);
         const bool k_ok = sp.eta_K == 0. || (std::fabs(sp.eta_K) >= std::ldexp(1., -500) && std::fabs(sp.eta_K) <= std::ldexp(1., 500));
-        sp.div_gate = d.dxdx.gate | d.dada.gate | d.dbdb.gate | d.dx.gate | d.da.gate | d.db.gate | d.dt.gate | (k_ok ? 0u : 1u);
+        bool in_range = k_ok, in_two = true;
+        for (double b : {d.dxdx.b, d.dada.b, d.dbdb.b, d.dt.b, d.dx.b, d.da.b, d.db.b}) {
+            in_range = in_range && div_in_range(b);
+            in_two = in_two && division_in_two(b);
+        }
+        sp.div_gate = !in_range ? 1u : in_two ? 2u : 0u;
         return d;
     }
     FastC f{};

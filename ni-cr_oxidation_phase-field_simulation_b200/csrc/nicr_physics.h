@@ -6,6 +6,7 @@
 // 2D = mpi2d/NiCr2D_grains.cpp.
 #pragma once
 #include <cmath>
+#include <limits>
 
 #ifdef __CUDACC__
 #define NICR_HD __host__ __device__ __forceinline__
@@ -97,10 +98,11 @@ inline EtaCoef eta_coef(double fwhm, double dx, double W, double kappa, double p
 // The host stores y = RN(1/b) and the double-word reciprocal zh = RD(1/b),
 // zl = RN(1/b - zh) >= 0 (Brisebarre, Muller, Raina, "Accelerating correctly
 // rounded floating-point division when the divisor is known in advance",
-// IEEE Trans. Comput. 53(8), 2004). For b > 0 with 2^-60 <= b <= 2^60 and a
-// numerator a:
+// IEEE Trans. Comput. 53(8), 2004), also times 2^128 (uh, ul). For b > 0 with
+// 2^-60 <= b <= 2^60 and a numerator a:
 //   as = a * 2^128                  exact for |a| < 2^895, subnormals included,
-//   q0 = RN(as*zh + RN(as*zl))      within (1/2 + 2^-51) ulp of as/b,
+//   q0 = RN(as*zh + RN(as*zl))      = RN(a*uh + RN(a*ul)), the same products:
+//                                   within (1/2 + 2^-51) ulp of as/b,
 //   e  = q0*b - as                  exact: q0 is within one ulp of as/b, and
 //                                   as/b >= 2^-1006 keeps its bits normal,
 //   qs = RN(q0 - e*y)               = RN(as/b), Markstein's correction theorem
@@ -108,24 +110,31 @@ inline EtaCoef eta_coef(double fwhm, double dx, double W, double kappa, double p
 //                                   ulp, y within half an ulp of 1/b, exact
 //                                   remainder => the correctly rounded quotient),
 //   q  = qs * 2^-128                exact whenever a/b is normal or zero.
+// For most divisors q0 is RN(as/b) already, whatever the numerator, and
+// division_in_two() proves it (the same paper): two operations instead of five.
 // The scaling keeps tiny numerators (the tails of diffusing fields) exact.
 // Zeros come out with the IEEE sign because zl >= 0 and e is formed as
 // q0*b - as. A quotient that is subnormal (qs nonzero below 2^-894, which the
 // final scaling would round a second time), infinite or NaN (infinite, NaN or
-// huge numerators), or any quotient of a divisor outside the range, is
-// flagged. tests/division_check.c restates this on the host and checks it
-// against IEEE division, near-midpoint quotients included. Sums and products
-// of scaled quotients round as the unscaled ones do (a power of two, and sums
-// that reach the subnormal range are exact), so the kernels keep quotients
-// scaled through a sum and fold 2^-128 into the constant that follows it.
+// huge numerators) is flagged, and so is any quotient of a divisor outside the
+// range, whose reciprocals are NaN here. tests/division_check.c restates this
+// on the host and checks it against IEEE division, near-midpoint quotients
+// included. Sums and products of scaled quotients round as the unscaled ones
+// do (a power of two, and sums that reach the subnormal range are exact), so
+// the kernels keep quotients scaled through a sum and fold 2^-128 into the
+// constant that follows it.
 struct DivC {
     double b, rb;      // divisor and y = RN(1/b) (the reciprocal form multiplies by it)
-    double zh, zl;     // RD(1/b) and RN(1/b - RD(1/b))
-    unsigned gate;     // 0 when b is in range, else 1 (every quotient flagged)
-    unsigned pad;
+    double uh, ul;     // 2^128 times RD(1/b) and RN(1/b - RD(1/b))
 };
-inline DivC make_divc(double b) {
-    DivC d;
+struct DivF : DivC {   // numerators in the carried scale too
+    double zh, zl;     // RD(1/b) and RN(1/b - RD(1/b))
+};
+inline bool div_in_range(double b) {
+    return std::isnormal(b) && b > 0. && b >= std::ldexp(1.0, -60) && b <= std::ldexp(1.0, 60);
+}
+inline DivF make_divc(double b) {
+    DivF d;
     d.b = b;
     d.rb = 1.0 / b;
     double zh = d.rb;
@@ -136,29 +145,77 @@ inline DivC make_divc(double b) {
     }
     d.zh = zh;
     d.zl = rem / b;
-    const bool in_range = std::isnormal(b) && b > 0. && b >= std::ldexp(1.0, -60) && b <= std::ldexp(1.0, 60);
-    d.gate = in_range ? 0u : 1u;
-    d.pad = 0;
+    if (!div_in_range(b)) d.zh = d.zl = std::numeric_limits<double>::quiet_NaN();
+    d.uh = std::ldexp(d.zh, 128);
+    d.ul = std::ldexp(d.zl, 128);
     return d;
+}
+// Whether RN(X*zh + RN(X*zl)) = RN(X/b) for every numerator. With zl at most
+// 2^-52 of zh and two roundings of relative size 2^-53 in X*zl, the sum before
+// its rounding lies within 2^-103 of X/b (relative), so it can round otherwise
+// only if a rounding midpoint lies that close to X/b. For significands X and Y
+// (53-bit integers) midpoints are M/2^s with M odd, 2^53 < M < 2^54 and s = 53
+// (X >= Y) or 54; X/Y - M/2^s = k/(2^s Y) with k = 2^s X - M Y an integer, not
+// zero, and the distance bounds |k| by 16. Each k leaves few M modulo 2^s:
+// those numerators are tried against IEEE division.
+inline bool division_in_two(double b) {
+    if (!div_in_range(b)) return false;
+    int e;
+    const double y = std::ldexp(std::frexp(b, &e), 53);   // Y, an integer below 2^53
+    const DivF d = make_divc(y);
+    const unsigned long long Y = (unsigned long long)y;
+    const int t = __builtin_ctzll(Y);
+    const unsigned long long Yo = Y >> t;
+    unsigned long long inv = Yo;   // 1 / Yo modulo 2^64 (Newton)
+    for (int i = 0; i < 6; ++i) inv *= 2 - Yo * inv;
+    for (int s = 53; s <= 54; ++s) {
+        const unsigned long long mod = 1ull << (s - t), most = 1ull << 54;
+        for (int k = -16; k <= 16; ++k) {
+            if (k == 0 || t > 4 || k % (1 << t) != 0 || (k / (1 << t)) % 2 == 0) continue;   // M odd needs k / 2^t odd
+            // M Y = -k modulo 2^s
+            for (unsigned long long M = (0ull - (unsigned long long)(long long)(k / (1 << t))) * inv & (mod - 1); M < most; M += mod) {
+                if (M <= (most >> 1)) continue;
+                const __int128 n = (__int128)M * (__int128)Y + k;
+                const double X = (double)(long long)(n >> s);
+                if (X < 0x1p52 || X >= 0x1p53) continue;
+                if (std::fma(X, d.zh, X * d.zl) != X / y) return false;
+            }
+        }
+    }
+    return true;
 }
 #ifdef __CUDACC__
 // IEEE division kept out of line: it is only the rare fallback, and inlining
 // it at every call site would multiply the kernels' instruction footprint.
 __device__ __noinline__ double ieee_div(double a, double b);
-// The exact quotient; a flagged one (see DivC) sets `bad` (the value returned
-// for it is then not the IEEE quotient), so a caller can test once for a
-// whole group of divisions and recompute the group with IEEE division.
-// the scaled quotient of a scaled numerator (uncertified)
-__device__ __forceinline__ double xdiv_scaled(double as, const DivC& d) {
+// the scaled quotient (uncertified) of an unscaled numerator
+__device__ __forceinline__ double xdiv_up(double a, const DivC& d) {
+    const double q0 = __fma_rn(a, d.uh, __dmul_rn(a, d.ul));
+    const double e = __fma_rn(q0, d.b, -__dmul_rn(a, 0x1p128));
+    return __fma_rn(-e, d.rb, q0);
+}
+// and of a scaled one
+__device__ __forceinline__ double xdiv_scaled(double as, const DivF& d) {
     const double q0 = __fma_rn(as, d.zh, __dmul_rn(as, d.zl));
     const double e = __fma_rn(q0, d.b, -as);
     return __fma_rn(-e, d.rb, q0);
 }
-__device__ __forceinline__ double xdiv_flag(double a, const DivC& d, unsigned& bad) {
-    const double qs = xdiv_scaled(__dmul_rn(a, 0x1p128), d);
-    // |qs| in (0, 2^-894): a subnormal quotient; >= 2^1024: infinite or NaN
+// The same where division_in_two(d.b)
+__device__ __forceinline__ double xdiv_up2(double a, const DivC& d) { return __fma_rn(a, d.uh, __dmul_rn(a, d.ul)); }
+__device__ __forceinline__ double xdiv_scaled2(double as, const DivF& d) {
+    return __fma_rn(as, d.zh, __dmul_rn(as, d.zl));
+}
+// |qs| in (0, 2^-894): a subnormal quotient; >= 2^1024: infinite or NaN
+__device__ __forceinline__ unsigned xdiv_uncertified(double qs) {
     const unsigned u = (unsigned)__double2hiint(qs) & 0x7FFFFFFFu;
-    bad |= ((u - 1u) < 0x080FFFFFu || u >= 0x7FF00000u || d.gate) ? 1u : 0u;
+    return ((u - 1u) < 0x080FFFFFu || u >= 0x7FF00000u) ? 1u : 0u;
+}
+// The exact quotient; a flagged one (see DivC) sets `bad` (the value returned
+// for it is then not the IEEE quotient), so a caller can test once for a
+// whole group of divisions and recompute the group with IEEE division.
+__device__ __forceinline__ double xdiv_flag(double a, const DivC& d, unsigned& bad) {
+    const double qs = xdiv_up(a, d);
+    bad |= xdiv_uncertified(qs);
     return __dmul_rn(qs, 0x1p-128);
 }
 __device__ __forceinline__ double xdiv(double a, const DivC& d) {

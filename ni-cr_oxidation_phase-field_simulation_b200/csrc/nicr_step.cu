@@ -56,13 +56,14 @@ __global__ void k_eta_mask(const StepParams P, int neta, const double* __restric
     }
 }
 
-// Self-check of xdiv on the device against IEEE division: random numerators
+// Self-check of xdiv, and of the two-operation form where it applies, on the
+// device against IEEE division: random numerators
 // (all finite bit patterns, values of typical magnitude, signed zeros) and,
 // every fifth one, a numerator whose quotient lies within ~2^-104 relative of
 // a rounding midpoint. The latter: b's odd mantissa part B, M = delta / B mod
 // 2^54 for delta in {-3, -1, 1, 3}, kept when M has 54 bits; then
 // B * M = A * 2^54 + delta and A (scaled) / b is next to the midpoint M * 2^-54.
-__global__ void k_check_division(DivC d, long long n, unsigned long long seed, unsigned long long* counts) {
+__global__ void k_check_division(DivF d, int two, long long n, unsigned long long seed, unsigned long long* counts) {
     unsigned long long bad = 0, total = 0;
     unsigned long long B = ((unsigned long long)__double_as_longlong(d.b) & 0x000FFFFFFFFFFFFFull) | (1ull << 52);
     while (!(B & 1)) B >>= 1;
@@ -99,6 +100,11 @@ __global__ void k_check_division(DivC d, long long n, unsigned long long seed, u
         }
         const double q = xdiv(a, d), w = __ddiv_rn(a, d.b);
         bad += __double_as_longlong(q) != __double_as_longlong(w);
+        if (two) {   // the two-operation quotients that are certified
+            const double qs = xdiv_up2(a, d), qt = xdiv_scaled2(__dmul_rn(a, 0x1p128), d);
+            for (double v : {qs, qt})
+                if (!xdiv_uncertified(v)) bad += __double_as_longlong(__dmul_rn(v, 0x1p-128)) != __double_as_longlong(w);
+        }
         ++total;
     }
     atomicAdd(counts, bad);
@@ -584,7 +590,7 @@ long long check_division(double b, long long n, unsigned long long seed, long lo
     unsigned long long* d = nullptr;
     if (cudaMalloc(&d, 2 * sizeof(unsigned long long)) != cudaSuccess) return -1;
     cudaMemset(d, 0, 2 * sizeof(unsigned long long));
-    k_check_division<<<148 * 8, 256>>>(make_divc(b), n, seed, d);
+    k_check_division<<<148 * 8, 256>>>(make_divc(b), division_in_two(b), n, seed, d);
     unsigned long long h[2] = {0, 0};
     const cudaError_t e = cudaMemcpy(h, d, sizeof h, cudaMemcpyDeviceToHost);
     cudaFree(d);

@@ -132,7 +132,7 @@ struct OnePassStep {
     // One march over the CTA's chunk with the division policy of DM (DivOf).
     // kb offsets the staging ring's plane counter (slot and phase of each
     // copy), so a second march continues the mbarrier phases of the first;
-    // DM 1 returns true, without publishing keys or partials, when a
+    // A first pass returns true, without publishing keys or partials, when a
     // numerator of the chunk left the exact-division range.
     template <int DM>
     __device__ static bool run_body(const StepParams& P, const CUtensorMap* m_int, const CUtensorMap* m_row,
@@ -157,7 +157,7 @@ struct OnePassStep {
         double* ering = reinterpret_cast<double*>(
             fused_smem + L::STEP_BYTES + ((128u - (smem_u32(fused_smem + L::STEP_BYTES) & 127u)) & 127u));
 
-        unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+        unsigned low = kFirstPass<DM> && P.div_gate == 1 ? 0u : ~0u;
         const typename DivOf<DM>::T dv{P, low};
 
         const bool o_on = MODE == 1 ? true : P.o_on != 0;
@@ -414,7 +414,7 @@ struct OnePassStep {
             return false;
         }
         const unsigned long long errkey = book.key();
-        if (DM == 1 && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
+        if (kFirstPass<DM> && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
         if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
         DD acc[5];
         long long clipped = book.clipped();
@@ -458,8 +458,10 @@ struct OnePassStep {
         __shared__ unsigned long long bars[L::RING];
         if (FAST) {
             run_body<0>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials, st, bars, 0, bx, by, bz);
-        } else if (run_body<1>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials, st, bars,
-                               0, bx, by, bz)) {
+        } else if (P.div_gate == 2 ? run_body<3>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials,
+                                                 st, bars, 0, bx, by, bz)
+                                   : run_body<1>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials,
+                                                 st, bars, 0, bx, by, bz)) {
             const int i0 = bz * P.xchunk, i1 = min(P.g.nx, i0 + P.xchunk);
             __syncthreads();
             run_body<2>(P, m_int, m_row, m_col, m_crn, o, cr, p, on, crn, pn, eta_next, partials, st, bars,

@@ -170,17 +170,21 @@ struct Reciprocal {
     const StepParams& P;
     unsigned& low;   // unused
 };
+// TWO: every divisor takes two operations (division_in_two; dx, dx^2 and dt of
+// the default configurations, 93% of random divisors), instead of four or, from
+// an unscaled numerator, five. FIGURES
+template <bool TWO>
 struct DivRun {
     static constexpr bool kFast = false;
     static constexpr double S = 0x1p-128;
     const StepParams& P;
     unsigned& low;
-    __device__ double same(double as, const DivC& d) const {
-        const double qs = xdiv_scaled(as, d);
+    __device__ double note(double qs) const {
         low = min(low, 2u * (unsigned)__double2hiint(qs) - 1u);
         return qs;
     }
-    __device__ double up(double a, const DivC& d) const { return same(__dmul_rn(a, 0x1p128), d); }
+    __device__ double same(double as, const DivF& d) const { return note(TWO ? xdiv_scaled2(as, d) : xdiv_scaled(as, d)); }
+    __device__ double up(double a, const DivC& d) const { return note(TWO ? xdiv_up2(a, d) : xdiv_up(a, d)); }
     __device__ double plain(double a, const DivC& d) const { return __dmul_rn(up(a, d), 0x1p-128); }
     // a quotient that no trial value depends on: infinite and NaN are noted here
     __device__ double plain_checked(double a, const DivC& d) const {
@@ -206,12 +210,15 @@ struct DivExact {
     __device__ double etaK() const { return P.eta_K; }
 };
 // The policy of a march pass: 0 the reciprocal form; 1 the drop-in form's
-// first pass (exact quotients, out-of-range numerators flagged); 2 the drop-in
-// form's recomputation of a CTA whose first pass raised the flag.
+// first pass (exact quotients, out-of-range numerators flagged), 3 the same
+// where two operations divide by every run constant; 2 the drop-in form's
+// recomputation of a CTA whose first pass raised the flag.
 template <int DM> struct DivOf;
 template <> struct DivOf<0> { using T = Reciprocal; };
-template <> struct DivOf<1> { using T = DivRun; };
+template <> struct DivOf<1> { using T = DivRun<false>; };
 template <> struct DivOf<2> { using T = DivExact; };
+template <> struct DivOf<3> { using T = DivRun<true>; };
+template <int DM> constexpr bool kFirstPass = (DM & 1) != 0;
 // The error word a launch with parameters P reports its first failing trial to.
 __device__ __forceinline__ unsigned long long* err_word(const StepParams& P, Status* st) {
     return P.err_slot < 0 ? &st->err_key : &st->slot_err[P.err_slot];
@@ -698,7 +705,7 @@ struct StepKernel {
         return carry;
     }
     // One march over the CTA's chunk with the division policy of DM (DivOf).
-    // DM 1 returns true, without publishing its failure keys or budget
+    // A first pass returns true, without publishing its failure keys or budget
     // partials, when a numerator of the chunk left the guarded range.
     template <int DM>
     __device__ static bool run_body(const StepParams& P, const double* __restrict__ o, const double* __restrict__ cr,
@@ -728,7 +735,7 @@ struct StepKernel {
 
         SharedBook<T::NT> book(smem + T::SMEM_DOUBLES + T::SCRATCH_DOUBLES + ta * TB + tb);
 
-        unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+        unsigned low = kFirstPass<DM> && P.div_gate == 1 ? 0u : ~0u;
         const typename DivOf<DM>::T dv{P, low};
 
         auto slot3 = [](int w) { return ((w % 3) + 3) % 3; };
@@ -852,7 +859,7 @@ struct StepKernel {
             s2u = s2n;
         }
         const unsigned long long errkey = book.key();
-        if (DM == 1 && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
+        if (kFirstPass<DM> && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
         if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
         DD acc[5];
         long long clipped = book.clipped();
@@ -893,7 +900,8 @@ struct StepKernel {
         }
         if (FAST) {
             run_body<0>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
-        } else if (run_body<1>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin)) {
+        } else if (P.div_gate == 2 ? run_body<3>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin)
+                                   : run_body<1>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin)) {
             __syncthreads();
             run_body<2>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
         }
@@ -931,7 +939,7 @@ __device__ __forceinline__ unsigned eta_cell_pass(const StepParams& P, int neta,
                                          double* __restrict__ s2_next, int x, int row, int col,
                                          unsigned long long& errkey) {
     const Grid& g = P.g;
-    unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+    unsigned low = kFirstPass<DM> && P.div_gate == 1 ? 0u : ~0u;
     const typename DivOf<DM>::T dv{P, low};
     const long long idx = (long long)x * g.plane + (long long)row * g.pb + col;
     const long long cell = ((long long)x * g.na + row) * g.nb + col + P.cell_off;
@@ -960,7 +968,7 @@ __device__ __forceinline__ unsigned eta_cell_pass(const StepParams& P, int neta,
     if (!in_range) errkey = min(errkey, eta_fail_key(eta_next + idx, neta, g.nstore, P.key_ncells, cell));
     s2_next[idx] = Sn;
     gb_next[idx] = P.eta_scale * smin(1., 16. * pairs);
-    return DM == 1 && (low <= kLowQuotient || errkey != ERR_NONE);
+    return kFirstPass<DM> && (low <= kLowQuotient || errkey != ERR_NONE);
 }
 // The cell's eta update with the division policy of the form; in the drop-in
 // form a cell whose numerators left the exact-division range is recomputed
@@ -977,7 +985,8 @@ __device__ __forceinline__ void eta_cell(const StepParams& P, int neta, const do
         return;
     }
     unsigned long long k = ERR_NONE;
-    if (eta_cell_pass<DIM, 1>(P, neta, eta, s2, p, eta_next, gb_next, s2_next, x, row, col, k)) {
+    if (P.div_gate == 2 ? eta_cell_pass<DIM, 3>(P, neta, eta, s2, p, eta_next, gb_next, s2_next, x, row, col, k)
+                        : eta_cell_pass<DIM, 1>(P, neta, eta, s2, p, eta_next, gb_next, s2_next, x, row, col, k)) {
         k = ERR_NONE;
         eta_cell_pass<DIM, 2>(P, neta, eta, s2, p, eta_next, gb_next, s2_next, x, row, col, k);
     }
@@ -1014,14 +1023,14 @@ __global__ void __launch_bounds__(256, 5) k_eta_update(const StepParams P, int n
 // instances keep them compile-time (the runtime range cost this kernel's
 // schedule 85% at 128 registers).
 // One march of a thread's column with the division policy of DM (DivOf);
-// returns the flag of numerators outside the exact-division range (DM 1).
+// returns the flag of numerators outside the exact-division range (first pass).
 template <int DIM, int DM, int NCAP, bool SLAB>
 __device__ __forceinline__ unsigned eta_march_pass(const StepParams& P, int n, const double* __restrict__ eta,
                                                    const double* __restrict__ p, double* __restrict__ eta_next,
                                                    double* __restrict__ gb_next, double* __restrict__ s2_next,
                                                    int row, int col, int i0, int i1, unsigned long long& errkey) {
     const Grid& g = P.g;
-    unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+    unsigned low = kFirstPass<DM> && P.div_gate == 1 ? 0u : ~0u;
     const typename DivOf<DM>::T dv{P, low};
     const long long rc = (long long)row * g.pb + col;
     const long long cbm = (long long)row * g.pb + (col == 0 ? g.nb - 1 : col - 1);
@@ -1078,7 +1087,7 @@ __device__ __forceinline__ unsigned eta_march_pass(const StepParams& P, int n, c
         for (int q = 0; q < NCAP; ++q)
             if (q < n) { ep[q] = ec[q]; ec[q] = en[q]; }
     }
-    return DM == 1 && (low <= kLowQuotient || errkey != ERR_NONE);
+    return kFirstPass<DM> && (low <= kLowQuotient || errkey != ERR_NONE);
 }
 
 // X-marching form of the eta update for a compile-time number of fields N:
@@ -1108,8 +1117,10 @@ __device__ __forceinline__ void eta_march_body(const StepParams& P, int n, const
     unsigned long long errkey = ERR_NONE;
     if (FAST) {
         eta_march_pass<DIM, 0, NCAP, SLAB>(P, n, eta, p, eta_next, gb_next, s2_next, row, col, i0, i1, errkey);
-    } else if (eta_march_pass<DIM, 1, NCAP, SLAB>(P, n, eta, p, eta_next, gb_next, s2_next, row, col, i0, i1,
-                                                   errkey)) {
+    } else if (P.div_gate == 2 ? eta_march_pass<DIM, 3, NCAP, SLAB>(P, n, eta, p, eta_next, gb_next, s2_next, row, col,
+                                                                    i0, i1, errkey)
+                               : eta_march_pass<DIM, 1, NCAP, SLAB>(P, n, eta, p, eta_next, gb_next, s2_next, row, col,
+                                                                    i0, i1, errkey)) {
         errkey = ERR_NONE;
         eta_march_pass<DIM, 2, NCAP, SLAB>(P, n, eta, p, eta_next, gb_next, s2_next, row, col, i0, i1, errkey);
     }

@@ -57,11 +57,11 @@ struct Steps2D {
     };
 
     // Lead points and cells of one step with the division policy of DM (DivOf);
-    // true (DM 1): the tile must be computed again with exact divisions.
+    // true (first pass): the tile must be computed again with exact divisions.
     template <int DM>
     __device__ static bool step_tile(const StepParams& P, const Steps2DArgs& A, Smem& s, int par, int gpar, int epar,
                                      double gbv, double o_raw, double s2u, int x0, int col, CellBook& book) {
-        unsigned low = DM == 1 && P.div_gate ? 0u : ~0u;
+        unsigned low = kFirstPass<DM> && P.div_gate == 1 ? 0u : ~0u;
         const typename DivOf<DM>::T dv{P, low};
         const Grid& g = P.g;
         const int tid = threadIdx.x;
@@ -134,7 +134,7 @@ struct Steps2D {
                 A.gb[gpar ^ 1][idx] = P.eta_scale * smin(1., 16. * pairs);
             }
         }
-        return DM == 1 && __syncthreads_or(low <= kLowQuotient || book.k != ERR_NONE);
+        return kFirstPass<DM> && __syncthreads_or(low <= kLowQuotient || book.k != ERR_NONE);
     }
     __device__ static double gb_own(const Steps2DArgs& A, int gpar, long long idx) { return __ldcg(A.gb[gpar] + idx); }
 
@@ -202,7 +202,8 @@ struct Steps2D {
             __syncthreads();
             if (FAST) {
                 step_tile<0>(P, A, s, par, gpar, epar, gbv, o_raw, s2u, x0, col, book);
-            } else if (step_tile<1>(P, A, s, par, gpar, epar, gbv, o_raw, s2u, x0, col, book)) {
+            } else if (P.div_gate == 2 ? step_tile<3>(P, A, s, par, gpar, epar, gbv, o_raw, s2u, x0, col, book)
+                                       : step_tile<1>(P, A, s, par, gpar, epar, gbv, o_raw, s2u, x0, col, book)) {
                 step_tile<2>(P, A, s, par, gpar, epar, gbv, o_raw, s2u, x0, col, book);
             }
             if (book.k != ERR_NONE) atomicMin(&st->slot_err[n & 1], book.k);
