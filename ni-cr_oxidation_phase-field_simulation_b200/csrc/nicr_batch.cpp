@@ -128,7 +128,7 @@ struct nicr_batch {
         };
         int best = doms[0]->m->params().xchunk;
         float best_ms = -1.f;
-        for (int c : nicr::xchunk_candidates(nxmax)) {
+        for (int c : nicr::xchunk_candidates(nxmax, best)) {
             for (auto* h : doms) h->m->set_xchunk(c);
             pass();
             nicr::check_cuda(cudaEventRecord(e0, stream), "cudaEventRecord");

@@ -197,9 +197,9 @@ int choose_xchunk(const Grid& g);
 // The same choice for the one-pass step (16 x 32 tiles, one CTA per SM).
 int choose_xchunk_fused(const Grid& g);
 int choose_xchunk_batch(const Grid* grids, int n);
-// The chunks the choosers consider for a largest X extent nxmax: nxmax halved
-// repeatedly and the powers of two below it, longest first.
-std::vector<int> xchunk_candidates(int nxmax);
+// The chunks a measured choice tries for a largest X extent nxmax: nxmax halved
+// repeatedly, the powers of two below it and the chunk in use, longest first.
+std::vector<int> xchunk_candidates(int nxmax, int in_use);
 // Per-device kernel attributes of the step kernel P selects, set outside any
 // stream capture (launch_step_main sets them on first use otherwise).
 void step_kernels_prepare(const StepParams& P);

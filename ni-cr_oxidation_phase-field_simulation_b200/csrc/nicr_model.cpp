@@ -835,7 +835,7 @@ void Model::tune(int reps, int* xchunk, int* minb) {
     int best_c = sp.xchunk, best_m = sp.minb;
     float best_ms = -1.f;
     const std::vector<int> minbs = dim == 3 ? std::vector<int>{2, 3} : std::vector<int>{0};
-    for (int c : xchunk_candidates(g.nx)) {
+    for (int c : xchunk_candidates(g.nx, sp.xchunk)) {
         set_xchunk(c);
         for (int mb : minbs) {
             sp.minb = mb;

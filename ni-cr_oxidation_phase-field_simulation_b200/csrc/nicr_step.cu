@@ -306,23 +306,33 @@ int choose_xchunk(const Grid& g) {
     return choose_xchunk_batch(&g, 1);
 }
 
-int choose_xchunk_fused(const Grid& g) {
-    if (forced_xchunk() > 0) return std::min(forced_xchunk(), g.nx);
-    const long long tiles = (long long)(g.na / FTA) * (g.nb / FTB), slots = 148;
-    int best = g.nx;
+// Waves of CTAs times the planes of a chunk and its overhead in planes (the
+// lead planes of its start, the first loads, the final reduction), least over
+// the even splits of nxmax planes. `ctas` counts a launch's CTAs for a chunk.
+namespace {
+template <class Ctas>
+int least_cost_chunk(int nxmax, long long slots, int overhead, Ctas ctas) {
+    int best = nxmax;
     long long best_cost = -1;
-    for (int c : xchunk_candidates(g.nx)) {
-        const long long ctas = tiles * ((g.nx + c - 1) / c);
-        const long long cost = ((ctas + slots - 1) / slots) * (c + 2);
+    for (int parts = 1; parts <= nxmax; ++parts) {
+        const int c = (nxmax + parts - 1) / parts;
+        const long long cost = ((ctas(c) + slots - 1) / slots) * (c + overhead);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = c; }
     }
     return best;
 }
+}  // namespace
 
-// One chunk for all domains of a batch: the same cost with the CTAs of every
-// domain sharing the waves (chunks above a domain's nx clamp to it).
-std::vector<int> xchunk_candidates(int nxmax) {
-    std::vector<int> cand;
+// 256^3 with 8 fields (128 tiles): 32 planes 1740 us per two steps, 29 1757, 128
+// 1809, 256 1862, 43 1890.
+int choose_xchunk_fused(const Grid& g) {
+    if (forced_xchunk() > 0) return std::min(forced_xchunk(), g.nx);
+    const long long tiles = (long long)(g.na / FTA) * (g.nb / FTB);
+    return least_cost_chunk(g.nx, 148, 2, [&](int c) { return tiles * ((g.nx + c - 1) / c); });
+}
+
+std::vector<int> xchunk_candidates(int nxmax, int in_use) {
+    std::vector<int> cand{std::min(in_use, nxmax)};
     for (int c = nxmax;; c = (c + 1) / 2) {
         cand.push_back(c);
         if (c == 1) break;
@@ -333,6 +343,13 @@ std::vector<int> xchunk_candidates(int nxmax) {
     return cand;
 }
 
+// One chunk for all domains of a batch: the CTAs of every domain share the
+// waves (chunks above a domain's nx clamp to it). In 3D a chunk costs 13 us and
+// 2.8 us per plane with two CTAs on an SM (64^3), an overhead of 5 planes, and
+// even splits matter where few chunks fill the GPU once: against halvings of nx
+// with an overhead of 2 planes, 97 x 61 x 75 415 -> 368 us per six steps (13 ->
+// 9 planes), 151 x 101 x 101 928 -> 899 us per ten (38 -> 31), a 20-domain
+// sweep of 32..96 edges 1988 -> 1871 us per ten (12 -> 16).
 int choose_xchunk_batch(const Grid* grids, int n) {
     int nxmax = 1;
     bool any3 = false;
@@ -341,17 +358,11 @@ int choose_xchunk_batch(const Grid* grids, int n) {
         any3 = any3 || grids[d].dim == 3;
     }
     if (forced_xchunk() > 0) return std::min(forced_xchunk(), nxmax);
-    const long long slots = 148LL * (any3 ? 2 : 4);
-    const std::vector<int> cand = xchunk_candidates(nxmax);
-    int best = nxmax;
-    long long best_cost = -1;
-    for (int c : cand) {
+    return least_cost_chunk(nxmax, 148LL * (any3 ? 2 : 4), any3 ? 5 : 2, [&](int c) {
         long long ctas = 0;
         for (int d = 0; d < n; ++d) ctas += step_tiles(grids[d]) * ((grids[d].nx + c - 1) / c);
-        const long long cost = ((ctas + slots - 1) / slots) * (c + 2);
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = c; }
-    }
-    return best;
+        return ctas;
+    });
 }
 
 int step_main_blocks(const StepParams& P) {

@@ -265,12 +265,13 @@ struct OnePassStep {
         double pP, FxO, FxCr;   // phi of plane u-1 (own point), left x-face fluxes of plane u
         double s2u, gbu;          // S and gb of the own point of the update plane
         double ep[N];             // own column of eta at plane u - 1
-        // ---- prologue: centre values of the first update plane and its left x-face flux
+        // ---- prologue: centre values of the first update plane and its left
+        // x-face flux; all planes it reads are requested at once
+        SK::load_oc(P, o, cr, i0 - 1, oslot(i0 - 1), cslot(i0 - 1), offs);
+        SK::load_oc(P, o, cr, i0, oslot(i0), cslot(i0), offs);
+        SK::load_oc(P, o, cr, i0 + 1, oslot(i0 + 1), cslot(i0 + 1), offs);
+        SK::load_p(P, p, i0, pslot(i0), offs);
         if (i0 == 0) {
-            SK::load_oc(P, o, cr, -1, oslot(-1), cslot(-1), offs);
-            SK::load_oc(P, o, cr, 0, oslot(0), cslot(0), offs);
-            SK::load_oc(P, o, cr, 1, oslot(1), cslot(1), offs);
-            SK::load_p(P, p, 0, pslot(0), offs);
             wait(-1);
             wait(0);
             __syncthreads();
@@ -287,17 +288,12 @@ struct OnePassStep {
             if (P.inlet) book.add(4, P.layer_o - __ldg(o + (long long)row * g.pb + col));
         } else {
             SK::load_oc(P, o, cr, i0 - 2, oslot(i0 - 2), cslot(i0 - 2), offs);
-            SK::load_oc(P, o, cr, i0 - 1, oslot(i0 - 1), cslot(i0 - 1), offs);
-            SK::load_oc(P, o, cr, i0, oslot(i0), cslot(i0), offs);
             SK::load_p(P, p, i0 - 1, pslot(i0 - 1), offs);
             wait(i0 - 1);
+            wait(i0);
             __syncthreads();
             double Sm, gbm;
             const CenterVals Pv = lead(i0 - 1, Sm, gbm);
-            SK::load_oc(P, o, cr, i0 + 1, oslot(i0 + 1), cslot(i0 + 1), offs);
-            SK::load_p(P, p, i0, pslot(i0), offs);
-            wait(i0);
-            __syncthreads();
             const CenterVals C = lead(i0, s2u, gbu);
             __syncthreads();
             FxO = SK::face_x(dv, Pv.mo, C.mo, Pv.muO, C.muO);

@@ -68,22 +68,34 @@ __device__ void block_reduce_dd(DD (&v)[N], long long& cnt, DD* sdd, long long* 
         scnt[w] = any ? cnt : -1;   // -1: nothing from this warp
     }
     __syncthreads();
-    if (tid == 0) {
-        for (int q = 0; q < N; ++q) v[q] = DD{0., 0.};
-        cnt = 0;
-        for (int ww = 0; ww < nw; ++ww) {
-            if (scnt[ww] < 0) continue;
-            for (int q = 0; q < N; ++q) v[q] = dd_add(v[q], sdd[ww * N + q]);
-            cnt += scnt[ww];
+    if (w == 0) {   // the warps' values by one warp: 3 dependent additions for 8 warps instead of 8
+        const bool has = lane < nw && scnt[lane] >= 0;
+        for (int q = 0; q < N; ++q) v[q] = has ? sdd[lane * N + q] : DD{0., 0.};
+        cnt = has ? scnt[lane] : 0;
+        int off = 16;
+        while (off >= nw) off >>= 1;
+        for (; off > 0; off >>= 1) {
+            for (int q = 0; q < N; ++q) v[q] = dd_add(v[q], shfl_dd(v[q], off));
+            cnt += __shfl_down_sync(0xffffffffu, cnt, off);
         }
     }
 }
 
 // Whether this step must not run: a step of this batch was rejected, or the
-// previous one just was (its commit has not run yet).
-__device__ __forceinline__ bool step_blocked(const StepParams& P, const Status* st) {
-    return st->failed || (!P.slab && P.err_slot >= 0 && st->slot_err[P.err_slot ^ 1] != ERR_NONE);
-}
+// previous one just was (its commit has not run yet, or runs beside this step).
+// The words are read where a Blocked is made and waited for where it is tested,
+// so a kernel can stage its first planes meanwhile.
+struct Blocked {
+    int failed;
+    unsigned long long key;
+    __device__ __forceinline__ Blocked(const StepParams& P, const Status* st)
+        : failed(*(const volatile int*)&st->failed),
+          key(!P.slab && P.err_slot >= 0 ? *(const volatile unsigned long long*)&st->slot_err[P.err_slot ^ 1] : ERR_NONE) {}
+    __device__ __forceinline__ explicit operator bool() const { return failed != 0 || key != ERR_NONE; }
+};
+__device__ __forceinline__ bool step_blocked(const StepParams& P, const Status* st) { return (bool)Blocked(P, st); }
+// What a march pass leaves.
+enum MarchEnd { kMarched, kMarchAgain, kMarchBlocked };
 
 // Commits the pending step of parity q, if any, by one CTA: partial sums
 // (thread t: partials t, t + nthreads, ...; deterministic), then the budget is
@@ -705,10 +717,11 @@ struct StepKernel {
         return carry;
     }
     // One march over the CTA's chunk with the division policy of DM (DivOf).
-    // A first pass returns true, without publishing its failure keys or budget
-    // partials, when a numerator of the chunk left the guarded range.
+    // A first pass returns kMarchAgain, without publishing its failure keys or
+    // budget partials, when a numerator of the chunk left the guarded range;
+    // kMarchBlocked when the step must not run (nothing written).
     template <int DM>
-    __device__ static bool run_body(const StepParams& P, const double* __restrict__ o, const double* __restrict__ cr,
+    __device__ static MarchEnd run_body(const StepParams& P, const double* __restrict__ o, const double* __restrict__ cr,
                                     const double* __restrict__ p, const double* __restrict__ gb,
                                     const double* __restrict__ s2, double* __restrict__ on,
                                     double* __restrict__ crn, double* __restrict__ pn,
@@ -731,6 +744,7 @@ struct StepKernel {
         const int i1 = min(SLAB ? P.x_hi : g.nx, i0 + P.xchunk);
         const int row = a0 + ta, col = b0 + tb;
         const bool active = (DIM == 3 ? row < g.na : true) && col < g.nb;
+        const Blocked blocked(P, st);
         const Offs offs = make_offs(g, a0, b0);
 
         SharedBook<T::NT> book(smem + T::SMEM_DOUBLES + T::SCRATCH_DOUBLES + ta * TB + tb);
@@ -770,15 +784,23 @@ struct StepKernel {
 
         CenterVals C, L;
         double pP, FxO, FxCr;
-        // ---- prologue: centre values of the first update plane and its left x-face flux
+        // ---- prologue: centre values of the first update plane and its left
+        // x-face flux. All planes it reads are requested at once, the march's
+        // first prefetch and the words of an earlier rejection with them: a round
+        // trip each was waited for before (64^3, 4 planes per chunk: 511 -> 491 us
+        // per twenty steps; a 20-domain sweep 2562 -> 2433 us per ten)
+        double gb0[2];
+        load_oc(P, o, cr, i0 - 1, oslot(i0 - 1), cslot(i0 - 1), offs);
+        load_oc(P, o, cr, i0, oslot(i0), cslot(i0), offs);
+        load_oc(P, o, cr, i0 + 1, oslot(i0 + 1), cslot(i0 + 1), offs);
+        load_p(P, p, i0, pslot(i0), offs);
+        fetch_gb(P, gb, i0, offs, gb0);
+        double s2u = (P.phi_eta && active) ? __ldg(s2 + (long long)i0 * g.plane + offs.gl[0]) : 0.;
+        Prefetch pf;
         if (i0 == 0) {
-            load_oc(P, o, cr, -1, oslot(-1), cslot(-1), offs);
-            load_oc(P, o, cr, 0, oslot(0), cslot(0), offs);
-            load_oc(P, o, cr, 1, oslot(1), cslot(1), offs);
-            load_p(P, p, 0, pslot(0), offs);
-            double gb0[2];
-            fetch_gb(P, gb, 0, offs, gb0);
+            if (i0 + 1 <= g.nx - 1) fetch(P, o, cr, p, gb, s2, i0 + 2, i0 + 1, i0 + 1, active, offs, pf);
             __syncthreads();
+            if (blocked) return kMarchBlocked;
             C = lead(0, gb0);
             __syncthreads();
             // ghost plane -1: copies of plane 0 (3S:187, 3S:613-615, 3S:616-619)
@@ -788,18 +810,13 @@ struct StepKernel {
             pP = C.p;
         } else {
             load_oc(P, o, cr, i0 - 2, oslot(i0 - 2), cslot(i0 - 2), offs);
-            load_oc(P, o, cr, i0 - 1, oslot(i0 - 1), cslot(i0 - 1), offs);
-            load_oc(P, o, cr, i0, oslot(i0), cslot(i0), offs);
             load_p(P, p, i0 - 1, pslot(i0 - 1), offs);
             double gbm[2];
             fetch_gb(P, gb, i0 - 1, offs, gbm);
+            if (i0 + 1 <= g.nx - 1) fetch(P, o, cr, p, gb, s2, i0 + 2, i0 + 1, i0 + 1, active, offs, pf);
             __syncthreads();
+            if (blocked) return kMarchBlocked;
             const CenterVals Pv = lead(i0 - 1, gbm);
-            load_oc(P, o, cr, i0 + 1, oslot(i0 + 1), cslot(i0 + 1), offs);
-            load_p(P, p, i0, pslot(i0), offs);
-            double gb0[2];
-            fetch_gb(P, gb, i0, offs, gb0);
-            __syncthreads();
             C = lead(i0, gb0);
             __syncthreads();
             FxO = face_x(dv, Pv.mo, C.mo, Pv.muO, C.muO);
@@ -807,9 +824,6 @@ struct StepKernel {
             pP = Pv.p;
         }
 
-        double s2u = (P.phi_eta && active) ? __ldg(s2 + (long long)i0 * g.plane + offs.gl[0]) : 0.;
-        Prefetch pf;
-        if (i0 + 1 <= g.nx - 1) fetch(P, o, cr, p, gb, s2, i0 + 2, i0 + 1, i0 + 1, active, offs, pf);
         for (int u = i0; u < i1; ++u) {
             const int x = u + 1;
             double s2n = 0.;
@@ -859,7 +873,7 @@ struct StepKernel {
             s2u = s2n;
         }
         const unsigned long long errkey = book.key();
-        if (kFirstPass<DM> && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return true;
+        if (kFirstPass<DM> && __syncthreads_or(low <= kLowQuotient || errkey != ERR_NONE)) return kMarchAgain;
         if (errkey != ERR_NONE) atomicMin(err_word(P, st), errkey);
         DD acc[5];
         long long clipped = book.clipped();
@@ -870,7 +884,7 @@ struct StepKernel {
             for (int q = 0; q < 5; ++q) { out.s[q][0] = acc[q].hi; out.s[q][1] = acc[q].lo; }
             out.clipped = clipped;
         }
-        return false;
+        return kMarched;
     }
 
     // One CTA's chunk of a step of nblocks CTAs (this one at blin); with a
@@ -893,18 +907,20 @@ struct StepKernel {
                 commit_pending(prev, P.err_slot ^ 1, budget, st, sdd, reinterpret_cast<long long*>(sdd + 32 * 5));
                 return;
             }
-            if (step_blocked(P, st)) return;
-            if (blin == 0 && threadIdx.x == 0 && threadIdx.y == 0) st->pending[P.err_slot] = nblocks;
-        } else if (st->failed) {
-            return;
         }
+        MarchEnd end;
         if (FAST) {
-            run_body<0>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
-        } else if (P.div_gate == 2 ? run_body<3>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin)
-                                   : run_body<1>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin)) {
-            __syncthreads();
-            run_body<2>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
+            end = run_body<0>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
+        } else {
+            end = P.div_gate == 2 ? run_body<3>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin)
+                                  : run_body<1>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
+            if (end == kMarchAgain) {
+                __syncthreads();
+                run_body<2>(P, o, cr, p, gb, s2, on, crn, pn, partials, st, bx, by, bz, blin);
+            }
         }
+        if (!SLAB && budget && end != kMarchBlocked && blin == 0 && threadIdx.x == 0 && threadIdx.y == 0)
+            st->pending[P.err_slot] = nblocks;
     }
 };
 
