@@ -496,8 +496,10 @@ struct StepKernel {
             v.muO = fma(-2. * Phys::ko, lapO, fma(hh, bo, (1. - hh) * ao));
             v.muCr = fma(-2. * Phys::kc, lapC, fma(hh, bc, (1. - hh) * ac));
             const double mbo = fma(f.gbo, gbv, Phys::bmo), mbc = fma(f.gbc, gbv, Phys::bmc);
-            v.mo = o_on ? oc * fma(hh, Phys::boo - mbo, mbo) : 0.;
-            v.mc = cc * fma(hh, Phys::boc - mbc, mbc);
+            // not mbo + h (boo - mbo): in oxide (h = 1) that would leave boo with
+            // the rounding of the GB-enhanced mbo, up to 1e4 times larger
+            v.mo = o_on ? oc * fma(hh, Phys::boo, (1. - hh) * mbo) : 0.;
+            v.mc = cc * fma(hh, Phys::boc, (1. - hh) * mbc);
         } else {
             double lapO, lapC;
             const DivSet& d = k.div;
