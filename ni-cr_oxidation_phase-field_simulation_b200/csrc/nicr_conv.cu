@@ -1043,10 +1043,12 @@ __global__ void __launch_bounds__(SH_THREADS) k_conv3d_fwd_shift(const __grid_co
     const int N = cout;
     const int boxes = C.order ? 1 : C.chunks;   // channel boxes per line
     struct Item {
-        int x0, y0, z, b, dz0, ndz, planes;
+        int x0, y0, z, b;
     };
-    // item i; planes in accumulation order: planes outside the grid hold
-    // zeros, which leave a sum as it is, and are skipped (dz = 0 is inside)
+    // A plane is a dz, or a channel chunk and a dz. Planes outside the grid
+    // (zero fill) take part, as in the forms before: their products carry an
+    // infinite or NaN weight into the sums.
+    const int planes = C.order ? 3 * C.chunks : 3;
     auto item = [&](int i) {
         Item m;
         m.x0 = i % C.tiles_x * TC_M;
@@ -1055,9 +1057,6 @@ __global__ void __launch_bounds__(SH_THREADS) k_conv3d_fwd_shift(const __grid_co
         i /= C.groups_y;
         m.z = i % V.d;
         m.b = i / V.d;
-        m.dz0 = m.z > 0 ? -1 : 0;
-        m.ndz = (m.z < V.d - 1 ? 1 : 0) - m.dz0 + 1;
-        m.planes = C.order ? C.chunks * m.ndz : m.ndz;
         return m;
     };
 
@@ -1076,8 +1075,8 @@ __global__ void __launch_bounds__(SH_THREADS) k_conv3d_fwd_shift(const __grid_co
             };
             for (int i = blockIdx.x; i < C.items && ok; i += gridDim.x) {
                 const Item m = item(i);
-                for (int p = 0; p < m.planes && ok; ++p) {
-                    const int dz = m.dz0 + p % m.ndz, c0 = C.order ? p / m.ndz * C.kc : 0;
+                for (int p = 0; p < planes && ok; ++p) {
+                    const int dz = p % 3 - 1, c0 = p / 3 * C.kc;
                     for (int r = 0, dy = 0; dy < 3 && ok; ++dy, ++step) {
                         // the lines step (p, dy) adds: 0 .. T-1, then one per step
                         for (; r < T + dy && ok; ++r) {
@@ -1113,12 +1112,11 @@ __global__ void __launch_bounds__(SH_THREADS) k_conv3d_fwd_shift(const __grid_co
         bool ok = true;
         int step = 0, l0 = 0, seen = 0, n = 0;   // steps, the plane's first line, lines seen, items
         for (int i = blockIdx.x; i < C.items && ok; i += gridDim.x, ++n) {
-            const Item m = item(i);
             const uint32_t d0 = tmem + (uint32_t)((n & 1) * T * N);
             // the accumulators' last item must have been stored
             if (n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_empty + (n & 1)), (uint32_t)((n / 2 - 1) & 1)));
             uint32_t fresh = 1;
-            for (int p = 0; p < m.planes && ok; ++p, l0 += T + 2)
+            for (int p = 0; p < planes && ok; ++p, l0 += T + 2)
                 for (int dy = 0; dy < 3 && ok; ++dy, ++step) {
                     ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bfull + step % C.nb), (uint32_t)((step / C.nb) & 1)));
                     for (; seen < l0 + T + dy && ok; ++seen)

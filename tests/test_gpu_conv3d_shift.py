@@ -58,3 +58,16 @@ def test_refuses_what_it_cannot_hold(require_gpu, shape):
     x, w = inputs(shape, 3)
     with pytest.raises(RuntimeError):
         surrogate.conv3d_raw(x, w, "shift")
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 5, 128, 32, 32), (1, 1, 4, 128, 48, 16), (1, 3, 4, 64, 64, 64)])
+@pytest.mark.parametrize("tap", [1, 13, 25])   # planes below, at and above the voxel
+def test_infinite_weights_reach_the_same_voxels(require_gpu, shape, tap):
+    """An infinite weight times the zero padding is NaN, in planes outside the grid as elsewhere."""
+    x, w = inputs(shape, 4)
+    w[3, tap, 5] = float("inf")
+    n, d, h, wd, ci, co = shape
+    a = surrogate.conv3d_raw(x, w, "shift")
+    b = surrogate.conv3d_raw(x, w, "halo" if co <= 32 and ci * co <= 768 and wd >= 128 else "tma")
+    assert torch.equal(torch.isnan(a), torch.isnan(b))
+    assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))
