@@ -277,8 +277,10 @@ def _module_classes():
         return eager(x) and x.dtype == torch.bfloat16 and x.is_contiguous()
 
     def eager(x):
-        """No gradients and no trace to be recorded: a trace would hold a pass of the library as a constant."""
-        return not torch.is_grad_enabled() and x.is_cuda and not torch.jit.is_tracing()
+        """No gradients, no trace and no forward-mode tangent to be recorded: a trace would hold a pass of the
+        library as a constant, and a pass would drop the tangent, which the convolutions refuse."""
+        return (not torch.is_grad_enabled() and x.is_cuda and not torch.jit.is_tracing()
+                and torch.autograd.forward_ad.unpack_dual(x).tangent is None)
 
     class UNet3d(nn.Module):
         """3 levels, `base` channels at full resolution (x2 per level)."""

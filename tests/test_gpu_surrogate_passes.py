@@ -94,3 +94,12 @@ def test_act_backward_of_other_layouts(require_gpu, y):
     ref = gy if act is None else gy * (act > 0)
     assert torch.equal(got, ref.to(torch.bfloat16))
     assert bool(((gb - ref.sum((0, 1))).abs() <= 2e-6 * ref.abs().sum((0, 1))).all())
+
+
+def test_forward_mode_stays_refused(require_gpu):
+    """The convolutions have no forward-mode rule; the passes around them must not drop the tangent."""
+    net = surrogate.unet(5, 16).cuda()
+    x = torch.randn((1, 4, 4, 8, 5), device="cuda")
+    with torch.no_grad(), torch.autograd.forward_ad.dual_level():
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            net(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)))
