@@ -1142,6 +1142,8 @@ void Model::launch_step_group(int n) {
     }
     check_cuda(cudaGraphLaunch(pg->exec, stream), "cudaGraphLaunch");
     launches += pg->kernels;
+    // replayed steps write neither gb nor eta_s2 (enqueue_step says so only when it captures)
+    if (onepass_step()) eta_dirty = true;
 }
 
 // The longest captured run (16, 8, 4 or 2 steps) that starts at step s of
