@@ -111,6 +111,7 @@ struct nicr_batch {
         int nxmax = 1;
         for (auto* h : doms) {
             h->m->prepare_step();
+            h->m->clear_status();   // an earlier rejection must not stop the trial launches
             nxmax = std::max(nxmax, h->m->g.nx);
         }
         std::vector<nicr::BatchDomain> descs((size_t)n);
@@ -142,7 +143,10 @@ struct nicr_batch {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         nicr::check_cuda(cudaGetLastError(), "tune");
-        for (auto* h : doms) h->m->set_xchunk(best);
+        for (auto* h : doms) {
+            h->m->set_xchunk(best);
+            h->m->clear_status();   // what the trial launches of a failing state left in the error words
+        }
         for (auto& q : graphs)
             if (q.exec) cudaGraphExecDestroy(q.exec);
         graphs.clear();

@@ -796,6 +796,11 @@ void Model::reset_status() {
     check_cuda(cudaMemcpyAsync(st, h_st, sizeof(Status), cudaMemcpyHostToDevice, stream), "H2D");
 }
 
+void Model::clear_status() {
+    status_clean = false;
+    reset_status();
+}
+
 void Model::set_xchunk(int c) {
     sync();
     sp.xchunk = std::max(1, std::min(c, g.nx));
@@ -827,8 +832,7 @@ void Model::launch_trial_kernels() {
 void Model::tune(int reps, int* xchunk, int* minb) {
     reps = std::max(1, reps);
     if (!onepass_step()) prepare_step();
-    status_clean = false;   // trial launches use the error word
-    reset_status();   // trial kernels of a failing state must not stop the timing runs
+    clear_status();   // an earlier rejection must not stop the trial launches
     cudaEvent_t e0, e1;
     check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
     check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
@@ -856,7 +860,7 @@ void Model::tune(int reps, int* xchunk, int* minb) {
     check_cuda(cudaGetLastError(), "tune");
     set_xchunk(best_c);   // also drops captured step graphs
     sp.minb = best_m;
-    reset_status();
+    clear_status();   // what the trial launches of a failing state left
     sync();
     if (xchunk) *xchunk = best_c;
     if (minb) *minb = best_m;

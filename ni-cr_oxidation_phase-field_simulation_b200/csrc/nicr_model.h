@@ -126,6 +126,9 @@ public:
     // Planes per CTA of this domain's step and eta kernels (a batch sets one
     // chunk for all its domains). Grows the partial-sum buffer when needed.
     void set_xchunk(int c);
+    // The status word sent again whatever an accepted run left: trial launches
+    // report failing trials to the error words that the next run reads.
+    void clear_status();
     // Times `reps` launches of this domain's step (and eta update) kernels for
     // each X chunk candidate and, in 3D, each occupancy variant, on the current
     // state without committing anything, and keeps the fastest pair.
