@@ -34,7 +34,10 @@ struct nicr_batch {
 
     // Step pairs of the whole batch captured as CUDA graphs, one per parity
     // state of all domains (they toggle together; a domain that was rolled
-    // back after a failed trial may differ), replayed when no domain scans
+    // back after a failed trial may differ) and launch form (a domain tuned by
+    // its own handle has another grid, and may have other partials: a graph
+    // that carried the old ones would write to freed memory, and the call's
+    // last commit would read what it never wrote), replayed when no domain scans
     // for Ksp in either step. Each graph holds the grouped step launches, the
     // domains' eta updates and the batched commit of two steps.
     struct PairGraph {
@@ -59,10 +62,11 @@ struct nicr_batch {
 
     void launch_pair(std::vector<nicr::BatchDomain>& descs) {
         const int n = (int)doms.size();
-        std::vector<int> key((size_t)n);
+        std::vector<int> key((size_t)2 * n);
         for (int i = 0; i < n; ++i) {
             doms[i]->m->prepare_step();   // stale eta masks are rebuilt outside the graph
-            key[i] = doms[i]->m->parity_key();
+            key[2 * i] = doms[i]->m->parity_key();
+            key[2 * i + 1] = doms[i]->m->launch_form();
         }
         PairGraph* pg = nullptr;
         for (auto& q : graphs)

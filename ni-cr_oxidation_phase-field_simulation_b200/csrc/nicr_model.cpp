@@ -811,6 +811,7 @@ void Model::set_xchunk(int c) {
         partial_cap = need;
         partials = dalloc_t<StepPartial>((size_t)2 * partial_cap);
     }
+    ++launch_form_;
     for (auto& q : pair_graphs)   // captured launches carry the old grid
         if (q.exec) { cudaGraphExecDestroy(q.exec); q.exec = nullptr; }
 }
@@ -858,8 +859,8 @@ void Model::tune(int reps, int* xchunk, int* minb) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     check_cuda(cudaGetLastError(), "tune");
-    set_xchunk(best_c);   // also drops captured step graphs
     sp.minb = best_m;
+    set_xchunk(best_c);   // also drops captured step graphs, a batch's through launch_form
     clear_status();   // what the trial launches of a failing state left
     sync();
     if (xchunk) *xchunk = best_c;

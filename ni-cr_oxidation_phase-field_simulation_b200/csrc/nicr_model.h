@@ -152,6 +152,9 @@ public:
     bool graphs_enabled() const;
     bool ksp_due(const RunPlan& r, int s) const;
     int parity_key() const { return cur | (ecur << 1) | (gcur << 2); }
+    // counts the changes of what launches carry besides the parities (X chunk,
+    // kernel variant, partials): a captured launch serves its own count only
+    int launch_form() const { return launch_form_; }
     void run_begin(RunPlan& r, int nsteps, bool schedule);
     void run_pre_step(RunPlan& r, int s);
     int run_end(RunPlan& r, int* completed, bool flush = true);   // flush: commit the last step first
@@ -240,6 +243,7 @@ private:
     bool eta_dirty = true;
     // reductions / status
     StepPartial* partials = nullptr;
+    int launch_form_ = 0;
     int partial_cap = 0;
     Status* st = nullptr;
     DevBudget* bud = nullptr;
