@@ -120,9 +120,10 @@ def _act_backward(gy, y):
     gy = gy.contiguous()
     c = gy.shape[-1]
     # torch's operations serve what the kernel cannot: host tensors, a gradient
-    # of this gradient, activations that a saved-tensor hook has handed back
-    # in another layout
+    # of this gradient, a forward-mode tangent of it (the bias gradient's), and
+    # activations that a saved-tensor hook has handed back in another layout
     if (gy.is_cuda and gy.dtype in (torch.bfloat16, torch.float32) and not torch.is_grad_enabled()
+            and torch.autograd.forward_ad.unpack_dual(gy).tangent is None
             and (y is None or (y.device == gy.device and y.shape == gy.shape and y.is_contiguous()
                                and y.dtype in (torch.bfloat16, torch.float32)))):
         L = _lib()
