@@ -1164,14 +1164,22 @@ int Model::group_length(const RunPlan& r, int s, int nsteps) const {
     return 1;
 }
 
+// The tile of the many-step launch and its CTAs, 0 when this handle's steps are
+// launched one by one: a domain other than 2D, too large for resident tiles, a
+// refused cooperative launch, or profiling (one event pair per kernel launch).
+int Model::steps2d_form(int* ctas) const {
+    if (dim != 2 || is_slab || prof_on || steps2d_failed) return 0;
+    const int tx = steps2d_tile(g, ctas);
+    return tx && *ctas <= partial_cap ? tx : 0;
+}
+
 // n steps (no Ksp scan due after the first) of a 2D domain that fits the
 // resident tiles, in launches of up to kSteps2DMost; false when it does not
-// apply. Not used while profiling (one event pair per kernel launch).
+// apply.
 bool Model::enqueue_steps2d(int n) {
-    if (dim != 2 || is_slab || prof_on || steps2d_failed) return false;
     int ctas = 0;
-    const int tx = steps2d_tile(g, &ctas);
-    if (!tx || ctas > partial_cap) return false;
+    const int tx = steps2d_form(&ctas);
+    if (!tx) return false;
     prepare_step();
     Steps2DArgs A{};
     for (int q = 0; q < 2; ++q) {
@@ -1232,8 +1240,10 @@ int Model::run(int nsteps, int* completed) {
     bool stepwise = false;   // the last step's commit is pending
     for (int s = 0; s < nsteps;) {
         run_pre_step(r, s);
-        int g = free_steps(r, s, nsteps);
-        if (!enqueue_steps2d(g)) {
+        // the look ahead to the next scan only where it is used: before each
+        // group of at most 16 steps it made a call's host time quadratic
+        int ctas = 0, g = steps2d_form(&ctas) ? free_steps(r, s, nsteps) : 0;
+        if (g == 0 || !enqueue_steps2d(g)) {
             stepwise = true;
             g = graphs ? group_length(r, s, nsteps) : 1;
             if (g > 1) launch_step_group(g);

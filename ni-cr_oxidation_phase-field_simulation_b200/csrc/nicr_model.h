@@ -141,6 +141,7 @@ public:
     BatchDomain step_desc() const;
     StepParams step_params() const;
     FlushDomain flush_desc() const;
+    int steps2d_form(int* ctas) const;
     bool enqueue_steps2d(int n);
     int free_steps(const RunPlan& r, int s, int nsteps) const;
     bool steps2d_failed = false;   // a cooperative launch was refused on this handle
