@@ -29,8 +29,10 @@ constexpr double PI = 3.14159265358979323846;
 
 // h(phi) interpolation (3S:171) and its derivative (3S:87)
 NICR_HD double h(double p) { return p * p * p * (10. - 15. * p + 6. * p * p); }
-// the same polynomial by Horner's rule, for the reciprocal form
-NICR_HD double h_fast(double p) { return (p * p) * p * fma(fma(6., p, -15.), p, 10.); }
+// the same for the reciprocal form: 10 - 15 p + 6 p^2 = 1 + (p - 1)(6 p - 9), whose
+// rounding vanishes with 1 - p (by Horner's rule 6 p - 15 rounds by 8 units of
+// the last place of h at p = 1, and a grain boundary's mobility multiplies 1 - h)
+NICR_HD double h_fast(double p) { return (p * p) * p * fma(p - 1., fma(6., p, -9.), 1.); }
 NICR_HD double hp(double p) { return 30. * p * p * (p - 1.) * (p - 1.); }
 // minimum-image offset for a periodic axis (3S:172)
 NICR_HD double min_image(double d, double period) { return d - period * round(d / period); }
