@@ -287,13 +287,13 @@ int nicr_step_noalloc(const nicr_config* cfg, const double* o, const double* cr,
 
 /* Autotuning (no counterpart in the reference). nicr_tune times `reps`
  * passes of the step kernels (and the eta update) on the handle's current
- * state for every X chunk the chooser considers (planes per CTA) and, in 3D,
- * both occupancy variants of the step kernel, writing only trial buffers, and
- * keeps the fastest; the state, budget and step count are unchanged. Fields
- * of later steps are the same bit for bit whatever is chosen; budget sums,
- * reduced per CTA, may differ in the last digits (~1e-16 relative).
+ * state for every X chunk the chooser considers (planes per CTA), writing only
+ * trial buffers, and keeps the fastest; the state, budget and step count are
+ * unchanged. Fields of later steps are the same bit for bit whatever is chosen;
+ * budget sums, reduced per CTA, may differ in the last digits (~1e-16 relative).
  * nicr_batch_tune chooses the batch's common X chunk the same way. The choice
- * is returned in *xchunk / *minb when not NULL. */
+ * is returned in *xchunk when not NULL; *minb receives the 3D step kernel's
+ * CTAs per SM (2, the one variant; 0 in 2D). */
 typedef struct nicr_batch nicr_batch;
 int nicr_tune(nicr_handle* h, int reps, int* xchunk, int* minb);
 int nicr_batch_tune(nicr_batch* b, int reps, int* xchunk);

@@ -102,7 +102,6 @@ struct StepParams {
     int inlet;                   // bc == concentration && oxygen_diffusion
     int xchunk;                  // planes per CTA along X
     int fast;                    // arithmetic form: 0 drop-in (bit-identical), 1 reciprocal divisions
-    int minb;                    // 3D step kernel: CTAs/SM variant 2 or 3 (0: the default)
     // Planes updated: [x_lo, x_hi) of the g.nx stored planes. A whole domain
     // updates all of them; an X slab of a larger domain stores halo planes
     // below and above its own, which the kernels read but do not write.

@@ -837,34 +837,29 @@ void Model::tune(int reps, int* xchunk, int* minb) {
     cudaEvent_t e0, e1;
     check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
     check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
-    int best_c = sp.xchunk, best_m = sp.minb;
+    int best_c = sp.xchunk;
     float best_ms = -1.f;
-    const std::vector<int> minbs = dim == 3 ? std::vector<int>{2, 3} : std::vector<int>{0};
     for (int c : xchunk_candidates(g.nx, sp.xchunk)) {
         set_xchunk(c);
-        for (int mb : minbs) {
-            sp.minb = mb;
-            step_kernels_prepare(sp);
-            if (onepass_step()) step_fused_prepare(sp, neta);
-            launch_trial_kernels();   // warm-up
-            check_cuda(cudaEventRecord(e0, stream), "cudaEventRecord");
-            for (int r = 0; r < reps; ++r) launch_trial_kernels();
-            check_cuda(cudaEventRecord(e1, stream), "cudaEventRecord");
-            check_cuda(cudaEventSynchronize(e1), "cudaEventSynchronize");
-            float ms = 0.f;
-            check_cuda(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
-            if (best_ms < 0.f || ms < best_ms) { best_ms = ms; best_c = c; best_m = mb; }
-        }
+        step_kernels_prepare(sp);
+        if (onepass_step()) step_fused_prepare(sp, neta);
+        launch_trial_kernels();   // warm-up
+        check_cuda(cudaEventRecord(e0, stream), "cudaEventRecord");
+        for (int r = 0; r < reps; ++r) launch_trial_kernels();
+        check_cuda(cudaEventRecord(e1, stream), "cudaEventRecord");
+        check_cuda(cudaEventSynchronize(e1), "cudaEventSynchronize");
+        float ms = 0.f;
+        check_cuda(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
+        if (best_ms < 0.f || ms < best_ms) { best_ms = ms; best_c = c; }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     check_cuda(cudaGetLastError(), "tune");
-    sp.minb = best_m;
     set_xchunk(best_c);   // also drops captured step graphs, a batch's through launch_form
     clear_status();   // what the trial launches of a failing state left
     sync();
     if (xchunk) *xchunk = best_c;
-    if (minb) *minb = best_m;
+    if (minb) *minb = dim == 3 ? 2 : 0;
 }
 
 void Model::prepare_step() {

@@ -130,8 +130,8 @@ public:
     // report failing trials to the error words that the next run reads.
     void clear_status();
     // Times `reps` launches of this domain's step (and eta update) kernels for
-    // each X chunk candidate and, in 3D, each occupancy variant, on the current
-    // state without committing anything, and keeps the fastest pair.
+    // each X chunk candidate, on the current state without committing anything,
+    // and keeps the fastest. minb: the step kernel's CTAs per SM (2 in 3D, else 0).
     void tune(int reps, int* xchunk, int* minb);
     // One pass of the step kernels into the trial buffers (no commit), and of
     // the eta update alone.
@@ -154,7 +154,7 @@ public:
     bool ksp_due(const RunPlan& r, int s) const;
     int parity_key() const { return cur | (ecur << 1) | (gcur << 2); }
     // counts the changes of what launches carry besides the parities (X chunk,
-    // kernel variant, partials): a captured launch serves its own count only
+    // partials): a captured launch serves its own count only
     int launch_form() const { return launch_form_; }
     void run_begin(RunPlan& r, int nsteps, bool schedule);
     void run_pre_step(RunPlan& r, int s);

@@ -377,9 +377,7 @@ void step_kernels_prepare(const StepParams& P) {
     }
     if (P.g.dim != 3) return;   // the 2D tile fits the default 48 KB
     using T = Tile<3, TA3, TB3>;
-    const bool m3 = step_minb_for(P) == 3;
-    const void* k = m3 ? (const void*)k_step_main<3, TA3, TB3, 3, false> : (const void*)k_step_main<3, TA3, TB3, 2, false>;
-    ensure_smem_attr(k, (int)T::SMEM_BYTES);
+    ensure_smem_attr((const void*)k_step_main<3, TA3, TB3, 2, false>, (int)T::SMEM_BYTES);
 }
 
 void launch_step_main(const StepParams& P, const double* o, const double* cr, const double* p, const double* gb,

@@ -1674,20 +1674,9 @@ __global__ void __launch_bounds__(TA * TB, MINB) k_step_batch(const __grid_const
 // and the powers of two below nx, the longer chunk on ties. Small domains get short chunks and use the whole GPU
 // (2D 128^2: 1 plane per CTA; 64^3: 4), large ones long chunks (256^3: 32).
 // NICR_XCHUNK forces a chunk for tuning runs.
-// Occupancy variant of the 3D step kernel: 2 CTAs/SM (no register cap, the
-// default: with the staging loads software-pipelined it is measured faster on
-// B200) or 3 CTAs/SM (80 registers, which spills). NICR_STEP_MINB=2|3 selects
-// one for tuning runs.
-static int step_minb() {
-    static int v = 0;
-    if (!v) {
-        const char* e = getenv("NICR_STEP_MINB");
-        v = (e && e[0] == '3') ? 3 : 2;
-    }
-    return v;
-}
-static int step_minb_for(const StepParams& P) { return P.minb == 2 || P.minb == 3 ? P.minb : step_minb(); }
-
+// The 3D step kernel holds 2 CTAs per SM: its staging loads are
+// software-pipelined, its budget books fill shared memory (85 KB per CTA), and
+// a third CTA's 80 registers spill.
 template <int DIM, int TA, int TB, int MINB, bool FAST, bool SLAB>
 static void launch_step_n(const StepParams& P, const double* o, const double* cr, const double* p, const double* gb,
                           const double* s2, double* on, double* crn, double* pn, StepPartial* partials,
@@ -1696,6 +1685,8 @@ static void launch_step_n(const StepParams& P, const double* o, const double* cr
     using T = Tile<DIM, TA, TB>;
     const dim3 grid = step_grid<DIM, TA, TB>(P);
     const int nblocks = (int)(grid.x * grid.y * grid.z);
+    // the CTAs of the launch bounds fit the SM's 228 KB (1 KB of it taken per CTA)
+    static_assert(MINB * (T::SMEM_BYTES + 1024) <= 228 * 1024, "shared memory holds fewer CTAs than the launch bounds state");
     ensure_smem_attr((const void*)k_step_main<DIM, TA, TB, MINB, FAST, SLAB>, (int)T::SMEM_BYTES);
     k_step_main<DIM, TA, TB, MINB, FAST, SLAB><<<nblocks + (budget ? 1 : 0), dim3(TB, TA), T::SMEM_BYTES, stream>>>(
         P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, (int)grid.x, (int)grid.y, nblocks);
@@ -1709,14 +1700,8 @@ static void launch_step_form(const StepParams& P, const double* o, const double*
                              cudaStream_t stream, int* nblocks_out) {
 #define NICR_STEP_FORM_ARGS P, o, cr, p, gb, s2, on, crn, pn, partials, prev, budget, st, stream, nblocks_out
     if (P.g.dim == 3) {
-        const bool m3 = step_minb_for(P) == 3;
-        if (P.slab) {
-            if (m3) launch_step_n<3, TA3, TB3, 3, FAST, true>(NICR_STEP_FORM_ARGS);
-            else launch_step_n<3, TA3, TB3, 2, FAST, true>(NICR_STEP_FORM_ARGS);
-        } else {
-            if (m3) launch_step_n<3, TA3, TB3, 3, FAST, false>(NICR_STEP_FORM_ARGS);
-            else launch_step_n<3, TA3, TB3, 2, FAST, false>(NICR_STEP_FORM_ARGS);
-        }
+        if (P.slab) launch_step_n<3, TA3, TB3, 2, FAST, true>(NICR_STEP_FORM_ARGS);
+        else launch_step_n<3, TA3, TB3, 2, FAST, false>(NICR_STEP_FORM_ARGS);
     } else {
         launch_step_n<2, TA2, TB2, 4, FAST, false>(NICR_STEP_FORM_ARGS);
     }

@@ -372,8 +372,8 @@ class Solver:
         return out
 
     def tune(self, reps: int = 3):
-        """Measures and keeps the fastest X chunk / occupancy variant (nicr_tune);
-        returns (xchunk, minb). The state is unchanged."""
+        """Measures and keeps the fastest X chunk (nicr_tune); returns it and the 3D
+        step kernel's CTAs per SM (0 in 2D). The state is unchanged."""
         c, m = ctypes.c_int(0), ctypes.c_int(0)
         self._check(lib().nicr_tune(self.h, reps, ctypes.byref(c), ctypes.byref(m)))
         return c.value, m.value
