@@ -445,7 +445,8 @@ int nicr_slab_box_half(const nicr_handle* h);
  * accumulation, on device pointers and the caller's CUDA stream. x: NDHWC
  * BF16 (n, d, h, w, cin); w: BF16 [cout][27][cin], tap = (dz+1)*9 +
  * (dy+1)*3 + (dx+1); y, dw: FP32. n*d*h*w a multiple of 64; cin and cout
- * multiples of 16. nicr_conv3d_fwd: y[v][co] = sum x[v+off(tap)][ci]
+ * multiples of 16; arrays that are not 16-byte aligned are refused with
+ * NICR_ERR_INVALID_ARG. nicr_conv3d_fwd: y[v][co] = sum x[v+off(tap)][ci]
  * w[co][tap][ci]. nicr_conv3d_wgrad: dw[co][tap][ci] = sum_v dy[v][co]
  * x[v+off(tap)][ci] (dy: BF16 NDHWC with cout channels). The data gradient
  * is nicr_conv3d_fwd of dy with w'[ci][tap][co] = w[co][26-tap][ci].

@@ -1528,6 +1528,12 @@ int check_args(long long voxels, int cin, int cout) {
     return NICR_OK;
 }
 
+// Every form moves 16 bytes at a time; a tensor map refuses another base, a
+// vector or cp.async access to it would fault.
+bool aligned16(const void* p) { return (reinterpret_cast<unsigned long long>(p) & 15ull) == 0; }
+template <class... P>
+bool aligned16(const void* p, const P*... more) { return aligned16(p) && aligned16(more...); }
+
 // ---------------------------------------------------------------- elementwise passes around the convolutions
 __device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -1670,7 +1676,6 @@ int elementwise_blocks(long long items) {
     const long long want = (items + 255) / 256;
     return (int)(want < 148 * 16 ? (want > 0 ? want : 1) : 148 * 16);
 }
-bool aligned16(const void* p) { return (reinterpret_cast<unsigned long long>(p) & 15ull) == 0; }
 
 }  // namespace
 
@@ -1741,7 +1746,8 @@ int nicr_conv3d_fwd_shift(const void* x, const void* w, const float* bias, int a
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
     ShiftConv C;
-    if (rc != NICR_OK || !x || !w || !y || (act & ~(ACT_RELU | ACT_BF16)) != 0 || !shift_plan(V, cin, cout, C))
+    if (rc != NICR_OK || !x || !w || !y || !aligned16(x, w, bias, y) || (act & ~(ACT_RELU | ACT_BF16)) != 0 ||
+        !shift_plan(V, cin, cout, C))
         return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     const auto enc = conv_map_encoder();
     if (!enc) return NICR_ERR_CUDA;
@@ -1821,7 +1827,8 @@ int nicr_conv3d_fwd_halo(const void* x, const void* w, const float* bias, int ac
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
     HaloConv H;
-    if (rc != NICR_OK || !x || !w || !y || (act & ~(ACT_RELU | ACT_BF16)) != 0 || !halo_plan(V, cin, cout, H))
+    if (rc != NICR_OK || !x || !w || !y || !aligned16(x, w, bias, y) || (act & ~(ACT_RELU | ACT_BF16)) != 0 ||
+        !halo_plan(V, cin, cout, H))
         return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     const auto enc = conv_map_encoder();
     if (!enc) return NICR_ERR_CUDA;
@@ -1848,7 +1855,8 @@ int nicr_conv3d_fwd_march(const void* x, const void* w, const float* bias, int a
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
     MarchConv M;
-    if (rc != NICR_OK || !x || !w || !y || (act & ~(ACT_RELU | ACT_BF16)) != 0 || !march_plan(V, cin, cout, M))
+    if (rc != NICR_OK || !x || !w || !y || !aligned16(x, w, bias, y) || (act & ~(ACT_RELU | ACT_BF16)) != 0 ||
+        !march_plan(V, cin, cout, M))
         return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     const auto enc = conv_map_encoder();
     if (!enc) return NICR_ERR_CUDA;
@@ -1878,7 +1886,7 @@ int launch_fwd_tma(const void* x, const void* w, const float* bias, int act, voi
                    int cin, int cout, void* stream) {
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
-    if (rc != NICR_OK || !x || !w || !y || (act & ~(ACT_RELU | ACT_BF16)) != 0)
+    if (rc != NICR_OK || !x || !w || !y || !aligned16(x, w, bias, y) || (act & ~(ACT_RELU | ACT_BF16)) != 0)
         return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     const auto enc = conv_map_encoder();
     if (!enc) return NICR_ERR_CUDA;
@@ -1932,7 +1940,7 @@ int nicr_conv3d_fwd_gather(const void* x, const void* w, float* y, int n, int d,
                            void* stream) {
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
-    if (rc != NICR_OK || !x || !w || !y) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
+    if (rc != NICR_OK || !x || !w || !y || !aligned16(x, w, y)) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     const int cmax = cout < 256 ? cout : 256;
     int kc = 64;   // channels per chunk: the largest of 64, 48, 32, 16 dividing Cin
     while (cin % kc != 0) kc -= 16;
@@ -1955,7 +1963,7 @@ int nicr_conv3d_fwd_mma_sync(const void* x, const void* w, float* y, int n, int 
                              void* stream) {
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
-    if (rc != NICR_OK || !x || !w || !y) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
+    if (rc != NICR_OK || !x || !w || !y || !aligned16(x, w)) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     const dim3 grid((unsigned)(V.voxels() / BM), (unsigned)((cout + BN - 1) / BN));
     k_conv3d_fwd<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), y, V, cin, cout);
@@ -1966,7 +1974,7 @@ int nicr_conv3d_wgrad_tma(const void* x, const void* dy, float* dw, int n, int d
                           void* stream) {
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
-    if (rc != NICR_OK || !x || !dy || !dw) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
+    if (rc != NICR_OK || !x || !dy || !dw || !aligned16(x, dy, dw)) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     TmaWgrad G;
     if (!tma_wgrad_plan(V, cin, cout, G)) return NICR_ERR_INVALID_ARG;
     const auto enc = conv_map_encoder();
@@ -2009,7 +2017,7 @@ int nicr_conv3d_wgrad_mma_sync(const void* x, const void* dy, float* dw, int n, 
                                void* stream) {
     const Vol V{n, d, h, w_};
     const int rc = check_args(V.voxels(), cin, cout);
-    if (rc != NICR_OK || !x || !dy || !dw) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
+    if (rc != NICR_OK || !x || !dy || !dw || !aligned16(x, dy)) return rc != NICR_OK ? rc : NICR_ERR_INVALID_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const long long M = V.voxels();
     // enough voxel slices to fill the GPU: 27 x (Cin/16) x (Cout/16) x parts CTAs
