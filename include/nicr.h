@@ -470,9 +470,9 @@ int nicr_conv3d_fwd_tma(const void* x, const void* w, float* y, int n, int d, in
 int nicr_conv3d_fwd_act(const void* x, const void* w, const float* bias, int act, void* y, int n, int d, int h, int w_,
                         int cin, int cout, void* stream);
 /* The same from a staged halo block (Cout <= 64 and rows of at least 128
- * voxels, else NICR_ERR_INVALID_ARG); nicr_conv3d_fwd_act and
- * nicr_conv3d_fwd use it for Cout <= 32 with Cin x Cout <= 768 where
- * nicr_conv3d_fwd_shift does not apply. */
+ * voxels, else NICR_ERR_INVALID_ARG): a reference form, which
+ * nicr_conv3d_fwd_act does not choose (nicr_conv3d_fwd_shift serves its
+ * shapes). */
 int nicr_conv3d_fwd_halo(const void* x, const void* w, const float* bias, int act, void* y, int n, int d, int h, int w_,
                          int cin, int cout, void* stream);
 /* The halo-block forward marching along y (a CTA keeps its input lines and

@@ -15,9 +15,11 @@
 // shape in nicr_conv3d_fwd_act from measured rates:
 //   k_conv3d_fwd_march  Cin 16, rows >= 128: halo lines kept on chip along y
 //   k_conv3d_fwd_shift  narrow outputs: input lines staged once, x taps as row shifts
-//   k_conv3d_fwd_halo   narrow outputs, rows >= 128: one halo block per chunk
 //   k_conv3d_fwd_tma    everything else: per-tap TMA boxes
 //   k_conv3d_fwd_tc     where the driver refuses a tensor map: cp.async gathers
+// k_conv3d_fwd_halo (one halo block per chunk) served the narrowest layers on
+// rows >= 128 before the row shifts, which take all of its shapes (halo_shape);
+// it stays as a reference form, called by name.
 // The weight gradient runs on tcgen05.mma with TMA-staged operands
 // (k_conv3d_wgrad_tma) for Cout 16, 32, 64 or multiples of 128. The
 // warp-level WMMA forms (16x16x16 BF16 tiles staged through shared memory)
@@ -1224,7 +1226,9 @@ __global__ void __launch_bounds__(SH_THREADS) k_conv3d_fwd_shift(const __grid_co
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C.cols));
 }
 
-// The halo block's shapes (its accumulation order is order 1 above).
+// The shapes that the halo block served; their sums keep its order (order 1
+// above). The row shifts fit all of them: one 16-channel box per line, so one
+// line per item (T = 1) needs 4 lines and 3 weight blocks, 30 KB.
 bool halo_shape(const Vol& V, int cin, int cout) { return cout <= 32 && cin * cout <= 768 && V.w >= TC_M; }
 
 // The row-shift plan, or false outside its shapes (Cout <= 64).
@@ -1812,11 +1816,6 @@ int nicr_conv3d_fwd_act(const void* x, const void* w, const float* bias, int act
     }
     if (w_ > TC_M / 2 || (w_ > TC_M / 4 && cout <= 32 && cin * cout <= 1024)) {
         const int rc = nicr_conv3d_fwd_shift(x, w, bias, act, y, n, d, h, w_, cin, cout, stream);
-        if (rc != NICR_ERR_INVALID_ARG) return rc;
-    }
-    HaloConv H;
-    if (halo_shape(Vol{n, d, h, w_}, cin, cout) && halo_plan(Vol{n, d, h, w_}, cin, cout, H)) {
-        const int rc = nicr_conv3d_fwd_halo(x, w, bias, act, y, n, d, h, w_, cin, cout, stream);
         if (rc != NICR_ERR_INVALID_ARG) return rc;
     }
     return launch_fwd_tma(x, w, bias, act, y, n, d, h, w_, cin, cout, stream);
