@@ -54,7 +54,7 @@ struct nicr_batch {
             nicr::Model& m = *doms[i]->m;
             m.prepare_step();
             descs[i] = m.step_desc();
-            m.enqueue_eta();   // before the step kernel, whose last CTA per domain commits the step
+            m.enqueue_eta();   // before the step kernel, which leaves this step pending and commits the domain's previous one
         }
         launches += nicr::launch_step_batch(descs.data(), n, stream);
         for (int i = 0; i < n; ++i) doms[i]->m->complete_step();

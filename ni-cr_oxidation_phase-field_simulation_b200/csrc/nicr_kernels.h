@@ -309,8 +309,6 @@ struct VtiArgs {
 };
 void launch_vti_arrays(const VtiArgs& a, void* out, bool f64, unsigned* range, cudaStream_t stream);
 
-// Commits the pending step, if any: its partials (of parity q at partials +
-// q * cap) reduced, then budget and counters unless a trial failed.
 // Many steps of a small 2D domain in one cooperative launch and its commit
 // (nicr_steps2d.cuh): steps2d_tile gives the tile's planes TX for which the
 // domain's CTAs of TX x 32 cells are resident one per SM (0: too large, or no
@@ -327,6 +325,9 @@ int steps2d_tile(const Grid& g, int* ctas);
 bool launch_steps2d(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, DevBudget* budget, Status* st,
                     Status* host, cudaStream_t stream);
 bool launch_steps2d_fast(const StepParams& P, const Steps2DArgs& A, int tx, int ctas, Status* st, cudaStream_t stream);
+// Commits each domain's pending step, if any: its partials (of parity q at
+// partials + q * cap) reduced, then budget and counters unless a trial failed;
+// the status word is written to the host either way.
 struct FlushDomain {
     const StepPartial* partials;
     DevBudget* budget;

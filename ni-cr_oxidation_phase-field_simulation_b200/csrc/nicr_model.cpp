@@ -964,7 +964,7 @@ void Model::enqueue_step() {
         complete_step();
         return;
     }
-    enqueue_eta();   // before the step kernel, whose last CTA commits the step
+    enqueue_eta();   // before the step kernel, which leaves this step pending and commits the previous one
     const size_t e = prof_begin();
     launch_step_main(d.sp, d.o, d.cr, d.p, d.gb, d.s2, d.on, d.crn, d.pn, d.partials, d.prev, bud, st, stream, &nb);
     prof_end(K_STEP_MAIN, e, 1);
@@ -1095,8 +1095,9 @@ bool Model::ksp_due(const RunPlan& r, int s) const {
 }
 
 // Step graphs. Replaying a captured run of 2..16 steps costs one host launch
-// instead of two or three per step, which decides the step rate of small
-// domains (a 2D 128^2 step is a few microseconds of GPU work). An even run
+// instead of one or two per step (the step kernel, and the eta update in the
+// two-kernel form), which decides the step rate of small domains (a 64^3 step
+// is 19 us; 2D domains of up to 37,888 cells take k_steps2d instead). An even run
 // returns the buffer parity to where it started, so one graph per length and
 // starting parity serves every run; the kernels read their run constants from their
 // parameters and the batch-stop flag from device memory, both unchanged

@@ -113,9 +113,11 @@ public:
     // One step split into phases, for batches that launch the step kernel of
     // many domains at once: prepare_step (eta mask when stale), step_desc (the
     // step kernel's parameters and buffers), enqueue_eta (the eta update, before
-    // the step kernel, whose last CTA commits the step), then complete_step
-    // (buffer parity). run_begin / run_pre_step / run_end are
-    // run()'s schedule (Ksp scans) and commit around those steps.
+    // the step kernel: its launch leaves the step pending and commits the one
+    // before, so budget and status are those of the call only after
+    // flush_commit), then complete_step (buffer parity). run_begin /
+    // run_pre_step / run_end are run()'s schedule (Ksp scans) and the last
+    // step's commit around those steps.
     struct RunPlan {
         long long before = 0;
         int nsteps = 0;

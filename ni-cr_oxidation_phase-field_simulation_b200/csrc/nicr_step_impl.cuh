@@ -168,8 +168,9 @@ struct Tile {
 // unscaled; the caller folds S into the constant that multiplies a sum.
 //
 // DivRun: quotients carried times 2^128 (xdiv_scaled), so a Laplacian's three
-// quotients and the faces of a divergence are never scaled back (4 to 6 FP64
-// operations per division instead of 6). It keeps in `low` the smallest
+// quotients and the faces of a divergence are never scaled back: 4 FP64
+// operations per division, 5 from an unscaled numerator, or 2 (TWO below),
+// instead of 6. It keeps in `low` the smallest
 // 2 * (high word) - 1 of the quotients (zero wraps to the largest), from which
 // one comparison at the end of the march tells whether any nonzero quotient
 // was subnormal (two integer operations per division instead of five).
@@ -184,7 +185,8 @@ struct Reciprocal {
 };
 // TWO: every divisor takes two operations (division_in_two; dx, dx^2 and dt of
 // the default configurations, 93% of random divisors), instead of four or, from
-// an unscaled numerator, five. FIGURES
+// an unscaled numerator, five: 256^3 with 8 fields 2720 -> 2356 us per two
+// steps, 151 x 101 x 101 static 1204 -> 1090 us per ten.
 template <bool TWO>
 struct DivRun {
     static constexpr bool kFast = false;
@@ -1011,9 +1013,11 @@ __device__ __forceinline__ void eta_cell(const StepParams& P, int neta, const do
     errkey = min(errkey, k);
 }
 
-// Bounds for 5 CTAs/SM (<= 51 registers, no spills): the load-latency-bound
-// per-cell kernel measured 1.13 ms vs 1.29 ms unbounded (62 registers, 4/SM)
-// at 256^3 with 8 fields; 6/SM spills (1.27 ms).
+// Bounds for 5 CTAs/SM: the load-latency-bound per-cell kernel measured 1.13 ms
+// vs 1.29 ms unbounded (62 registers, 4/SM) at 256^3 with 8 fields and the
+// division of that build, 1.27 ms at 6/SM. At the 48 registers of 5/SM the exact
+// form's three passes (div_gate is known at launch only) spill 84 bytes in 3D
+// and 192 in 2D, the reciprocal form 48 bytes in 3D.
 template <int DIM, bool FAST>
 __global__ void __launch_bounds__(256, 5) k_eta_update(const StepParams P, int neta, const double* __restrict__ eta,
                              const double* __restrict__ s2, const double* __restrict__ p,
@@ -1667,13 +1671,6 @@ __global__ void __launch_bounds__(TA * TB, MINB) k_step_batch(const __grid_const
 
 }  // namespace
 
-// X chunk of the step and eta kernels. A CTA marching c planes also computes
-// mu and M of the plane before its chunk and stages that plane's halo, about
-// two planes of extra work, and CTAs run in waves of 2 (3D) or 4 (2D) per SM,
-// so the chunk minimising waves x (c + 2) is taken among nx halved repeatedly
-// and the powers of two below nx, the longer chunk on ties. Small domains get short chunks and use the whole GPU
-// (2D 128^2: 1 plane per CTA; 64^3: 4), large ones long chunks (256^3: 32).
-// NICR_XCHUNK forces a chunk for tuning runs.
 // The 3D step kernel holds 2 CTAs per SM: its staging loads are
 // software-pipelined, its budget books fill shared memory (85 KB per CTA), and
 // a third CTA's 80 registers spill.
